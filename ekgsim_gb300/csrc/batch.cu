@@ -1458,22 +1458,47 @@ void launch_batch_gemm(cudaStream_t s, const BatchArgs &A) {
 // A layer's resting potential k0 adds k0_L sum_{a in L} W[l][a] to every sample of lead l (the AP
 // differences of the dipoles cancel it within a layer, simlib/simulator.cpp:509-525); the sum over
 // layers of sum_a W vanishes, so the term is taken relative to the first layer's k0.
-// Moved rows: thread per row' = l * S + s, the per-part unscaled sums P2 of each layer's stages
-// added in FP64 in a fixed order.
-__global__ void k_k0_moved(int rows_used, int n_sims, int nl, const int32_t *__restrict__ ls0,
-                           const int32_t *__restrict__ ls1, const float *__restrict__ P2,
-                           const double *__restrict__ layer_k, double *__restrict__ cmov) {
-    const int rp = blockIdx.x * blockDim.x + threadIdx.x;
+// Moved rows: the unscaled sums P2 of each layer's 8-AP parts added in FP64, in a fixed order, in two
+// passes.  k_k0_parts cuts a layer's parts into K0_SEGS segments, block per (32 rows, segment, layer), a
+// lane per row so that a part's read is one 128-byte line, the eight warps taking parts in turn:
+// Ks[row'][L][segment].  k_k0_moved adds the segments, a warp per row' = l * S + s.  Bound by the read of
+// P2 (HBM) once there are enough rows; one thread per row over all parts of a layer was a serial chain
+// of dependent loads and FP64 additions (128^3, 64 simulations x 3 moved leads: 1.89 ms of a 2.34 ms
+// call, which now takes 0.45).
+constexpr int K0_SEGS = 32;
+__global__ void __launch_bounds__(256) k_k0_parts(int rows_used, int nl, const int32_t *__restrict__ ls0,
+                                                  const int32_t *__restrict__ ls1, const float *__restrict__ P2,
+                                                  double *__restrict__ Ks) {
+    __shared__ double red[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int rp = blockIdx.x * 32 + lane, seg = blockIdx.y, L = blockIdx.z;
+    const int64_t p0 = (int64_t)ls0[L] * 4, n = (int64_t)(ls1[L] - ls0[L]) * 4;
+    const int64_t b = p0 + n * seg / K0_SEGS, e = p0 + n * (seg + 1) / K0_SEGS;
+    double v = 0.0;
+    if (rp < rows_used)
+#pragma unroll 4
+        for (int64_t p = b + w; p < e; p += 8) v += (double)P2[(size_t)p * rows_used + rp];
+    red[w][lane] = v;
+    __syncthreads();
+    if (w == 0 && rp < rows_used) {
+        double t = red[0][lane];
+        for (int k = 1; k < 8; ++k) t += red[k][lane];
+        Ks[((size_t)rp * nl + L) * K0_SEGS + seg] = t;
+    }
+}
+__global__ void __launch_bounds__(256) k_k0_moved(int rows_used, int n_sims, int nl, const double *__restrict__ Ks,
+                                                  const double *__restrict__ layer_k, double *__restrict__ cmov) {
+    const int lane = threadIdx.x & 31, rp = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (rp >= rows_used) return;
     const int s = rp % n_sims;
     const double k00 = layer_k[(size_t)s * nl * 9];
     double c = 0.0;
     for (int L = 0; L < nl; ++L) {
-        double sw = 0.0;
-        for (int p = ls0[L] * 4; p < ls1[L] * 4; ++p) sw += (double)P2[(size_t)p * rows_used + rp];
+        double sw = Ks[((size_t)rp * nl + L) * K0_SEGS + lane];
+        for (int o = 16; o > 0; o >>= 1) sw += __shfl_xor_sync(0xffffffffu, sw, o);
         c += (layer_k[((size_t)s * nl + L) * 9] - k00) * sw;
     }
-    cmov[rp] = c;
+    if (lane == 0) cmov[rp] = c;
 }
 
 // Static leads: K0s[L][l] = sum_{a in L} W0[l][a] in FP64, block per (lead, layer).
@@ -1509,10 +1534,14 @@ __global__ void k_k0_static(int n_sims, int nleads, int nmove, int nl, const dou
     cst[i] = c;
 }
 
-void launch_k0_moved(cudaStream_t s, const BandArgs &A, const int32_t *ls0, const int32_t *ls1,
-                     const double *layer_k, double *cmov) {
-    k_k0_moved<<<(unsigned)((A.rows_used + 127) / 128), 128, 0, s>>>(A.rows_used, A.n_sims, A.nl, ls0, ls1, A.P2,
-                                                                     layer_k, cmov);
+int k0_segments() { return K0_SEGS; }
+
+void launch_k0_moved(cudaStream_t s, const BandArgs &A, const int32_t *ls0, const int32_t *ls1, const double *layer_k,
+                     double *Ks, double *cmov) {
+    k_k0_parts<<<dim3((unsigned)((A.rows_used + 31) / 32), K0_SEGS, (unsigned)A.nl), 256, 0, s>>>(A.rows_used, A.nl, ls0,
+                                                                                                 ls1, A.P2, Ks);
+    EKG_CUDA(cudaGetLastError());
+    k_k0_moved<<<(unsigned)((A.rows_used + 7) / 8), 256, 0, s>>>(A.rows_used, A.n_sims, A.nl, Ks, layer_k, cmov);
     EKG_CUDA(cudaGetLastError());
 }
 

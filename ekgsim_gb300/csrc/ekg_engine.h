@@ -79,6 +79,7 @@ struct BatchState {
     // layer sums of the resident lead field (K0s, valid while the band tables are)
     DBuf<float> P2;                        // [stages * 4][rows_used]
     DBuf<double> cmov, cst;                // [rows_used], [S][L]
+    DBuf<double> k0seg;                    // [rows_used][nl][k0_segments()] segment sums behind cmov
     DBuf<double> K0s;                      // [nl][L]
     bool k0s_ok = false;
 };

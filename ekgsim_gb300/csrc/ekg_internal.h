@@ -327,8 +327,10 @@ void launch_band_u(cudaStream_t s, const BandArgs &a);
 // Resting-potential term of the batched form where k0 differs between layers:
 //   moved rows   cmov[l * S + s] = sum_L (k0_L - k0_0) sum_{a in L} W_s[l][a]   (from P2)
 //   static leads K0s[L][l] = sum_{a in L} W0[l][a] (per heart), cst[s][l] = sum_L (k0_L - k0_0) K0s[L][l]
-void launch_k0_moved(cudaStream_t s, const BandArgs &a, const int32_t *ls0, const int32_t *ls1,
-                     const double *layer_k, double *cmov);
+//   (Ks: scratch, [rows'][nl][k0_segments()])
+int k0_segments();
+void launch_k0_moved(cudaStream_t s, const BandArgs &a, const int32_t *ls0, const int32_t *ls1, const double *layer_k,
+                     double *Ks, double *cmov);
 void launch_k0_static_sums(cudaStream_t s, int nleads, int64_t apad, int nl, const int32_t *ls0,
                            const int32_t *ls1, const float *W0, double *K0s);
 // cst[s][l] (l >= nmove) = sum_L (k0_L - k0_0) K0s[L][l], or sum_L k0_L K0s[L][l] when !relative

@@ -1069,6 +1069,8 @@ void upload_inputs(ekg_heart *h, const PassPlan &P, const double *layer_k, const
             if (P.k0) {
                 if (B.P2.n < 4 * p1) B.P2.alloc(4 * p1);
                 if (B.cmov.n < (size_t)P.rows_used) B.cmov.alloc(P.rows_used);
+                const size_t ks = (size_t)P.rows_used * D.nlayers * k0_segments();
+                if (B.k0seg.n < ks) B.k0seg.alloc(ks);
             }
             if (!B.work.p) B.work.alloc(1);
             const size_t ub = (size_t)P.rows_used * D.nlayers * B.max_ent;
@@ -1173,8 +1175,8 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
             }
             launch_band_u(sx, U);
             if (P.k0) {
-                launch_k0_moved(sx, U, B.ls0.p, B.ls1.p, in.layer_k, B.cmov.p);
-                ++launches;
+                launch_k0_moved(sx, U, B.ls0.p, B.ls1.p, in.layer_k, B.k0seg.p, B.cmov.p);
+                launches += 2;
             }
             if (fork) EKG_CUDA(cudaEventRecord(h->ev_join, sx));
             launches += 2;
@@ -1299,7 +1301,7 @@ std::vector<uint64_t> pass_signature(const ekg_heart *h, const PassPlan &P, int 
                           (const void *)B.tref.p, (const void *)h->dev.stage_order.p, (const void *)B.nent.p, (const void *)B.esplit.p, (const void *)B.ls0.p,
                           (const void *)B.ls1.p, (const void *)B.ent.p, (const void *)B.goff.p, (const void *)B.gtab.p,
                           (const void *)B.E.p, (const void *)B.work.p, (const void *)h->W0.p, (const void *)B.P2.p,
-                          (const void *)B.cmov.p, (const void *)B.cst.p, (const void *)B.K0s.p, (const void *)E.band.p,
+                          (const void *)B.cmov.p, (const void *)B.k0seg.p, (const void *)B.cst.p, (const void *)B.K0s.p, (const void *)E.band.p,
                           (const void *)E.csum.p, (const void *)E.cinfo.p, (const void *)h->W0_layer.p, (const void *)E.work.p,
                           (const void *)h->dev.stage_order.p})
         v.push_back(u(p));
