@@ -604,8 +604,8 @@ def run_ours(args):
         "roofline": roof,
         # the activation-time relaxation (once per heart): N^3 x 1 B layers in + N^3 x 8 B times out;
         # latency-bound (one dependent launch per time bucket), so the fraction is its byte floor
-        "ca": {"kernel": "k_ca_bucket" if info.ca_buckets else "k_ca_round_list", "steps": int(info.ca_rounds),
-               "form": "time buckets" if info.ca_buckets else "tile rounds", "ms": info.ca_ms,
+        "ca": {"kernel": "k_ca_round", "steps": int(info.ca_rounds),
+               "form": "tile rounds up to a horizon", "ms": info.ca_ms,
                "algorithmic_bytes": 9 * int(info.n_cells),
                "achieved_gbs": 9 * info.n_cells / (info.ca_ms / 1000.0) / 1e9 if info.ca_ms > 0 else None,
                "frac": 9 * info.n_cells / (info.ca_ms / 1000.0) / 1e9 / hbm if info.ca_ms > 0 else None},

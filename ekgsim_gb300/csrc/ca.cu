@@ -9,17 +9,21 @@
 // +inf converges to the same doubles bit for bit, in any order.  Products and sums use
 // __dmul_rn / __dadd_rn so the compiler cannot fuse them into an FMA.
 //
-// Layout: the grid is cut into 8x8x8 tiles.  A round processes the active tiles, one CTA each:
-// the tile and a one-voxel halo are staged in shared memory (the FP64 times as their bit patterns,
-// which order like the values for non-negative doubles, + uint8 layers).  The tile relaxes
-// locally: a first sweep pulls every voxel's candidates from its 26 neighbours, later sweeps only
-// push from the voxels that improved in the sweep before (64-bit atomicMin on the bit patterns),
-// until a block-wide vote (__syncthreads_or) finds no change.  A candidate is skipped without the
-// FP64 add when the offering voxel is not earlier than the receiving one (lags are positive).  The
-// changed interior voxels are written back and the neighbour tiles that touch a changed face,
-// edge or corner are flagged.  A compaction kernel turns the flags into the next round's tile list
-// with warp ballots and one atomic per warp.  The host loops until no tile is active.
+// Layout: the grid is cut into 8x8x8 tiles.  A round visits the tiles that hold pending times, one
+// CTA each: the tile and a one-voxel halo are staged in shared memory (the FP64 times as their bit
+// patterns, which order like the values for non-negative doubles, + uint8 layers), the tile settles up to
+// the round's horizon, the settled times are written back, and the tiles that were offered a time or
+// hold later ones form the next round's list (k_ca_round).  The host queues rounds in chunks and reads
+// the lists' length once per chunk.
+//
+// GB300, 12 leads aside (relaxation alone, CUDA events): 24^3 0.13 ms, 64^3 0.34, 128^3 0.77, 160^3 1.02
+// (49 rounds), 192^3 1.32, 256^3 2.45.  One launch per time bucket over queues in global memory took
+// 0.24, 0.57, 1.40, 1.96, 3.04 and 5.64 ms (9 us a bucket, every access of its chain a trip to L2); rounds
+// of block-wide sweeps to local convergence, without a horizon, 3.4 ms at 160^3 in the calls that
+// allocate nothing.
+#include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <mutex>
 #include <vector>
@@ -32,500 +36,302 @@ namespace {
 
 constexpr int TS = 8;            // tile edge
 constexpr int HS = TS + 2;       // tile + halo
-constexpr int CA_THREADS = 256;  // 2 voxels per thread
-constexpr int MAX_LOCAL_ITERS = 64;
+constexpr int HCELLS = HS * HS * HS;
+constexpr int CA_THREADS = TS * TS * TS;  // one thread per voxel of the tile
+constexpr int CA_WARPS = CA_THREADS / 32;
 
 __device__ __forceinline__ uint8_t layer_id(uint8_t v) { return v; }
 __device__ __forceinline__ uint8_t layer_id(int32_t v) { return (uint8_t)(v < 0 ? -v : v); }
 
-// One tile of a round (all threads of the block): stage, relax, write back, flag neighbours.
+// While the relaxation runs, a cell's entry holds 2 * (bits of its time) + 1 while the time is pending (the
+// cell has not offered it to its neighbours yet), 2 * bits once it has.  Entries order by time, and
+// an offer of the same time does not replace a settled one.
+typedef unsigned long long u64;
+constexpr u64 INF_BITS = 0x7ff0000000000000ULL;
+
+// The active tiles of consecutive rounds.  Round r walks list r & 1 (counts[r % 3] tiles), appends the
+// tiles that hold pending times to list (r + 1) & 1 and clears the slot of round r + 2.
+struct TileLists {
+    int32_t *list;     // [2][cap]
+    int cap;
+    int32_t *counts;   // [3] tiles of a round, then the number of rounds that had a tile
+    uint32_t *first;   // [3] high word of the earliest pending time of a round
+    uint32_t *flags;   // one byte per tile, in words: bit (r & 1) set while the tile is in round r's list
+};
+constexpr int CA_CTRL_WORDS = 4 + 3;  // words of counts and first, one behind the other
+
+__device__ __forceinline__ void tile_append(const TileLists &T, int tile, int round) {
+    const uint32_t bit = 1u << (8 * (tile & 3) + (round & 1));
+    if (!(atomicOr(&T.flags[tile >> 2], bit) & bit))
+        T.list[(size_t)(round & 1) * T.cap + atomicAdd(&T.counts[round % 3], 1)] = tile;
+}
+// One round: a block per active tile, the grid walking the list, so that rounds can be queued back to
+// back without the host reading the count.
+//
+// What bounds it: latency -- a chain of rounds, in a round the slowest tile's chain of settling steps,
+// in a step its barriers and dependent shared-memory accesses.  Hence:
+//  - a tile settles its voxels in the order of their times, as the search itself does: per step the
+//    voxels whose pending time lies within the smallest lag of the earliest pending one (nothing
+//    later inside the tile can improve them) offer to their 26 neighbours, a warp per voxel and a
+//    lane per neighbour, so that each voxel offers about once;
+//  - a step has one barrier and no list: a warp expands the selected ones of its own 32 voxels, which
+//    lie spread over the tile so that a front falls on all warps, and the earliest pending time of
+//    the next step is taken from each warp's own voxels and the offers that it made;
+//  - offers across the tile's surface go to the neighbour's cells in global memory (an atomicMin whose
+//    result nothing waits for), so that a visit starts from the pending cells alone;
+//  - a round settles only times up to its horizon, the earliest pending time of the heart + `window`
+//    (a few of the largest lags), and later ones wait for their round: the front then moves at the
+//    speed of the wave and not a tile per round, so that times which a faster path would replace are
+//    not spread first.
 template <typename LT>
-__device__ __forceinline__ void ca_tile(const int tile, int nz, int ny, int nx, int ntz, int nty, int ntx,
-                                        const LT *__restrict__ layers, const double *__restrict__ lag, int nl1,
-                                        double *__restrict__ at, uint8_t *__restrict__ next_flag) {
-    __shared__ unsigned long long s_b[HS][HS][HS];  // activation-time bits
-    __shared__ uint8_t s_l[HS][HS][HS];
-    __shared__ uint8_t s_ch[2][HS][HS][HS];         // improved in the last sweep (tile interior)
-    __shared__ uint32_t s_mark;  // 27-bit mask of neighbour tiles to flag (bit = (dz+1)*9+(dy+1)*3+(dx+1))
-
-    const int tx0 = (tile % ntx) * TS;
-    const int ty0 = ((tile / ntx) % nty) * TS;
-    const int tz0 = (tile / (ntx * nty)) * TS;
-    const int tid = threadIdx.x;
-    if (tid == 0) s_mark = 0;
-
-    // stage tile + halo
-    const unsigned long long INF_BITS = 0x7ff0000000000000ULL;
-    for (int i = tid; i < HS * HS * HS; i += CA_THREADS) {
-        int hx = i % HS, hy = (i / HS) % HS, hz = i / (HS * HS);
-        int gx = tx0 + hx - 1, gy = ty0 + hy - 1, gz = tz0 + hz - 1;
-        unsigned long long b = INF_BITS;
-        uint8_t l = 0;
-        if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && gz >= 0 && gz < nz) {
-            size_t g = ((size_t)gz * ny + gy) * nx + gx;
-            l = layer_id(layers[g]);
-            if (l) b = (unsigned long long)__double_as_longlong(at[g]);
+__global__ void __launch_bounds__(CA_THREADS, 3)
+    k_ca_round(int round, int nz, int ny, int nx, int ntz, int nty, int ntx, const LT *__restrict__ layers,
+               const double *__restrict__ lag, int nl1, double window, u64 *__restrict__ at, TileLists T) {
+    __shared__ u64 s_e[HCELLS];       // entries of the tile and its halo
+    __shared__ uint8_t s_l[HCELLS];   // layers
+    __shared__ uint8_t s_dir[HCELLS]; // which of the 27 tiles a cell lies in, 13 = this one ((dz+1)*9+(dy+1)*3+(dx+1))
+    __shared__ uint32_t s_min[2][CA_WARPS];  // by the step's parity: each warp's earliest pending time
+    __shared__ uint32_t s_mark;       // tiles to queue, one bit each
+    __shared__ uint32_t s_first;      // earliest time they wait for
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t NONE = 0xffffffffu;
+    for (int i = tid; i < HCELLS; i += CA_THREADS) {
+        const int hx = i % HS, hy = (i / HS) % HS, hz = i / (HS * HS);
+        s_dir[i] = (uint8_t)((hz == 0 ? 0 : (hz > TS ? 18 : 9)) + (hy == 0 ? 0 : (hy > TS ? 6 : 3)) +
+                             (hx == 0 ? 0 : (hx > TS ? 2 : 1)));
+    }
+    // the thread's voxel: a warp's 32 voxels share no plane of the tile with more than a few of one another
+    const int q4 = (warp + 5 * (lane >> 2) + 3 * (lane & 3)) & 15;
+    const int lx = (q4 & 7) + 1, ly = 2 * (lane & 3) + (q4 >> 3) + 1, lz = (lane >> 2) + 1;
+    const int me = (lz * HS + ly) * HS + lx;
+    // lane -> neighbour (26 of the 32 lanes)
+    int off = 0, kind = 0;
+    if (lane < 26) {
+        const int c = lane < 13 ? lane : lane + 1;  // skip the centre of the 3x3x3 cube
+        const int dz = c / 9 - 1, dy = (c / 3) % 3 - 1, dx = c % 3 - 1;
+        off = (dz * HS + dy) * HS + dx;
+        kind = (dz != 0) + (dy != 0) + (dx != 0) - 1;
+    }
+    // everything above runs beside the round before (programmatic launch)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int n = T.counts[round % 3];
+    const u64 upto = (u64)__double_as_longlong(__dadd_rn(__hiloint2double((int)T.first[round % 3], -1), window));
+    if (blockIdx.x == 0 && tid == 0) {
+        T.counts[(round + 2) % 3] = 0;
+        T.first[(round + 2) % 3] = NONE;
+        if (n > 0) T.counts[3] = round + 1;
+    }
+    for (int it = blockIdx.x; it < n; it += gridDim.x) {
+        const int tile = T.list[(size_t)(round & 1) * T.cap + it];
+        const int tx0 = (tile % ntx) * TS, ty0 = ((tile / ntx) % nty) * TS, tz0 = (tile / (ntx * nty)) * TS;
+        __syncthreads();  // the previous tile's reads of the shared arrays are done
+        if (tid == 0) {
+            atomicAnd(&T.flags[tile >> 2], ~(1u << (8 * (tile & 3) + (round & 1))));
+            s_mark = 0;
+            s_first = NONE;
         }
-        s_b[hz][hy][hx] = b;
-        s_l[hz][hy][hx] = l;
-        s_ch[0][hz][hy][hx] = 0;
-        s_ch[1][hz][hy][hx] = 0;
-    }
-    __syncthreads();
-
-    const int lx = (tid & 7) + 1, ly = ((tid >> 3) & 7) + 1, lz0 = (tid >> 6) + 1;
-    unsigned long long orig[2];
-    uint8_t myl[2];
-    bool inside[2];
+        // stage tile + halo
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        int lz = lz0 + 4 * r;
-        orig[r] = s_b[lz][ly][lx];
-        myl[r] = s_l[lz][ly][lx];
-        inside[r] = (tx0 + lx - 1 < nx) && (ty0 + ly - 1 < ny) && (tz0 + lz - 1 < nz);
-    }
-
-    // sweep 0: pull from the 26 neighbours (the halo may carry new times from other tiles)
-    bool changed = false;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        if (!inside[r] || myl[r] == 0) continue;
-        const int lz = lz0 + 4 * r;
-        unsigned long long best = s_b[lz][ly][lx];
-        const double *lagd = lag + (size_t)myl[r] * 3;  // lag[src][dst=myl][k]
-#pragma unroll
-        for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-            for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-                for (int dx = -1; dx <= 1; ++dx) {
-                    if (dz == 0 && dy == 0 && dx == 0) continue;
-                    const uint8_t lu = s_l[lz + dz][ly + dy][lx + dx];
-                    if (lu == 0) continue;
-                    const unsigned long long bu = s_b[lz + dz][ly + dy][lx + dx];
-                    if (bu >= best) continue;
-                    const int k = (dz != 0) + (dy != 0) + (dx != 0);
-                    const double c = __dadd_rn(__longlong_as_double((long long)bu),
-                                               __ldg(lagd + (size_t)lu * nl1 * 3 + (k - 1)));
-                    const unsigned long long cb = (unsigned long long)__double_as_longlong(c);
-                    if (cb < best) best = cb;
-                }
-        if (best < s_b[lz][ly][lx]) {
-            s_b[lz][ly][lx] = best;
-            s_ch[0][lz][ly][lx] = 1;
-            changed = true;
+        for (int q = 0; q < 2; ++q) {
+            const int i = tid + q * CA_THREADS;
+            if (i >= HCELLS) break;
+            const int hx = i % HS, hy = (i / HS) % HS, hz = i / (HS * HS);
+            const int gx = tx0 + hx - 1, gy = ty0 + hy - 1, gz = tz0 + hz - 1;
+            u64 e = 2 * INF_BITS;
+            uint8_t l = 0;
+            if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && gz >= 0 && gz < nz) {
+                const size_t g = ((size_t)gz * ny + gy) * nx + gx;
+                l = layer_id(layers[g]);
+                const u64 v = at[g];
+                if (l) e = v;
+            }
+            s_e[i] = e;
+            s_l[i] = l;
         }
-    }
-    int iters = 1, cur = 0;
-    bool again = __syncthreads_or(changed);
-    // later sweeps: the voxels that improved push to their interior neighbours
-    while (again && iters < MAX_LOCAL_ITERS) {
-        changed = false;
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int lz = lz0 + 4 * r;
-            if (!inside[r] || myl[r] == 0 || !s_ch[cur][lz][ly][lx]) continue;
-            s_ch[cur][lz][ly][lx] = 0;
-            const unsigned long long bu = s_b[lz][ly][lx];
-            const double au = __longlong_as_double((long long)bu);
-            const double *lags = lag + (size_t)myl[r] * nl1 * 3;  // lag[src=myl][dst][k]
-#pragma unroll
-            for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-                for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        if (dz == 0 && dy == 0 && dx == 0) continue;
-                        const int wz = lz + dz, wy = ly + dy, wx = lx + dx;
-                        if (wz < 1 || wz > TS || wy < 1 || wy > TS || wx < 1 || wx > TS) continue;
-                        const uint8_t lw = s_l[wz][wy][wx];
-                        if (lw == 0) continue;
-                        const unsigned long long bw = s_b[wz][wy][wx];
-                        if (bu >= bw) continue;
-                        const int k = (dz != 0) + (dy != 0) + (dx != 0);
-                        const unsigned long long cb = (unsigned long long)__double_as_longlong(
-                            __dadd_rn(au, __ldg(lags + (size_t)lw * 3 + (k - 1))));
-                        if (cb < bw && cb < atomicMin(&s_b[wz][wy][wx], cb)) {
-                            s_ch[cur ^ 1][wz][wy][wx] = 1;
-                            changed = true;
+        __syncthreads();
+        const u64 orig = s_e[me];
+        const int myl = s_l[me];
+        u64 offered = orig & 1 ? ~0ULL : orig >> 1;  // the time that the voxel has offered
+        uint32_t mark = 0, first = NONE, sent = NONE;  // sent: earliest offer of the last step within the tile
+        // settling steps: every voxel with a pending time up to the horizon offers it; they end, as times only fall
+        for (;;) {
+            const u64 mine = s_e[me] >> 1;
+            const bool sel = mine != offered && mine <= upto;
+            // an offer made in the last step may have come too late for its target's read
+            if (!__syncthreads_or(sel || sent != NONE)) break;
+            sent = NONE;
+            if (sel) offered = mine;
+            for (unsigned b = __ballot_sync(0xffffffffu, sel); b; b &= b - 1) {
+                const int src = __ffs(b) - 1;
+                const u64 t = __shfl_sync(0xffffffffu, mine, src);
+                const int v = __shfl_sync(0xffffffffu, me, src) + off, lu = __shfl_sync(0xffffffffu, myl, src);
+                const int lv = s_l[v];
+                const u64 ev = s_e[v];
+                if (lane < 26 && lv && 2 * t < ev) {
+                    const u64 c = (u64)__double_as_longlong(__dadd_rn(
+                        __longlong_as_double((long long)t), __ldg(lag + ((size_t)lu * nl1 + lv) * 3 + kind)));
+                    const u64 ce = 2 * c + 1;
+                    if (ce < ev && ce < atomicMin(&s_e[v], ce)) {
+                        const int dir = s_dir[v];
+                        if (dir == 13) {
+                            if (c <= upto) sent = min(sent, (uint32_t)(c >> 32));
+                        } else {
+                            const int hx = v % HS, hy = (v / HS) % HS, hz = v / (HS * HS);
+                            atomicMin(&at[((size_t)(tz0 + hz - 1) * ny + (ty0 + hy - 1)) * nx + (tx0 + hx - 1)], ce);
+                            mark |= 1u << dir;
+                            first = min(first, (uint32_t)(c >> 32));
                         }
                     }
+                }
+            }
         }
-        cur ^= 1;
-        again = __syncthreads_or(changed);
-        ++iters;
-    }
-
-    // write back and flag neighbour tiles touched by changed boundary voxels
-    uint32_t mark = 0;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int lz = lz0 + 4 * r;
-        if (!inside[r] || myl[r] == 0) continue;
-        const unsigned long long v = s_b[lz][ly][lx];
-        if (v < orig[r]) {
-            size_t g = ((size_t)(tz0 + lz - 1) * ny + (ty0 + ly - 1)) * nx + (tx0 + lx - 1);
-            at[g] = __longlong_as_double((long long)v);
-            const int fz = (lz == 1) ? -1 : (lz == TS ? 1 : 0);
-            const int fy = (ly == 1) ? -1 : (ly == TS ? 1 : 0);
-            const int fx = (lx == 1) ? -1 : (lx == TS ? 1 : 0);
-            for (int a = 0; a <= (fz != 0); ++a)
-                for (int b = 0; b <= (fy != 0); ++b)
-                    for (int c = 0; c <= (fx != 0); ++c) {
-                        int dz = a ? fz : 0, dy = b ? fy : 0, dx = c ? fx : 0;
-                        if (dz || dy || dx) mark |= 1u << ((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
-                    }
+        // write back (a neighbour tile's block may have offered an earlier time meanwhile, and then has
+        // queued this tile); a tile with waiting voxels stays queued
+        const u64 mine = s_e[me] >> 1;
+        if (myl) {
+            const u64 e = 2 * mine + (mine != offered);
+            if (e != orig) atomicMin(&at[((size_t)(tz0 + lz - 1) * ny + (ty0 + ly - 1)) * nx + (tx0 + lx - 1)], e);
+            if (mine != offered) {
+                mark |= 1u << 13;
+                first = min(first, (uint32_t)(mine >> 32));
+            }
         }
-    }
-    if (again) mark |= 1u << 13;  // local iteration cap hit: run this tile again
-    // warp-level OR, then one shared atomic per warp
-    for (int o = 16; o > 0; o >>= 1) mark |= __shfl_xor_sync(0xffffffffu, mark, o);
-    if ((tid & 31) == 0 && mark) atomicOr(&s_mark, mark);
-    __syncthreads();
-    if (tid < 27) {
-        const uint32_t m = s_mark;
-        if (m & (1u << tid)) {
-            int dz = tid / 9 - 1, dy = (tid / 3) % 3 - 1, dx = tid % 3 - 1;
-            int tzz = tz0 / TS + dz, tyy = ty0 / TS + dy, txx = tx0 / TS + dx;
-            if (tzz >= 0 && tzz < ntz && tyy >= 0 && tyy < nty && txx >= 0 && txx < ntx)
-                next_flag[((size_t)tzz * nty + tyy) * ntx + txx] = 1;
+        mark = __reduce_or_sync(0xffffffffu, mark);
+        first = __reduce_min_sync(0xffffffffu, first);
+        if (lane == 0 && mark) {
+            atomicOr(&s_mark, mark);
+            atomicMin(&s_first, first);
         }
-    }
-}
-
-// A round with one block per active tile (the tile list's length is the grid).
-template <typename LT>
-__global__ void k_ca_round(int nz, int ny, int nx, int ntz, int nty, int ntx, const LT *__restrict__ layers,
-                           const double *__restrict__ lag, int nl1, double *__restrict__ at,
-                           const int32_t *__restrict__ active, uint8_t *__restrict__ next_flag) {
-    ca_tile<LT>(active[blockIdx.x], nz, ny, nx, ntz, nty, ntx, layers, lag, nl1, at, next_flag);
-}
-
-// A round over a device-resident tile list: a fixed grid walks the count_cur active tiles, so
-// rounds can be queued back to back without the host reading the count.  Block 0 clears the next
-// round's count, which only the compaction after this kernel adds to.
-__global__ void __launch_bounds__(CA_THREADS) k_ca_round_list(int nz, int ny, int nx, int ntz, int nty, int ntx,
-                                                              const uint8_t *__restrict__ layers,
-                                                              const double *__restrict__ lag, int nl1,
-                                                              double *__restrict__ at,
-                                                              const int32_t *__restrict__ active,
-                                                              const int32_t *__restrict__ count_cur,
-                                                              int32_t *__restrict__ count_next,
-                                                              uint8_t *__restrict__ next_flag) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *count_next = 0;
-    const int n = *count_cur;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
-        ca_tile<uint8_t>(active[i], nz, ny, nx, ntz, nty, ntx, layers, lag, nl1, at, next_flag);
-        __syncthreads();  // the next tile restages the shared arrays
-    }
-}
-
-// next_flag -> compact list (order irrelevant); clears the flags.
-__global__ void k_ca_compact(int ntiles, uint8_t *__restrict__ flag, int32_t *__restrict__ list,
-                             int32_t *__restrict__ count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool f = (i < ntiles) && flag[i];
-    const unsigned b = __ballot_sync(0xffffffffu, f);
-    int base = 0;
-    if ((threadIdx.x & 31) == 0 && b) base = atomicAdd(count, __popc(b));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (f) {
-        list[base + __popc(b & ((1u << (threadIdx.x & 31)) - 1))] = i;
-        flag[i] = 0;
+        __syncthreads();
+        if (tid < 27 && (s_mark >> tid) & 1u) {
+            const int tz = tz0 / TS + tid / 9 - 1, ty = ty0 / TS + (tid / 3) % 3 - 1, tx = tx0 / TS + tid % 3 - 1;
+            tile_append(T, (tz * nty + ty) * ntx + tx, round + 1);  // inside the grid: it holds a voxel
+        }
+        if (tid == 32 && s_mark) atomicMin(&T.first[(round + 1) % 3], s_first);
     }
 }
 
 __global__ void k_ca_init(size_t n, const uint8_t *__restrict__ layers, const uint8_t *__restrict__ start,
-                          double *__restrict__ at) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        double v = 0.0;
-        if (layers[i]) v = start[i] ? 1.0 : __longlong_as_double(0x7ff0000000000000LL);
-        at[i] = v;
-    }
-}
-
-__global__ void k_ca_finish(size_t n, double *__restrict__ at) {
+                          u64 *__restrict__ at) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        if (isinf(at[i])) at[i] = 0.0;  // unreachable voxels keep excitationDelay 0
+        at[i] = layers[i] ? (start[i] ? 2 * 0x3ff0000000000000ULL + 1 : 2 * INF_BITS) : 0;
 }
 
-// ------------------------------------------------------------------ bucketed relaxation
-// Dijkstra by time buckets (delta-stepping with a bucket width just below the smallest lag): the
-// voxels whose time falls into bucket k = floor(t / delta) are final once every earlier bucket has
-// been relaxed, because each of their predecessors on a shortest path is at least one lag, so more
-// than delta, earlier.  Bucket k is one launch: a warp per queued entry (cell, layer, time), one
-// lane per neighbour, offers fl(at(u) + lag) with a 64-bit atomicMin on the time bits; an improved
-// neighbour is queued in the bucket of its new time with its new time (warp-aggregated appends per
-// bucket).  A cell can be queued more than once: an entry whose cell has improved since offers a
-// later time than the one already offered from the cell's better entry, which was relaxed in an
-// earlier bucket or in this one, so it changes nothing.  Offers reach at most
-// ceil(max lag / delta) + 1 buckets ahead, so the lists form a ring of that many slots; the slot
-// of bucket k - 1 is emptied by bucket k's launch (nothing can still be queued there).
-struct QEntry {
-    int32_t cell, layer;
-    unsigned long long bits;
-};
-struct BucketArgs {
-    int nz, ny, nx;
-    const uint8_t *layers;
-    const double *lag;  // [nl1][nl1][3]
-    int nl1;
-    unsigned long long *at;  // time bits per cell (non-negative doubles order like their bits)
-    QEntry *lists;           // [ring][cap]
-    int32_t *counts;         // [ring]
-    int32_t *overflow;
-    int ring, cap;
-    double inv_delta;
-};
-
-__device__ __forceinline__ int bucket_of(double t, double inv_delta) {
-    return (int)floor(__dmul_rn(t, inv_delta));
-}
-
-__global__ void k_ca_bucket_init(size_t n, const uint8_t *__restrict__ layers, const uint8_t *__restrict__ start,
-                                 BucketArgs A) {
+// entries -> times; unreachable voxels keep excitationDelay 0
+__global__ void k_ca_finish(size_t n, u64 *__restrict__ at) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        double v = 0.0;
-        if (layers[i]) v = start[i] ? 1.0 : __longlong_as_double(0x7ff0000000000000LL);
-        const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-        A.at[i] = bits;
-        if (layers[i] && start[i]) {
-            const int b = bucket_of(1.0, A.inv_delta);
-            const int idx = atomicAdd(&A.counts[b % A.ring], 1);
-            if (idx < A.cap) A.lists[(size_t)(b % A.ring) * A.cap + idx] = QEntry{(int32_t)i, (int32_t)layers[i], bits};
-            else atomicOr(A.overflow, 1);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) k_ca_bucket(int k, BucketArgs A) {
-    const int slot = k % A.ring;
-    if (blockIdx.x == 0 && threadIdx.x == 0) A.counts[(k + A.ring - 1) % A.ring] = 0;
-    const int n = min(A.counts[slot], A.cap);
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    // lane -> neighbour offset (26 of the 32 lanes)
-    int dz = 0, dy = 0, dx = 0, kind = 1;
-    const bool nb = lane < 26;
-    if (nb) {
-        const int c = lane < 13 ? lane : lane + 1;  // skip the centre of the 3x3x3 cube
-        dz = c / 9 - 1;
-        dy = (c / 3) % 3 - 1;
-        dx = c % 3 - 1;
-        kind = (dz != 0) + (dy != 0) + (dx != 0);
-    }
-    // the loop bound is uniform over the warp, so every lane reaches the warp votes below
-    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n; e += warps) {
-        const QEntry q = A.lists[(size_t)slot * A.cap + e];
-        const int u = q.cell;
-        const int x = u % A.nx, y = (u / A.nx) % A.ny, z = u / (A.nx * A.ny);
-        const int vz = z + dz, vy = y + dy, vx = x + dx;
-        const bool inside = nb && vz >= 0 && vz < A.nz && vy >= 0 && vy < A.ny && vx >= 0 && vx < A.nx;
-        const int v = inside ? (vz * A.ny + vy) * A.nx + vx : u;
-        const uint8_t lv = inside ? A.layers[v] : 0;
-        const unsigned long long bv = inside ? A.at[v] : 0ull;
-        bool improved = false;
-        double c = 0.0;
-        if (lv != 0 && q.bits < bv) {
-            c = __dadd_rn(__longlong_as_double((long long)q.bits),
-                          __ldg(A.lag + ((size_t)q.layer * A.nl1 + lv) * 3 + (kind - 1)));
-            const unsigned long long cb = (unsigned long long)__double_as_longlong(c);
-            improved = cb < bv && cb < atomicMin(&A.at[v], cb);
-        }
-        // queue the improved neighbours: one atomic per bucket and warp
-        const int b = improved ? bucket_of(c, A.inv_delta) : -1;
-        const unsigned same = __match_any_sync(0xffffffffu, b);
-        if (improved) {
-            const int leader = __ffs(same) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(&A.counts[b % A.ring], __popc(same));
-            base = __shfl_sync(same, base, leader);
-            const int idx = base + __popc(same & ((1u << lane) - 1u));
-            if (idx < A.cap)
-                A.lists[(size_t)(b % A.ring) * A.cap + idx] =
-                    QEntry{v, (int32_t)lv, (unsigned long long)__double_as_longlong(c)};
-            else
-                atomicOr(A.overflow, 1);
-        }
-    }
-}
-
-__global__ void k_ca_bucket_finish(size_t n, const unsigned long long *__restrict__ bits, double *__restrict__ at) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const double v = __longlong_as_double((long long)bits[i]);
-        at[i] = isinf(v) ? 0.0 : v;  // unreachable voxels keep excitationDelay 0
+        const u64 t = at[i] >> 1;
+        at[i] = t == INF_BITS ? 0 : t;
     }
 }
 
 }  // namespace
 
-// Bucketed relaxation when the smallest lag allows it (returns false to fall back to the tile
-// rounds: a zero lag, a time span of too many buckets, or a full bucket list).
-bool ca_run_buckets(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const uint8_t *d_start,
-                    const std::vector<double> &lag_h, int nl1, const double *d_lag, double *d_at, int64_t nvox,
-                    int round_cap, int sm_count, CaResult &res) {
-    double min_lag = INFINITY, max_lag = 0;
+// The lists over `ctrl` (CA_CTRL_WORDS words) and its words before round 0: the stimulus (time 1.0)
+// pending in n_start tiles.
+static TileLists tile_lists(int32_t *ctrl, uint32_t *flags, int32_t *list, int cap) {
+    TileLists T;
+    T.counts = ctrl;
+    T.first = reinterpret_cast<uint32_t *>(ctrl + 4);
+    T.flags = flags;
+    T.list = list;
+    T.cap = cap;
+    return T;
+}
+static void first_round(int32_t (&ctrl)[CA_CTRL_WORDS], int32_t n_start) {
+    std::fill(ctrl, ctrl + CA_CTRL_WORDS, 0);
+    ctrl[0] = n_start;
+    ctrl[4] = 0x3ff00000;  // high word of 1.0
+    ctrl[5] = ctrl[6] = -1;
+}
+
+// The width of a round, 5 of the largest lag between present layers: in a narrower one the rounds' fixed
+// cost shows (launch, staging, write-back), in a wider one the wave leaves the tile and its successors
+// wait.  160^3 heart with lags 1, 2, 2 ms: 1.06, 1.03, 1.02, 1.04, 1.15, 1.69 ms at 2.5, 4, 6, 8, 16 and
+// without an end; 256^3: 2.47, 2.43, 2.50, 2.58, 3.3, 7.7 ms.
+static double round_window(const double *lag, int nl1, const char *present) {
+    double hi = 0.0;
     for (int a = 1; a < nl1; ++a)
         for (int b = 1; b < nl1; ++b)
-            for (int k = 0; k < 3; ++k) {
-                const double l = lag_h[((size_t)a * nl1 + b) * 3 + k];
-                min_lag = std::min(min_lag, l);
-                max_lag = std::max(max_lag, l);
-            }
-    if (!(min_lag >= 0.05) || !std::isfinite(max_lag)) return false;
-    // a bucket width just below the smallest lag keeps a margin far above FP64 rounding
-    const double delta = min_lag * (1.0 - 1e-6);
-    const int ring = (int)std::ceil(max_lag / delta) + 3;
-    if (ring > 256) return false;
-    const size_t n = (size_t)nz * ny * nx;
-    // bucket indices stay far inside int: the latest time is below 1 + n * max_lag
-    if ((1.0 + (double)n * max_lag) / delta > 1e9) return false;
-    // per bucket slot; a cell can be queued more than once, a full slot falls back to the tile rounds
-    const int cap = (int)std::min<int64_t>(std::max<int64_t>(65536, nvox / 2), INT32_MAX / 32);
-    DBuf<unsigned long long> bits;
-    DBuf<QEntry> lists;
-    DBuf<int32_t> counts;
-    bits.alloc(n);
-    lists.alloc((size_t)ring * cap);
-    counts.alloc(ring + 1);  // + the overflow flag
-    BucketArgs A;
-    A.nz = nz;
-    A.ny = ny;
-    A.nx = nx;
-    A.layers = d_layers;
-    A.lag = d_lag;
-    A.nl1 = nl1;
-    A.at = bits.p;
-    A.lists = lists.p;
-    A.counts = counts.p;
-    A.overflow = counts.p + ring;
-    A.ring = ring;
-    A.cap = cap;
-    A.inv_delta = 1.0 / delta;
-    EKG_CUDA(cudaMemsetAsync(counts.p, 0, (ring + 1) * sizeof(int32_t), s));
-    cudaEvent_t e0, e1;
-    EKG_CUDA(cudaEventCreate(&e0));
-    EKG_CUDA(cudaEventCreate(&e1));
-    struct Events {
-        cudaEvent_t a, b;
-        ~Events() {
-            cudaEventDestroy(a);
-            cudaEventDestroy(b);
+            if (present[a] && present[b]) hi = std::max(hi, lag[((size_t)a * nl1 + b) * 3]);
+    return 5.0 * hi;
+}
+
+// Queues rounds in chunks until a round has no tile; the host reads the counts once per chunk (rounds
+// after convergence find an empty list).  `read` copies the four counters to the host, waiting.
+template <typename LT, class Read>
+static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, const double *lag, int nl1, double w,
+                      u64 *at, const TileLists &T, int cap, int sm_count, Read read) {
+    const int ntz = (nz + TS - 1) / TS, nty = (ny + TS - 1) / TS, ntx = (nx + TS - 1) / TS;
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::max(1, std::min(ntz * nty * ntx, 3 * std::max(1, sm_count))));
+    cfg.blockDim = dim3(CA_THREADS);
+    cfg.stream = s;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = 1;
+    constexpr int CHUNK = 12;
+    int32_t h[4];
+    for (int r = 0;;) {
+        const int end = std::min(cap, r + CHUNK);
+        for (; r < end; ++r) {
+            EKG_CUDA(cudaLaunchKernelEx(&cfg, k_ca_round<LT>, r, nz, ny, nx, ntz, nty, ntx, layers, lag, nl1, w, at, T));
         }
-    } ev{e0, e1};
-    EKG_CUDA(cudaEventRecord(e0, s));
-    k_ca_bucket_init<<<1024, 256, 0, s>>>(n, d_layers, d_start, A);
-    EKG_CUDA(cudaGetLastError());
-    // buckets before the first start time are empty
-    int k = (int)std::floor(1.0 * A.inv_delta);
-    const int grid = std::max(1, sm_count) * 8;
-    std::vector<int32_t> h(ring + 1);
-    int32_t *hc = nullptr;
-    EKG_CUDA(cudaMallocHost(&hc, (ring + 1) * sizeof(int32_t)));
-    struct Pinned {
-        int32_t *p;
-        ~Pinned() { cudaFreeHost(p); }
-    } pin{hc};
-    // every cell settles at most once per bucket it is queued in; more buckets than cells plus the
-    // ring means the queues never drain
-    const int64_t kmax = round_cap > 0 ? (int64_t)round_cap : (int64_t)n + 4LL * ring + 1024;
-    constexpr int CHUNK = 16;
-    int steps = 0;
-    for (;;) {
-        for (int i = 0; i < CHUNK; ++i, ++k, ++steps) {
-            if (steps >= kmax) throw Error{EKG_ERR_CA_NOT_CONVERGED, "activation-time relaxation did not converge"};
-            k_ca_bucket<<<grid, 256, 0, s>>>(k, A);
-            EKG_CUDA(cudaGetLastError());
-        }
-        EKG_CUDA(cudaMemcpyAsync(hc, counts.p, (ring + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        EKG_CUDA(cudaStreamSynchronize(s));
-        if (hc[ring]) return false;  // a bucket list overflowed: the tile rounds redo it
-        // the slot of the last bucket launched holds processed entries; any other non-empty slot
-        // is a bucket still to come
-        bool pending = false;
-        for (int r = 0; r < ring; ++r)
-            if (r != (k - 1) % ring && hc[r] > 0) pending = true;
-        if (!pending) break;
+        read(h);
+        if (h[r % 3] == 0) return h[3];
+        if (r >= cap) throw Error{EKG_ERR_CA_NOT_CONVERGED, "activation-time relaxation did not converge"};
     }
-    k_ca_bucket_finish<<<1024, 256, 0, s>>>(n, bits.p, d_at);
-    EKG_CUDA(cudaGetLastError());
-    EKG_CUDA(cudaEventRecord(e1, s));
-    EKG_CUDA(cudaEventSynchronize(e1));
-    EKG_CUDA(cudaEventElapsedTime(&res.ms, e0, e1));
-    res.rounds = steps;
-    res.buckets = true;
-    return true;
 }
 
 CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const uint8_t *d_start,
-                const std::vector<int32_t> &start_tiles, int nl1, const double *d_lag, double *d_at, int round_cap,
+                const std::vector<int32_t> &start_tiles, const std::vector<double> &lag_h,
+                const std::vector<char> &present, int nl1, const double *d_lag, double *d_at, int round_cap,
                 int sm_count) {
     CaResult res;
     const int ntz = (nz + TS - 1) / TS, nty = (ny + TS - 1) / TS, ntx = (nx + TS - 1) / TS;
     const int ntiles = ntz * nty * ntx;
-    const size_t n = (size_t)nz * ny * nx;
-    DBuf<int32_t> lists, count;
-    DBuf<uint8_t> flag;
-    lists.alloc(2 * (size_t)ntiles);
-    count.alloc(2);
-    flag.alloc(ntiles);
-    int32_t *list[2] = {lists.p, lists.p + ntiles};
+    const size_t n = (size_t)nz * ny * nx, nflag = (size_t)(ntiles + 3) / 4;
+    DBuf<int32_t> buf;  // control words, flags, two lists
+    buf.alloc(CA_CTRL_WORDS + nflag + 2 * (size_t)ntiles);
+    const TileLists T = tile_lists(buf.p, reinterpret_cast<uint32_t *>(buf.p + CA_CTRL_WORDS),
+                                   buf.p + CA_CTRL_WORDS + nflag, ntiles);
     const int32_t n_start = (int32_t)start_tiles.size();
-    EKG_CUDA(cudaMemsetAsync(flag.p, 0, ntiles, s));
-    EKG_CUDA(cudaMemcpyAsync(list[0], start_tiles.data(), start_tiles.size() * sizeof(int32_t),
+    EKG_CUDA(cudaMemsetAsync(T.flags, 0, nflag * sizeof(int32_t), s));
+    int32_t ctrl[CA_CTRL_WORDS];
+    first_round(ctrl, n_start);
+    EKG_CUDA(cudaMemcpyAsync(buf.p, ctrl, sizeof(ctrl), cudaMemcpyHostToDevice, s));
+    EKG_CUDA(cudaMemcpyAsync(T.list, start_tiles.data(), start_tiles.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(count.p, &n_start, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    cudaEvent_t e0, e1;
-    EKG_CUDA(cudaEventCreate(&e0));
-    EKG_CUDA(cudaEventCreate(&e1));
-    EKG_CUDA(cudaEventRecord(e0, s));
-    k_ca_init<<<1024, 256, 0, s>>>(n, d_layers, d_start, d_at);
-    EKG_CUDA(cudaGetLastError());
-    // Every round finalises at least the next tile along each shortest path; a path can
-    // cross a tile boundary at most once per hop, so this cap is far above any real heart.
-    const int cap = round_cap > 0 ? round_cap : 16 * (ntz + nty + ntx) + 4 * ntiles + 64;
-    // Rounds are queued in chunks (round over the device-resident list, then its compaction); the
-    // host reads the active count once per chunk.  Rounds after convergence find an empty list.
-    constexpr int CHUNK = 8;
-    int blocks_per_sm = 0;
-    EKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_ca_round_list, CA_THREADS, 0));
-    const int grid = std::max(1, std::min(ntiles, std::max(1, blocks_per_sm) * std::max(1, sm_count)));
-    int32_t *h_count = nullptr;
-    EKG_CUDA(cudaMallocHost(&h_count, sizeof(int32_t)));
-    int n_active = n_start, r = 0;
-    while (n_active > 0) {
-        if (r >= cap) {
-            cudaFreeHost(h_count);
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            throw Error{EKG_ERR_CA_NOT_CONVERGED, "activation-time relaxation did not converge"};
+    struct Events {
+        cudaEvent_t a = nullptr, b = nullptr;
+        ~Events() {
+            if (a) cudaEventDestroy(a);
+            if (b) cudaEventDestroy(b);
         }
-        const int chunk = std::min(CHUNK, cap - r);
-        for (int k = 0; k < chunk; ++k, ++r) {
-            const int c = r & 1;
-            k_ca_round_list<<<grid, CA_THREADS, 0, s>>>(nz, ny, nx, ntz, nty, ntx, d_layers, d_lag, nl1, d_at,
-                                                       list[c], count.p + c, count.p + (c ^ 1), flag.p);
-            EKG_CUDA(cudaGetLastError());
-            k_ca_compact<<<(ntiles + 255) / 256, 256, 0, s>>>(ntiles, flag.p, list[c ^ 1], count.p + (c ^ 1));
-            EKG_CUDA(cudaGetLastError());
-        }
-        EKG_CUDA(cudaMemcpyAsync(h_count, count.p + (r & 1), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        EKG_CUDA(cudaStreamSynchronize(s));
-        n_active = *h_count;
-    }
-    cudaFreeHost(h_count);
-    res.rounds = r;
-    k_ca_finish<<<1024, 256, 0, s>>>(n, d_at);
+    } ev;
+    EKG_CUDA(cudaEventCreate(&ev.a));
+    EKG_CUDA(cudaEventCreate(&ev.b));
+    EKG_CUDA(cudaEventRecord(ev.a, s));
+    u64 *entries = reinterpret_cast<u64 *>(d_at);
+    k_ca_init<<<1024, 256, 0, s>>>(n, d_layers, d_start, entries);
     EKG_CUDA(cudaGetLastError());
-    EKG_CUDA(cudaEventRecord(e1, s));
-    EKG_CUDA(cudaEventSynchronize(e1));
-    EKG_CUDA(cudaEventElapsedTime(&res.ms, e0, e1));
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    // every round settles at least the voxels with the earliest pending time for good
+    const int cap = round_cap > 0 ? round_cap : (int)std::min<size_t>(n, INT32_MAX / 2) + 64;
+    res.rounds = run_rounds(s, nz, ny, nx, d_layers, d_lag, nl1, round_window(lag_h.data(), nl1, present.data()),
+                            entries, T, cap, sm_count, [&](int32_t *h) {
+                                EKG_CUDA(cudaMemcpyAsync(h, T.counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+                                EKG_CUDA(cudaStreamSynchronize(s));
+                            });
+    k_ca_finish<<<1024, 256, 0, s>>>(n, entries);
+    EKG_CUDA(cudaGetLastError());
+    EKG_CUDA(cudaEventRecord(ev.b, s));
+    EKG_CUDA(cudaEventSynchronize(ev.b));
+    EKG_CUDA(cudaEventElapsedTime(&res.ms, ev.a, ev.b));
     return res;
 }
-
-
 
 // ------------------------------------------------------------------ no-allocation entry point
 // ekg_activation_noalloc: the same relaxation for callers that cannot allocate device memory
@@ -541,8 +347,8 @@ constexpr int NOALLOC_MAX_TILES = 65536;  // 8x8x8 tiles, e.g. a 320^3 grid
 constexpr int NOALLOC_MAX_LAYER = 31;     // highest layer id (lag table 32 x 32 x 3)
 struct NoAllocScratch {
     int32_t list[2][NOALLOC_MAX_TILES];
-    uint8_t flag[NOALLOC_MAX_TILES];
-    int32_t count;
+    uint32_t flag[NOALLOC_MAX_TILES / 4];  // one byte per tile (TileLists)
+    int32_t ctrl[CA_CTRL_WORDS];
     int32_t nstart;
     uint32_t layer_mask;
     int32_t bad;
@@ -576,17 +382,17 @@ __global__ void k_na_validate(size_t n, const int32_t *__restrict__ layers, NoAl
 }
 
 __global__ void k_na_init(int nz, int ny, int nx, int nty, int ntx, const int32_t *__restrict__ layers,
-                          double *__restrict__ at, uint8_t *__restrict__ flag) {
+                          u64 *__restrict__ at, TileLists T) {
     const size_t n = (size_t)nz * ny * nx;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int32_t v = layers[i];
-        double a = 0.0;
+        u64 a = 0;
         if (v < 0) {
-            a = 1.0;
+            a = 2 * 0x3ff0000000000000ULL + 1;
             const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
-            flag[((size_t)(z / TS) * nty + (y / TS)) * ntx + (x / TS)] = 1;
+            tile_append(T, ((z / TS) * nty + (y / TS)) * ntx + (x / TS), 0);
         } else if (v > 0) {
-            a = __longlong_as_double(0x7ff0000000000000LL);
+            a = 2 * INF_BITS;
         }
         at[i] = a;
     }
@@ -621,17 +427,16 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
         NoAllocScratch *sc = noalloc_scratch();
         const size_t n = (size_t)nz * ny * nx;
         cudaStream_t s = 0;
-        // clear what must start at zero: flags, counters, layer mask
-        EKG_CUDA(cudaMemsetAsync(sc->flag, 0, sizeof(sc->flag), s));
-        EKG_CUDA(cudaMemsetAsync(&sc->count, 0, 4 * sizeof(int32_t), s));
+        // clear what must start at zero: flags, counters, layer mask (they are contiguous)
+        EKG_CUDA(cudaMemsetAsync(sc->flag, 0, offsetof(NoAllocScratch, lag) - offsetof(NoAllocScratch, flag), s));
         k_na_validate<<<1024, 256, 0, s>>>(n, d_layers, sc);
         EKG_CUDA(cudaGetLastError());
         struct {
-            int32_t count, nstart;
+            int32_t nstart;
             uint32_t mask;
             int32_t bad;
         } hdr;
-        EKG_CUDA(cudaMemcpy(&hdr, &sc->count, sizeof(hdr), cudaMemcpyDeviceToHost));
+        EKG_CUDA(cudaMemcpy(&hdr, &sc->nstart, sizeof(hdr), cudaMemcpyDeviceToHost));
         EKG_CHECK(!hdr.bad, EKG_ERR_BAD_INPUT, "layer ids must be at most 31 for ekg_activation_noalloc");
         EKG_CHECK(hdr.nstart > 0, EKG_ERR_NO_START, "Could not find starting point for excitation sequence");
         int nl = 0;
@@ -642,6 +447,8 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
                     throw Error{EKG_ERR_TRANSFER, "transfer (conduction) matrix does not define layer " + std::to_string(a)};
             }
         const int nl1 = nl + 1;
+        char present[NOALLOC_MAX_LAYER + 1];
+        for (int a = 0; a <= NOALLOC_MAX_LAYER; ++a) present[a] = (hdr.mask >> a) & 1u;
         double lag[(NOALLOC_MAX_LAYER + 1) * (NOALLOC_MAX_LAYER + 1) * 3];
         for (int i = 0; i < nl1 * nl1 * 3; ++i) lag[i] = 0.0;
         for (int a = 1; a <= nl; ++a)
@@ -657,28 +464,21 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
                 }
             }
         EKG_CUDA(cudaMemcpy(sc->lag, lag, (size_t)nl1 * nl1 * 3 * sizeof(double), cudaMemcpyHostToDevice));
-        k_na_init<<<1024, 256, 0, s>>>(nz, ny, nx, nty, ntx, d_layers, d_at, sc->flag);
+        const TileLists T = tile_lists(sc->ctrl, sc->flag, sc->list[0], NOALLOC_MAX_TILES);
+        int32_t ctrl[CA_CTRL_WORDS];
+        first_round(ctrl, 0);  // k_na_init appends the stimulus tiles
+        EKG_CUDA(cudaMemcpy(sc->ctrl, ctrl, sizeof(ctrl), cudaMemcpyHostToDevice));
+        u64 *entries = reinterpret_cast<u64 *>(d_at);
+        k_na_init<<<1024, 256, 0, s>>>(nz, ny, nx, nty, ntx, d_layers, entries, T);
         EKG_CUDA(cudaGetLastError());
-        int32_t *cur = sc->list[0], *nxt = sc->list[1];
-        k_ca_compact<<<(unsigned)((ntiles + 255) / 256), 256, 0, s>>>((int)ntiles, sc->flag, cur, &sc->count);
-        EKG_CUDA(cudaGetLastError());
-        int32_t n_active = 0;
-        EKG_CUDA(cudaMemcpy(&n_active, &sc->count, sizeof(int32_t), cudaMemcpyDeviceToHost));
-        const int cap = 16 * (ntz + nty + ntx) + 4 * (int)ntiles + 64;
-        int rounds = 0;
-        while (n_active > 0) {
-            EKG_CHECK(rounds < cap, EKG_ERR_CA_NOT_CONVERGED, "activation-time relaxation did not converge");
-            k_ca_round<int32_t><<<n_active, CA_THREADS, 0, s>>>(nz, ny, nx, ntz, nty, ntx, d_layers, sc->lag, nl1,
-                                                               d_at, cur, sc->flag);
-            EKG_CUDA(cudaGetLastError());
-            EKG_CUDA(cudaMemsetAsync(&sc->count, 0, sizeof(int32_t), s));
-            k_ca_compact<<<(unsigned)((ntiles + 255) / 256), 256, 0, s>>>((int)ntiles, sc->flag, nxt, &sc->count);
-            EKG_CUDA(cudaGetLastError());
-            EKG_CUDA(cudaMemcpy(&n_active, &sc->count, sizeof(int32_t), cudaMemcpyDeviceToHost));
-            std::swap(cur, nxt);
-            ++rounds;
-        }
-        k_ca_finish<<<1024, 256, 0, s>>>(n, d_at);
+        int dev = 0, sm_count = 0;
+        EKG_CUDA(cudaGetDevice(&dev));
+        EKG_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
+        const int rounds = run_rounds(s, nz, ny, nx, d_layers, sc->lag, nl1, round_window(lag, nl1, present), entries, T,
+                                      (int)std::min<size_t>(n, INT32_MAX / 2) + 64, sm_count, [&](int32_t *h) {
+                                          EKG_CUDA(cudaMemcpy(h, T.counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost));
+                                      });
+        k_ca_finish<<<1024, 256, 0, s>>>(n, entries);
         EKG_CUDA(cudaGetLastError());
         EKG_CUDA(cudaStreamSynchronize(s));
         if (rounds_out) *rounds_out = rounds;

@@ -21,9 +21,6 @@ struct ekg_engine {
     // rounds after which the activation-time relaxation gives up with EKG_ERR_CA_NOT_CONVERGED
     // (0 = the default bound from the grid size; EKG_CA_ROUND_CAP sets it, e.g. to test that error)
     int ca_round_cap = 0;
-    // activation-time relaxation: 0 = by time buckets where the lags allow it (else tile rounds),
-    // 1 = tile rounds always (EKG_CA=tiles)
-    int ca_mode = 0;
     // autotuning of the batched form's launch shapes: EKG_TUNE=1 tunes every new pass shape on its
     // first pass (ekg_heart_tune does it on request); EKG_TUNE_CACHE names a file that keeps the
     // choices across processes
@@ -197,7 +194,6 @@ struct ekg_heart {
     int64_t ncell = 0, nvox = 0, naps = 0;
     double start = 0, length = 0, dt = 1;
     int ca_rounds = 0;
-    bool ca_buckets = false;  // the relaxation ran by time buckets (else tile rounds)
     double ca_ms = 0, setup_ms = 0;
     std::vector<double> t;            // time axis
     std::vector<double> leads0;       // loaded lead positions (z,y,x)

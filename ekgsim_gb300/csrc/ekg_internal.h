@@ -123,18 +123,15 @@ struct DBuf {
 
 // ------------------------------------------------------------------ CA (ca.cu)
 struct CaResult {
-    int rounds = 0;        // tile rounds, or bucket launches of the bucketed relaxation
+    int rounds = 0;  // rounds that had a tile
     float ms = 0.f;
-    bool buckets = false;  // the bucketed relaxation ran
 };
-// Bucketed relaxation (Dijkstra by time buckets); false when it does not apply and ca_run must run.
-bool ca_run_buckets(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const uint8_t *d_start,
-                    const std::vector<double> &lag_h, int nl1, const double *d_lag, double *d_at, int64_t nvox,
-                    int round_cap, int sm_count, CaResult &res);
 // layers_u8: stripped layer per cell; start flags in `is_start`; lag: [nl1][nl1][3] FP64 with
-// lag[s][d][k-1] = T[s][d] * sqrt(k).  at_out: FP64 per cell (0 for empty / unreachable).
+// lag[s][d][k-1] = T[s][d] * sqrt(k) (lag_h the same on the host, present[layer] != 0 where the heart has
+// the layer).  at_out: FP64 per cell (0 for empty / unreachable).
 CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const uint8_t *d_start,
-                const std::vector<int32_t> &start_tiles, int nl1, const double *d_lag, double *d_at, int round_cap,
+                const std::vector<int32_t> &start_tiles, const std::vector<double> &lag_h,
+                const std::vector<char> &present, int nl1, const double *d_lag, double *d_at, int round_cap,
                 int sm_count);
 
 // ------------------------------------------------------------------ ECG kernels (ecg.cu)

@@ -361,17 +361,10 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
         h->at_cells.alloc(n);
         EKG_CUDA(cudaMemcpyAsync(ds.p, st.data(), n, cudaMemcpyHostToDevice, s));
         EKG_CUDA(cudaMemcpyAsync(dlag.p, lag.data(), lag.size() * 8, cudaMemcpyHostToDevice, s));
-        int64_t nvox_h = 0;
-        for (int64_t i = 0; i < n; ++i) nvox_h += lay[i] != 0;
-        CaResult r;
-        if (h->eng->ca_mode == 1 ||
-            !ca_run_buckets(s, d->nz, d->ny, d->nx, dl.p, ds.p, lag, nl1, dlag.p, h->at_cells.p, nvox_h,
-                            h->eng->ca_round_cap, h->sm_count, r))
-            r = ca_run(s, d->nz, d->ny, d->nx, dl.p, ds.p, start_tiles, nl1, dlag.p, h->at_cells.p,
-                       h->eng->ca_round_cap, h->sm_count);
+        const CaResult r = ca_run(s, d->nz, d->ny, d->nx, dl.p, ds.p, start_tiles, lag, present, nl1, dlag.p,
+                                  h->at_cells.p, h->eng->ca_round_cap, h->sm_count);
         h->ca_rounds = r.rounds;
         h->ca_ms = r.ms;
-        h->ca_buckets = r.buckets;
         EKG_CUDA(cudaStreamSynchronize(s));
     }
     h->at_host.clear();  // copied to the host on first use (ensure_at_host)
@@ -1908,7 +1901,6 @@ int ekg_engine_create(int device, ekg_engine **out) {
         if (const char *v = std::getenv("EKG_BATCH_CTAS")) e->batch_ctas = std::atoi(v);
         if (const char *v = std::getenv("EKG_GRAPHS")) e->graphs = std::string(v) != "0";
         if (const char *v = std::getenv("EKG_CA_ROUND_CAP")) e->ca_round_cap = std::max(0, std::atoi(v));
-        if (const char *v = std::getenv("EKG_CA")) e->ca_mode = std::string(v) == "tiles" ? 1 : 0;
         if (const char *v = std::getenv("EKG_TUNE")) e->tune = std::string(v) == "1";
         if (const char *v = std::getenv("EKG_TUNE_CACHE")) e->tune_cache = v;
         EKG_CUDA(cudaSetDevice(device));
@@ -1967,7 +1959,7 @@ int ekg_heart_get_info(ekg_heart *h, ekg_heart_info *info) {
         info->device_bytes = heart_device_bytes(h);
         info->ca_ms = h->ca_ms;
         info->setup_ms = h->setup_ms;
-        info->ca_buckets = h->ca_buckets ? 1 : 0;
+        info->ca_buckets = 0;
     });
 }
 

@@ -86,12 +86,11 @@ typedef struct {
     int32_t n_layers;          /* highest layer id */
     int32_t n_leads;
     int32_t steps;             /* ceil(length / dt) */
-    int32_t ca_rounds;         /* steps of the activation relaxation: time buckets, or tile rounds
-                                * where the lags do not allow buckets (a zero lag) */
+    int32_t ca_rounds;         /* rounds of the activation relaxation over tiles of 8x8x8 cells */
     int64_t device_bytes;      /* device memory held by this heart */
     double ca_ms;              /* device time of the activation relaxation */
     double setup_ms;           /* host wall time of ekg_heart_create */
-    int32_t ca_buckets;        /* 1: the relaxation ran by time buckets, 0: by tile rounds (or loaded) */
+    int32_t ca_buckets;        /* always 0: kept for the layout (1 meant a relaxation by time buckets) */
 } ekg_heart_info;
 
 /* Upload a heart, compute its activation times on the device (bit-exact FP64 equivalent of

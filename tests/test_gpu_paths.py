@@ -1,0 +1,81 @@
+"""Kernel variants at the sizes where they can go wrong: edges of tiles, remainders, ties, extremes."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from ekgsim_gb300 import synth
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+ECG_TOL = 1e-4  # the engine's bar against the FP64 oracle (rel-L2 over leads x steps)
+
+
+@pytest.fixture(scope="module")
+def engine():
+    from ekgsim_gb300.engine import Engine
+    e = Engine(0)
+    yield e
+    e.close()
+
+
+def rel_l2(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("shape,delays", [
+    ((8, 8, 8), [1, 2, 2]),           # one tile
+    ((9, 16, 17), [1, 2, 2]),         # one cell over a tile, exact tiles
+    ((1, 70, 3), [0.3, 3, 1]),        # a strip through many tiles
+    ((24, 23, 25), [0, 2, 1]),        # a zero delay: ties within a step
+    ((24, 23, 25), [1e-9, 40, 0.7]),  # lags below the resolution of a time's high word
+    ((31, 33, 32), [1.37, 0.71, 2.9]),
+    ((40, 40, 9), [300, 0.5, 2]),     # most of a round's horizon empty
+])
+def test_activation_tiles(engine, shape, delays):
+    """Activation times bit-exact against the oracle, through the heart's set-up and in caller-owned buffers:
+    random layers with holes, two stimuli, tiles cut by the grid's edge."""
+    import torch
+    from ekgsim_gb300 import _lib as L
+    from ekgsim_gb300.engine import Heart
+    rng = np.random.Generator(np.random.PCG64(shape[0] * 100 + shape[2]))
+    grid = rng.integers(0, 4, size=shape).astype(np.int32)
+    grid[0, 0, 0] = -1
+    grid[-1, shape[1] // 2, -1] = -3
+    tm = synth.transfer_matrix(3, delays)
+    ref, _ = O.activation(grid, tm)
+    h = Heart.create(engine, grid, tm, np.array([[90.0, 95.0, 100.0]]), "3D4", 0.0, 10.0, 1.0)
+    assert np.array_equal(h.activation().view(np.int64), ref.view(np.int64))
+    h.close()
+    layers = torch.from_numpy(grid).cuda()
+    at = torch.full(shape, -7.0, dtype=torch.float64, device="cuda")
+    t = np.ascontiguousarray(tm, dtype=np.float64)
+    torch.cuda.synchronize()
+    L.check(L.load().ekg_activation_noalloc(*shape, ctypes.c_void_p(layers.data_ptr()), t.shape[0], L.dptr(t),
+                                            ctypes.c_void_p(at.data_ptr()), None))
+    assert np.array_equal(at.cpu().numpy().view(np.int64), ref.view(np.int64))
+
+
+@pytest.mark.parametrize("n,sims,moved", [(12, 2, 1), (20, 11, 3), (28, 33, 2)])
+def test_resting_potential_rows(engine, n, sims, moved):
+    """The resting-potential constant of the moved leads with fewer 8-AP parts in a layer than segments
+    (12^3), rows that are no multiple of a warp or a block's rows, and a row over 64."""
+    from ekgsim_gb300.engine import Heart, layer_aps, move_leads
+    spec = synth.small_spec(n, n_leads=4, seed=5)
+    grid, tm = synth.ellipsoid_heart(spec), synth.transfer_matrix(3, spec.delays)
+    rng = np.random.Generator(np.random.PCG64(n))
+    leads = synth.leads(spec, rng)[:, ::-1].copy()
+    base = [[k0] + list(synth.BASE_AP[1:]) for k0 in (-86.0, -80.0, -90.0)]
+    h = Heart.create(engine, grid, tm, leads, "3D4", 0.0, 200.0, 1.0)
+    h.set_eval(base, synth.K_MIN, synth.K_MAX, [5, 6, 7, 8], list(synth.analytic_target(4, 200, 3)), mid_position=0.6)
+    genes = np.zeros((sims, 12 + 8))
+    genes[:, :12] = synth.GENE_MIN[:12] + (synth.GENE_MAX - synth.GENE_MIN)[:12] * rng.random((sims, 12))
+    genes[:, 12:12 + 2 * moved] = rng.uniform(-20, 20, size=(sims, 2 * moved))
+    ecg = h.eval_batch(genes, want_ecg=True)[2]
+    at, layer = O.activation(grid, tm)
+    for i in {0, sims // 2, sims - 1}:
+        lk = layer_aps(h._cfg, 3, genes[i, :12])[0]
+        ref = O.run(layer, at, lk, move_leads(leads, genes[i, 12:].reshape(-1, 2)), "3D4", 0.0, 200.0, 1.0)
+        assert rel_l2(ecg[i], ref) <= ECG_TOL, i
+    h.close()
