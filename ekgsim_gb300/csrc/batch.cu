@@ -231,6 +231,17 @@ __device__ __forceinline__ MSquares msq(float4 pos, float4 r) {
     q.s = q.h + q.c;
     return q;
 }
+// with every operation rounded
+__device__ __forceinline__ MSquares msq_rn(float4 pos, float4 r) {
+    const float mz = r.x - pos.x, my = r.y - pos.y, mx = r.z - pos.z;
+    MSquares q;
+    q.a = __fmul_rn(mz, mz);
+    q.b = __fmul_rn(my, my);
+    q.c = __fmul_rn(mx, mx);
+    q.h = __fadd_rn(q.a, q.b);
+    q.s = __fadd_rn(q.h, q.c);
+    return q;
+}
 __device__ __forceinline__ float interior_w(const InteriorField &ic, const MSquares &q, float rho) {
     const float u = rho * rho, u2 = u * u;
     const float ab = q.a * q.b;
@@ -238,6 +249,16 @@ __device__ __forceinline__ float interior_w(const InteriorField &ic, const MSqua
     const float c1 = fmaf(u, ic.B0, ic.A0), c2 = fmaf(u, ic.B1, ic.A1);
     const float inner = fmaf(P, c2, Q * (ic.B2 * u2));
     return (rho * u2) * fmaf(u2, inner, c1);
+}
+
+// the same as a product of two factors
+__device__ __forceinline__ float2 interior_f(const InteriorField &ic, const MSquares &q, float rho) {
+    const float u = rho * rho, u2 = u * u;
+    const float ab = q.a * q.b;
+    const float P = fmaf(q.c, q.h, ab), Q = ab * q.c;
+    const float c1 = fmaf(u, ic.B0, ic.A0), c2 = fmaf(u, ic.B1, ic.A1);
+    const float inner = fmaf(P, c2, Q * (ic.B2 * u2));
+    return make_float2(rho * u2, fmaf(u2, inner, c1));
 }
 
 // w(v) for one lead position r relative to the same centre as the voxel positions, general
@@ -554,14 +575,19 @@ __global__ void __launch_bounds__(LF_THREADS, 8) k_batch_lead_field(
     }
 }
 
-// Small batches (up to SMALL_SIMS simulations; above that the persistent kernel with one row per
-// thread is faster, measured at 160^3: 6 simulations 0.119 against 0.132 ms per pass, 16
-// simulations 0.128 against 0.237): one thread per (AP, simulation), so the work spreads
+// Small batches (up to SMALL_SIMS simulations): one thread per (AP, simulation), so the work spreads
 // over the heart instead of over simulations.  A block is four 32-AP stages of one simulation, one
 // per warp; eight consecutive lanes are one 8-AP chunk and write its BF16 hi/lo row segment two
 // bytes each.  The steady sums of a stage are reduced by a shuffle butterfly within its warp.
 // Same outputs as k_batch_lead_field.
+// The field is evaluated with a thread per voxel of the block's range, read in order, into shared
+// memory, as the two factors of its last product (1 and the value where there is none), and each
+// AP's thread then adds its voxels' products in order: a thread walking its own AP's voxels waits for
+// their loads one behind the other while its warp diverges over voxel kinds and counts.  Moved-lead
+// operand, one simulation with 2 leads: 128^3 heart 23.4 -> 14.5 us, 64^3 17.9 -> 9.9; 160^3, 4 simulations with
+// 3 leads 79.5 -> 54; 26-cell neighbourhood, 128^3, 2 with 5 leads 210 -> 106.
 constexpr int SMALL_SIMS = 4;
+constexpr int LFS_VCAP = 512;  // voxels evaluated at a time
 template <int N, bool DIAG>
 __global__ void __launch_bounds__(128) k_batch_lead_field_small(
     int nst, InteriorField ic, const int64_t *__restrict__ a_vox_begin, const float4 *__restrict__ vox_pos,
@@ -571,6 +597,7 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
     const int32_t *__restrict__ nent, const int32_t *__restrict__ esplit, uint8_t *__restrict__ Bt,
     float2 *__restrict__ P1, float *__restrict__ P2) {
     __shared__ float s_d[26 * 4];
+    __shared__ float4 s_f[LFS_VCAP];
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid < nnb) {
         const float dz = difs[3 * tid], dy = difs[3 * tid + 1], dx = difs[3 * tid + 2];
@@ -596,26 +623,41 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
     const float e = pad ? 0.f : ex2a(fmaf(k5, at.x, k5 * at.y));
     const float ez = pad ? 0.f : ex2a(-k4 * ((T.x - at.x) + (T.y - at.y)));
     const int vb = (int)a_vox_begin[a], ve = (int)a_vox_begin[a + 1];
+    // the block's voxels, one behind the other
+    const int64_t a0 = (int64_t)blockIdx.x * 128;
+    const int v0 = (int)a_vox_begin[a0], v1 = (int)a_vox_begin[a0 + 128 < apad ? a0 + 128 : apad];
     for (int l0 = 0; l0 < nmove; l0 += 2) {
         const int np = l0 + 1 < nmove ? 2 : 1;
         const float4 r0 = lrel[(size_t)s * nmove + l0];
         const float4 r1 = np == 2 ? lrel[(size_t)s * nmove + l0 + 1] : r0;
         float acc0 = 0.f, acc1 = 0.f;
-        if (valid)
-            for (int v = vb; v < ve; ++v) {
+        for (int c = v0; c < v1; c += LFS_VCAP) {
+            const int ce = min(c + LFS_VCAP, v1);
+            __syncthreads();
+            for (int v = c + tid; v < ce; v += 128) {
                 const float4 pos = vox_pos[v];
                 const uint32_t mi = __float_as_uint(pos.w);
-                const MSquares q0 = msq(pos, r0), q1 = msq(pos, r1);
+                const MSquares q0 = msq_rn(pos, r0), q1 = msq_rn(pos, r1);
+                float2 f0, f1 = make_float2(0.f, 0.f);
                 if ((mi & VOX_INTERIOR) && q0.s >= INTERIOR_S_MIN && q1.s >= INTERIOR_S_MIN) {
-                    acc0 += interior_w(ic, q0, rsqa(q0.s));
-                    if (np == 2) acc1 += interior_w(ic, q1, rsqa(q1.s));
+                    f0 = interior_f(ic, q0, rsqa(q0.s));
+                    if (np == 2) f1 = interior_f(ic, q1, rsqa(q1.s));
                 } else {
                     const float4 out = vox_out[v];
-                    acc0 += DIAG ? voxel_w_diag(pos, mi, out, r0) : voxel_w_general(pos, mi, out, r0, nnb, s_d);
+                    f0 = make_float2(1.f, DIAG ? voxel_w_diag(pos, mi, out, r0) : voxel_w_general(pos, mi, out, r0, nnb, s_d));
                     if (np == 2)
-                        acc1 += DIAG ? voxel_w_diag(pos, mi, out, r1) : voxel_w_general(pos, mi, out, r1, nnb, s_d);
+                        f1 = make_float2(1.f, DIAG ? voxel_w_diag(pos, mi, out, r1) : voxel_w_general(pos, mi, out, r1, nnb, s_d));
                 }
+                s_f[v - c] = make_float4(f0.x, f0.y, f1.x, f1.y);
             }
+            __syncthreads();
+            if (valid)
+                for (int v = max(vb, c); v < min(ve, ce); ++v) {
+                    const float4 f = s_f[v - c];
+                    acc0 = __fmaf_rn(f.x, f.y, acc0);
+                    acc1 = __fmaf_rn(f.z, f.w, acc1);
+                }
+        }
         if (P2 && valid) {
             // unscaled field sums per 8-AP part of the stage (the resting-potential term): the warp
             // is one stage, eight lanes one part
@@ -633,9 +675,9 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if (q >= np) break;
-            const float w = (q ? acc1 : acc0) * e;
+            const float w = __fmul_rn(q ? acc1 : acc0, e);
             const __nv_bfloat16 hb = __float2bfloat16_rn(w);
-            const __nv_bfloat16 lb = __float2bfloat16_rn(w - __bfloat162float(hb));
+            const __nv_bfloat16 lb = __float2bfloat16_rn(__fsub_rn(w, __bfloat162float(hb)));
             const int row = s * nmove + l0 + q;
             if (valid) {
                 const int nt = row / N, n = row % N;
@@ -646,7 +688,7 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
             }
             // the warp is one stage of one layer: every test below is uniform over it
             if (valid && ne > 0 && st < esplit[L * MAXE + ne - 1]) {
-                float x = w, y = w * ez;
+                float x = w, y = __fmul_rn(w, ez);
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     x += __shfl_xor_sync(0xffffffffu, x, o);

@@ -79,3 +79,40 @@ def test_resting_potential_rows(engine, n, sims, moved):
         ref = O.run(layer, at, lk, move_leads(leads, genes[i, 12:].reshape(-1, 2)), "3D4", 0.0, 200.0, 1.0)
         assert rel_l2(ecg[i], ref) <= ECG_TOL, i
     h.close()
+
+
+@pytest.mark.parametrize("kind,sims,moved,nhood", [
+    ("ellipsoid", 1, 1, "3D4"), ("ellipsoid", 4, 3, "3D4"), ("ellipsoid", 2, 2, "cube"),
+    ("few times", 3, 2, "3D4"),  # thousands of voxels in an AP: the block's range in many parts
+    ("few times", 1, 3, "cube"),
+])
+def test_few_simulations_operand(engine, kind, sims, moved, nhood):
+    """The moved-lead operand of one to four simulations (a thread per voxel, then one per AP): odd and even
+    numbers of moved leads, APs of one voxel up to thousands, both neighbourhoods."""
+    from ekgsim_gb300.engine import Heart, layer_aps, move_leads
+    rng = np.random.Generator(np.random.PCG64(sims * 10 + moved))
+    if kind == "ellipsoid":
+        spec = synth.small_spec(24, n_leads=4, seed=9)
+        grid, tm = synth.ellipsoid_heart(spec), synth.transfer_matrix(3, spec.delays)
+        at, layer = O.activation(grid, tm)
+        given = None
+    else:
+        grid = rng.integers(1, 4, size=(17, 20, 19)).astype(np.int32)
+        grid[rng.random(grid.shape) < 0.05] = 0
+        tm = synth.transfer_matrix(3, [1, 2, 2])
+        layer = grid.copy()
+        given = at = np.where(grid > 0, np.floor(np.arange(20) / 10)[None, :, None] * 7.0 + 3.0, 0.0)
+    leads = np.array(grid.shape) / 2 + 30.0 * np.array([[1.0, 0.2, 0.1], [-0.3, 1.0, 0.4], [0.2, -0.5, -1.0], [0.6, 0.7, 0.5]])
+    h = Heart.create(engine, grid, tm, leads, nhood, 0.0, 150.0, 1.0, activation=given)
+    h.set_eval([synth.BASE_AP] * 3, synth.K_MIN, synth.K_MAX, [5, 6, 7, 8], list(synth.analytic_target(4, 150, 3)),
+               mid_position=0.6)
+    genes = np.zeros((sims, 12 + 8))
+    genes[:, :12] = synth.GENE_MIN[:12] + (synth.GENE_MAX - synth.GENE_MIN)[:12] * rng.random((sims, 12))
+    genes[:, 12:12 + 2 * moved] = rng.uniform(-8, 8, size=(sims, 2 * moved))
+    for _ in range(2):  # a single simulation takes the batched form from its second call on
+        ecg = h.eval_batch(genes, want_ecg=True)[2]
+    for i in range(sims):
+        lk = layer_aps(h._cfg, 3, genes[i, :12])[0]
+        ref = O.run(layer, at, lk, move_leads(leads, genes[i, 12:].reshape(-1, 2)), nhood, 0.0, 150.0, 1.0)
+        assert rel_l2(ecg[i], ref) <= ECG_TOL, i
+    h.close()
