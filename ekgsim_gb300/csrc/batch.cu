@@ -121,15 +121,17 @@ __global__ void k_reduce_layers(int steps, int rows, int nl, const int32_t *__re
 // per layer in FP32 (the basis is stored in FP32), the sum over layers in float-float; written as
 // FP64 and as float-float.  Block = 128 steps of one static lead for SC_SIMS simulations: a
 // thread loads the basis rows of its step once per layer and applies them to every simulation of
-// the group (coefficients broadcast from shared memory).
-constexpr int SC_SIMS = 16;
+// the group (coefficients broadcast from shared memory).  With few simulations a layer is a handful of
+// operations behind a load, so the coefficients of SC_LAYERS layers are staged at once and the next
+// layer's basis rows are on their way while one is summed.
+constexpr int SC_SIMS = 16, SC_LAYERS = 8;
 __global__ void __launch_bounds__(128) k_static_combine(int steps, int nleads, int nl, int J, int Jb, int nmove,
                                                         int n_sims, const float *__restrict__ F,
                                                         const float *__restrict__ coef, const double *__restrict__ k3,
                                                         const float *__restrict__ Q1, const float *__restrict__ Q2,
                                                         double *__restrict__ ecg, float2 *__restrict__ ecg_ff,
                                                         const double *__restrict__ cst) {
-    __shared__ float s_c[SC_SIMS][11];  // [simulation][j < J: coefficient, 10: k3] of the current layer
+    __shared__ float s_c[SC_LAYERS][SC_SIMS][11];  // [layer][simulation][j < J: coefficient, 10: k3]
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int l = nmove + blockIdx.y, s0 = blockIdx.z * SC_SIMS;
     const int ns = min(SC_SIMS, n_sims - s0);
@@ -139,33 +141,47 @@ __global__ void __launch_bounds__(128) k_static_combine(int steps, int nleads, i
     float2 acc[SC_SIMS];
 #pragma unroll
     for (int i = 0; i < SC_SIMS; ++i) acc[i] = make_float2(0.f, 0.f);
-    for (int L = 0; L < nl; ++L) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < ns * 11; k += blockDim.x) {
-            const int i = k / 11, j = k % 11;
-            const size_t sl = (size_t)(s0 + i) * nl + L;
-            s_c[i][j] = j < J ? coef[sl * J + j] : (j == 10 ? (float)k3[sl] : 0.f);
-        }
-        __syncthreads();
+    float n1[10], n2[10];  // the next layer's basis rows
+    auto fetch = [&](int L) {
         const size_t q0 = ((size_t)L * rows + (size_t)l * Jb) * steps + tc;
-        float q1[10], q2[10];
 #pragma unroll
         for (int j = 0; j < 10; ++j) {  // J <= 10 (the basis order)
-            q1[j] = j < J ? Q1[q0 + (size_t)j * steps] : 0.f;
-            q2[j] = j < J ? Q2[q0 + (size_t)j * steps] : 0.f;
+            n1[j] = j < J ? Q1[q0 + (size_t)j * steps] : 0.f;
+            n2[j] = j < J ? Q2[q0 + (size_t)j * steps] : 0.f;
         }
+    };
+    fetch(0);
+    for (int L0 = 0; L0 < nl; L0 += SC_LAYERS) {
+        const int nL = min(SC_LAYERS, nl - L0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < nL * ns * 11; k += blockDim.x) {
+            const int Lk = k / (ns * 11), i = (k / 11) % ns, j = k % 11;
+            const size_t sl = (size_t)(s0 + i) * nl + L0 + Lk;
+            s_c[Lk][i][j] = j < J ? coef[sl * J + j] : (j == 10 ? (float)k3[sl] : 0.f);
+        }
+        __syncthreads();
+        for (int Lk = 0; Lk < nL; ++Lk) {
+            float q1[10], q2[10];
 #pragma unroll
-        for (int i = 0; i < SC_SIMS; ++i)
-            if (i < ns) {
-                float v1 = 0.f, v2 = 0.f;
-#pragma unroll
-                for (int j = 0; j < 10; ++j)
-                    if (j < J) {
-                        v1 = fmaf(s_c[i][j], q1[j], v1);
-                        v2 = fmaf(s_c[i][j], q2[j], v2);
-                    }
-                acc[i] = ff_add_f(acc[i], F[((size_t)(s0 + i) * nl + L) * steps + tc] * fmaf(s_c[i][10], v2 - v1, v1));
+            for (int j = 0; j < 10; ++j) {
+                q1[j] = n1[j];
+                q2[j] = n2[j];
             }
+            const int L = L0 + Lk;
+            if (L + 1 < nl) fetch(L + 1);
+#pragma unroll
+            for (int i = 0; i < SC_SIMS; ++i)
+                if (i < ns) {
+                    float v1 = 0.f, v2 = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 10; ++j)
+                        if (j < J) {
+                            v1 = fmaf(s_c[Lk][i][j], q1[j], v1);
+                            v2 = fmaf(s_c[Lk][i][j], q2[j], v2);
+                        }
+                    acc[i] = ff_add_f(acc[i], F[((size_t)(s0 + i) * nl + L) * steps + tc] * fmaf(s_c[Lk][i][10], v2 - v1, v1));
+                }
+        }
     }
     if (!on) return;
 #pragma unroll

@@ -106,7 +106,9 @@ __global__ void k_lead_field(int64_t apad, const int64_t *__restrict__ a_vox_beg
 //     ln(1 + e^u) = log1p(exp(u)) (u + log1p(exp(-u)) for u > 0),  R = -expm1(-(k6/k7) ln(1 + e^u)).
 // layer_k: [S][nl][9].
 // cpre: the constants ln(2^(k7/k6) - 1) per (sim, layer) when the host computed them (small
-// passes, where the FP64 pow/log would be one block's latency), else NULL.
+// passes, where the FP64 pow/log would be one block's latency), else NULL.  With them the steps are cut
+// into blocks too (grid.y): a pass of one simulation has only as many (sim, layer) pairs as layers, whose
+// five steps a thread, one behind the other, took 7.7 us (three layers, 600 steps).
 __global__ void k_layer_factors(int nl, int steps, const double *__restrict__ t, const double *__restrict__ layer_k,
                                 const double *__restrict__ cpre, int n_sims, double *__restrict__ F,
                                 float *__restrict__ Ff, float *__restrict__ layer_c, const double *__restrict__ centre,
@@ -116,10 +118,12 @@ __global__ void k_layer_factors(int nl, int steps, const double *__restrict__ t,
     __shared__ double c;
     if (threadIdx.x == 0) {
         c = cpre ? cpre[sl] : log(pow(2.0, k[7] / k[6]) - 1);
+    }
+    if (threadIdx.x == 0 && blockIdx.y == 0) {
         const double L2E = 1.4426950408889634;
         reinterpret_cast<float4 *>(layer_c)[sl] =
             make_float4((float)(k[1] * L2E), (float)(k[4] * L2E), (float)(1.0 - k[3]), (float)k[3]);
-    } else if (threadIdx.x == 32 && coef) {
+    } else if (threadIdx.x == 32 && blockIdx.y == 0 && coef) {
         // Taylor coefficients of the static-lead basis: coef[sl][j] = exp(k5 c_L) (k5 s_L)^j / j!
         const int L = (int)(sl % nl);
         const double x = k[5] * scale[L];
@@ -131,7 +135,7 @@ __global__ void k_layer_factors(int nl, int steps, const double *__restrict__ t,
     }
     __syncthreads();
     const float r = (float)(k[6] / k[7]);
-    for (int step = threadIdx.x; step < steps; step += blockDim.x) {
+    for (int step = blockIdx.y * blockDim.x + threadIdx.x; step < steps; step += gridDim.y * blockDim.x) {
         const double tt = t[step];
         const float u = (float)fma(-k[7], tt - k[8], c);
         const float sp = u > 0.f ? u + log1pf(expf(-u)) : log1pf(expf(u));
@@ -759,7 +763,8 @@ void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads,
 void launch_layer_factors(cudaStream_t s, const HeartDev &h, const double *d_layer_k, const double *d_cpre,
                           int n_sims, double *d_F, float *d_Ff, float *d_layer_c, const double *d_centre,
                           const double *d_scale, int J, float *d_coef) {
-    k_layer_factors<<<(unsigned)((int64_t)n_sims * h.nlayers), 128, 0, s>>>(
+    const dim3 grid((unsigned)((int64_t)n_sims * h.nlayers), d_cpre ? (unsigned)((h.steps + 127) / 128) : 1u);
+    k_layer_factors<<<grid, 128, 0, s>>>(
         h.nlayers, h.steps, h.t.p, d_layer_k, d_cpre, n_sims, d_F, d_Ff, d_layer_c, d_centre, d_scale, J, d_coef);
     EKG_CUDA(cudaGetLastError());
 }

@@ -1087,12 +1087,12 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[0], s));
     EKG_CUDA(cudaMemsetAsync(E.err.p, 0, sizeof(uint32_t), s));
     const ekg_heart::PassInputs &in = h->in();
-    // batched form with both static and moved leads: the layer factors and the static combine
-    // (beside the moved-lead operand kernel, which needs neither) and the steady-sum reduction
-    // (beside the band GEMM) run on the auxiliary stream, joined before the band reduction
+    // batched form with moved leads: the layer factors and the static combine (beside the moved-lead
+    // operand kernel, which needs neither) and the steady-sum reduction (beside the band GEMM) run on the
+    // auxiliary stream, joined before the band reduction
     // (measured: other placements of the small kernels, such as the criteria of the static leads
     // beside the GEMM, lengthen the pass)
-    const bool fork = P.batch && nmove > 0 && nmove < (int)L;
+    const bool fork = P.batch && nmove > 0;
     cudaStream_t sx = fork ? h->aux_stream : s;
     if (fork) {
         EKG_CUDA(cudaEventRecord(h->ev_fork, s));
