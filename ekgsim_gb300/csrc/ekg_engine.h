@@ -140,6 +140,7 @@ struct ekg_heart {
         uint8_t *host = nullptr;
         ekg::DBuf<uint8_t> dev;
         size_t cap = 0;
+        size_t used = 0;  // bytes of the current pass's inputs
         PassInputs in;
     };
     Staging stg[2];
@@ -150,9 +151,10 @@ struct ekg_heart {
         bool busy = false;
         int64_t ticket = 0;
         cudaEvent_t done = nullptr;        // the pass and its copies to the host are complete
-        uint32_t *err = nullptr;           // pinned error word of the pass
-        double *crit2 = nullptr;           // pinned per-lead criterion values and peaks
-        size_t crit2_cap = 0;
+        double *out = nullptr;             // pinned copy of the pass's results (EvalDev::out, small ECGs included)
+        size_t out_cap = 0;
+        double *ecg = nullptr;             // the caller's ECG buffer where it is filled from `out`
+        size_t ecg_off = 0, ecg_n = 0;     // where the ECG lies in `out`, and its values
         int n_sims = 0;
         bool single = false;               // an ekg_eval call (sets simulationDone when handed over)
         std::vector<double> lk_all, leads_all, viol, acrit, endo_epi;
@@ -175,8 +177,7 @@ struct ekg_heart {
             if (g.host) cudaFreeHost(g.host);
         for (Pending &p : pend) {
             if (p.done) cudaEventDestroy(p.done);
-            if (p.err) cudaFreeHost(p.err);
-            if (p.crit2) cudaFreeHost(p.crit2);
+            if (p.out) cudaFreeHost(p.out);
         }
         if (copies_done) cudaEventDestroy(copies_done);
         if (pass_end) cudaEventDestroy(pass_end);

@@ -214,14 +214,18 @@ struct EvalDev {
     DBuf<int4> cinfo;       // [S][nchunks] (first band step, first steady step, amax bits, 0)
     DBuf<int> work;         // work-item counter of the moved-row field kernel
     DBuf<float> coef;       // [S][nl][J] static-lead Taylor coefficients (batched form)
-    DBuf<double> ecg;       // [S][L][steps]
+    // a pass's results, one behind the other so that they reach the host in one copy:
+    // [error words of the two staging slots | criterion values and peaks [S][ncrit][2] | ECG [S][L][steps]]
+    DBuf<double> out;
+    uint32_t *err = nullptr;   // the current pass's error word (only ever set; cleared when reported)
+    double *crit = nullptr;    // within out, placed per pass
+    double *ecg = nullptr;
     DBuf<float2> ecg_ff;    // [S][L][steps] the same as float-float (hi, lo), read by the criteria
-    DBuf<double> crit;      // [S][ncrit]
     DBuf<double> targets;   // concatenated targets
     DBuf<float2> targets_ff;  // the same as float-float
     DBuf<int64_t> target_len;
     DBuf<double> target_off;
-    DBuf<uint32_t> err;     // [1]
+    DBuf<uint32_t> basis_err;  // [1] error word of the basis build
 };
 
 void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads, int nleads_in, int lead_stride,

@@ -337,7 +337,7 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
     }
     if (!h->err_host) EKG_CUDA(cudaMallocHost(&h->err_host, sizeof(uint32_t)));
     EKG_CUDA(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->eng->device));
-    h->ev.err.alloc(1);
+    h->ev.basis_err.alloc(1);
     cudaStream_t s = h->stream;
     // activation times (the layer grid stays on the device for the de-duplication)
     DBuf<uint8_t> dl;
@@ -483,7 +483,7 @@ int64_t heart_device_bytes(const ekg_heart *h) {
                 h->W0.bytes() + h->at_cells.bytes() + D.vox_pos.bytes() + D.vox_out.bytes() + D.stage_box.bytes();
     const EvalDev &E = h->ev;
     b += (int64_t)h->stg[0].dev.bytes() + (int64_t)h->stg[1].dev.bytes() + E.layer_c.bytes() + E.F.bytes() + E.k0w.bytes() + E.W.bytes() +
-         E.Wp.bytes() + E.partial.bytes() + E.ecg.bytes() + E.ecg_ff.bytes() + E.coef.bytes() + E.crit.bytes() + E.targets.bytes() +
+         E.Wp.bytes() + E.partial.bytes() + E.out.bytes() + E.ecg_ff.bytes() + E.coef.bytes() + E.targets.bytes() +
          E.targets_ff.bytes();
     return b;
 }
@@ -497,6 +497,8 @@ int64_t eval_bytes_per_sim(const ekg_heart *h) {
 }
 int64_t eval_bytes_held(const ekg_heart *h) { return (int64_t)h->ev.cap_sims * eval_bytes_per_sim(h); }
 
+// values of EvalDev::out before the ECG: the error words and the criteria, rounded to 16 bytes
+size_t out_ecg_offset(int n_sims, int n_crit_leads) { return (1 + (size_t)n_sims * n_crit_leads * 2 + 1) / 2 * 2; }
 void ensure_eval_capacity(ekg_heart *h, int n_sims) {
     EvalDev &E = h->ev;
     const HeartDev &D = h->dev;
@@ -506,11 +508,17 @@ void ensure_eval_capacity(ekg_heart *h, int n_sims) {
     E.F.alloc(S * D.nlayers * D.steps);
     E.Ff.alloc(S * D.nlayers * D.steps);
     E.k0w.alloc(S * D.nleads);
-    E.ecg.alloc(S * D.nleads * D.steps);
+    E.out.alloc(out_ecg_offset(n_sims, std::max(1, D.nleads)) + S * D.nleads * D.steps);
+    EKG_CUDA(cudaMemsetAsync(E.out.p, 0, sizeof(double), h->stream));  // the error words
     E.ecg_ff.alloc(S * D.nleads * D.steps);
-    E.crit.alloc(S * std::max(1, D.nleads) * 2);
-    E.err.alloc(1);
     E.cap_sims = n_sims;
+}
+// Places a pass's results in EvalDev::out.
+void place_outputs(ekg_heart *h, int n_sims, int n_crit_leads) {
+    EvalDev &E = h->ev;
+    E.err = reinterpret_cast<uint32_t *>(E.out.p) + h->cur;
+    E.crit = E.out.p + 1;
+    E.ecg = E.out.p + out_ecg_offset(n_sims, n_crit_leads);
 }
 // moved rows (simulations x moved leads) from which the per-simulation form evaluates their field
 // with the persistent row kernel (below: one thread per (AP, simulation)); measured at 160^3 with 2
@@ -766,11 +774,11 @@ void ensure_basis(ekg_heart *h, const std::vector<double> &key) {
         A.layer_c = lc.p;
         A.F = ones.p;
         A.partial = part.p;
-        A.err = h->ev.err.p;
-        EKG_CUDA(cudaMemsetAsync(h->ev.err.p, 0, 4, s));
+        A.err = h->ev.basis_err.p;
+        EKG_CUDA(cudaMemsetAsync(h->ev.basis_err.p, 0, 4, s));
         launch_contract_umma_args(s, A);
         launch_reduce_layers(s, D.steps, rows, nl, B.lc0.p, B.lc1.p, part.p, basis == 0 ? B.Q1.p : B.Q2.p);
-        EKG_CUDA(cudaMemcpyAsync(h->err_host, h->ev.err.p, 4, cudaMemcpyDeviceToHost, s));
+        EKG_CUDA(cudaMemcpyAsync(h->err_host, h->ev.basis_err.p, 4, cudaMemcpyDeviceToHost, s));
         EKG_CUDA(cudaStreamSynchronize(s));
         if (*h->err_host) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (basis build)"};
     }
@@ -904,7 +912,7 @@ PassPlan plan_pass(ekg_heart *h, int n_sims, const double *layer_k, const double
         P.rows_used = n_sims * P.nmove;
         // launch shape: the autotuner's choice for this pass shape, else the built-in one
         const TuneChoice *tc = h->tune_force;
-        if (!tc) {
+        if (!tc && (!h->tuned.empty() || !h->eng->tune_cache.empty())) {
             const std::string key = tune_key(h, n_sims, P.nmove, P.two_bases);
             auto it = h->tuned.find(key);
             if (it == h->tuned.end() && !h->eng->tune_cache.empty()) {
@@ -962,11 +970,15 @@ PassPlan plan_pass(ekg_heart *h, int n_sims, const double *layer_k, const double
 
 
 
-void upload_inputs(ekg_heart *h, const PassPlan &P, const double *layer_k, const double *leads) {
+// Buffers for a pass and its inputs, packed into the staging buffer: copied to the device at once
+// (`now`), or by the pass itself (compute).
+void upload_inputs(ekg_heart *h, const PassPlan &P, const double *layer_k, const double *leads, int n_crit_leads,
+                   bool now) {
     HeartDev &D = h->dev;
     cudaStream_t s = h->stream;
     const int n_sims = P.n_sims;
     ensure_eval_capacity(h, n_sims);
+    place_outputs(h, n_sims, n_crit_leads);
     const size_t L = D.nleads, S = n_sims, nl = D.nlayers;
     h->any_k0 = false;
     for (size_t i = 0; i < S * nl; ++i) h->any_k0 = h->any_k0 || layer_k[9 * i] != 0.0;
@@ -1017,7 +1029,8 @@ void upload_inputs(ekg_heart *h, const PassPlan &P, const double *layer_k, const
         sg.cap = cap;
     }
     for (const Slot &sl : slots) std::memcpy(sg.host + sl.off, sl.src, sl.bytes);
-    if (off) EKG_CUDA(cudaMemcpyAsync(sg.dev.p, sg.host, off, cudaMemcpyHostToDevice, s));
+    sg.used = off;
+    if (now && off) EKG_CUDA(cudaMemcpyAsync(sg.dev.p, sg.host, off, cudaMemcpyHostToDevice, s));
     const uint8_t *dv = sg.dev.p;
     ekg_heart::PassInputs &in = sg.in;
     in = ekg_heart::PassInputs();
@@ -1077,7 +1090,16 @@ void upload_inputs(ekg_heart *h, const PassPlan &P, const double *layer_k, const
     }
 }
 
-void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTiming *tm, bool mark_static = false) {
+// What a pass copies itself: its staged inputs to the device, and the first `out_n` values of
+// EvalDev::out to `out`.
+struct PassIO {
+    bool in = false;
+    double *out = nullptr;
+    size_t out_n = 0;
+};
+
+void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTiming *tm, bool mark_static = false,
+             const PassIO &io = PassIO()) {
     HeartDev &D = h->dev;
     EvalDev &E = h->ev;
     cudaStream_t s = h->stream;
@@ -1085,7 +1107,8 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     const size_t L = D.nleads, S = n_sims;
     int launches = 0;
     if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[0], s));
-    EKG_CUDA(cudaMemsetAsync(E.err.p, 0, sizeof(uint32_t), s));
+    const ekg_heart::Staging &sg = h->stg[h->cur];
+    if (io.in && sg.used) EKG_CUDA(cudaMemcpyAsync(sg.dev.p, sg.host, sg.used, cudaMemcpyHostToDevice, s));
     const ekg_heart::PassInputs &in = h->in();
     // batched form with moved leads: the layer factors and the static combine (beside the moved-lead
     // operand kernel, which needs neither) and the steady-sum reduction (beside the band GEMM) run on the
@@ -1105,7 +1128,7 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     if (P.batch) {
         BatchState &B = h->bs;
         auto static_part = [&]() {
-            launch_static_combine(sx, D, P.J, B.J, nmove, n_sims, E.Ff.p, E.coef.p, in.k3, B.Q1.p, B.Q2.p, E.ecg.p,
+            launch_static_combine(sx, D, P.J, B.J, nmove, n_sims, E.Ff.p, E.coef.p, in.k3, B.Q1.p, B.Q2.p, E.ecg,
                                   E.ecg_ff.p, P.k0 ? B.cst.p : nullptr);
             launches += nmove < (int)L;
             if (mark_static) {
@@ -1156,7 +1179,7 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
             U.cmov = P.k0 ? B.cmov.p : nullptr;
             U.U = B.U.p;
             U.Up = B.Up.p;
-            U.ecg = E.ecg.p;
+            U.ecg = E.ecg;
             U.ecg_ff = E.ecg_ff.p;
             if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[4], s));
             launch_batch_lead_field(s, D, P.tile_rows, P.op_small != 0, P.op_bps, in.k5l, in.hconst, in.lrel, nmove,
@@ -1192,7 +1215,7 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
             A.hconst = in.hconst;
             A.Bt = B.Bt.p;
             A.partial = B.partial.p;
-            A.err = E.err.p;
+            A.err = E.err;
             launch_batch_gemm(s, A);
             launches += P.nitems > 0;
             if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[2], s));
@@ -1247,29 +1270,31 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
             launch_contract_band(s, D, E.W.p, nmove, h->W0.p, in.layer_k, E.layer_c.p, n_sims, E.band.p, E.csum.p,
                                  E.cinfo.p);
             if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[2], s));
-            launch_reduce_chunks(s, D, E.layer_c.p, E.F.p, E.band.p, E.csum.p, E.cinfo.p, E.k0w.p, n_sims, E.ecg.p,
+            launch_reduce_chunks(s, D, E.layer_c.p, E.F.p, E.band.p, E.csum.p, E.cinfo.p, E.k0w.p, n_sims, E.ecg,
                                  E.ecg_ff.p);
         } else {
             if (h->eng->contract != EKG_CONTRACT_DENSE_CUDA)
-                launch_contract_umma(s, D, E.Wp.p, E.layer_c.p, E.F.p, n_sims, E.partial.p, E.err.p);
+                launch_contract_umma(s, D, E.Wp.p, E.layer_c.p, E.F.p, n_sims, E.partial.p, E.err);
             else
                 launch_contract_cuda(s, D, E.Wp.p, E.layer_c.p, E.F.p, n_sims, E.partial.p);
             if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[2], s));
-            launch_reduce_ecg(s, D, E.partial.p, E.k0w.p, n_sims, E.ecg.p, E.ecg_ff.p);
+            launch_reduce_ecg(s, D, E.partial.p, E.k0w.p, n_sims, E.ecg, E.ecg_ff.p);
         }
         launches += 2;
     }
     if (n_crit_leads > 0) {
-        launch_criteria(s, D, E.ecg.p, E.ecg_ff.p, n_sims, n_crit_leads, 0, n_crit_leads, mode, E.targets.p,
-                        E.targets_ff.p, E.target_len.p, E.target_off.p, E.crit.p);
+        launch_criteria(s, D, E.ecg, E.ecg_ff.p, n_sims, n_crit_leads, 0, n_crit_leads, mode, E.targets.p,
+                        E.targets_ff.p, E.target_len.p, E.target_off.p, E.crit);
         ++launches;
     }
+    if (io.out_n) EKG_CUDA(cudaMemcpyAsync(io.out, E.out.p, io.out_n * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[3], s));
     g_launch_count = launches;
 }
 
 // Everything the launches of compute() depend on: the pass shape and every device pointer it passes.
-std::vector<uint64_t> pass_signature(const ekg_heart *h, const PassPlan &P, int ncl, int mode, bool mark_static) {
+std::vector<uint64_t> pass_signature(const ekg_heart *h, const PassPlan &P, int ncl, int mode, bool mark_static,
+                                     const PassIO &io) {
     const EvalDev &E = h->ev;
     const BatchState &B = h->bs;
     auto u = [](const void *p) { return (uint64_t)(uintptr_t)p; };
@@ -1278,14 +1303,16 @@ std::vector<uint64_t> pass_signature(const ekg_heart *h, const PassPlan &P, int 
                                (uint64_t)P.nitems, (uint64_t)ncl, (uint64_t)mode, (uint64_t)mark_static,
                                (uint64_t)h->cpre_on, (uint64_t)h->any_k0, (uint64_t)h->eng->contract, (uint64_t)B.J,
                                (uint64_t)B.max_ent, (uint64_t)B.ntt, (uint64_t)P.tile_rows, (uint64_t)P.op_small,
-                               (uint64_t)P.op_bps, (uint64_t)P.k0};
+                               (uint64_t)P.op_bps, (uint64_t)P.k0, (uint64_t)io.in, (uint64_t)io.out_n,
+                               (uint64_t)h->stg[h->cur].used};
     const ekg_heart::PassInputs &in = h->in();
     for (const void *p : {(const void *)in.layer_k, (const void *)in.cpre, (const void *)in.leads, (const void *)in.k3,
                           (const void *)B.d_centre.p, (const void *)B.d_scale.p, (const void *)E.coef.p,
                           (const void *)in.k5l, (const void *)in.hconst, (const void *)in.lrel,
                           (const void *)in.items, (const void *)in.ti0, (const void *)in.ti1,
                           (const void *)E.F.p, (const void *)E.Ff.p,
-                          (const void *)E.layer_c.p, (const void *)E.ecg.p, (const void *)E.crit.p, (const void *)E.err.p,
+                          (const void *)E.layer_c.p, (const void *)E.ecg, (const void *)E.crit, (const void *)E.err, (const void *)io.out,
+                          (const void *)h->stg[h->cur].host, (const void *)h->stg[h->cur].dev.p,
                           (const void *)E.ecg_ff.p, (const void *)E.targets_ff.p, (const void *)E.targets.p, (const void *)E.target_len.p, (const void *)E.target_off.p,
                           (const void *)E.W.p, (const void *)E.Wp.p, (const void *)E.partial.p, (const void *)E.k0w.p,
                           (const void *)B.Q1.p,
@@ -1304,12 +1331,12 @@ std::vector<uint64_t> pass_signature(const ekg_heart *h, const PassPlan &P, int 
 // compute() as a CUDA graph: the first pass with a signature runs directly (it also performs the
 // launchers' one-time set-up), the second is captured (thread-local capture on the heart's stream)
 // and instantiated, later ones replay it.  Up to four graphs per heart, least recently used out.
-void run_pass(ekg_heart *h, const PassPlan &P, int ncl, int mode, bool mark_static) {
+void run_pass(ekg_heart *h, const PassPlan &P, int ncl, int mode, bool mark_static, const PassIO &io = PassIO()) {
     if (!h->eng->graphs) {
-        compute(h, P, ncl, mode, nullptr, mark_static);
+        compute(h, P, ncl, mode, nullptr, mark_static, io);
         return;
     }
-    const std::vector<uint64_t> sig = pass_signature(h, P, ncl, mode, mark_static);
+    const std::vector<uint64_t> sig = pass_signature(h, P, ncl, mode, mark_static, io);
     ekg_heart::PassGraph *g = nullptr, *victim = &h->graphs[0];
     for (auto &c : h->graphs) {
         if (!c.sig.empty() && c.sig == sig) g = &c;
@@ -1326,13 +1353,13 @@ void run_pass(ekg_heart *h, const PassPlan &P, int ncl, int mode, bool mark_stat
         *victim = ekg_heart::PassGraph();
         victim->sig = sig;
         victim->used = ++h->graph_clock;
-        compute(h, P, ncl, mode, nullptr, mark_static);
+        compute(h, P, ncl, mode, nullptr, mark_static, io);
         return;
     }
     cudaGraph_t graph = nullptr;
     EKG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     try {
-        compute(h, P, ncl, mode, nullptr, mark_static);
+        compute(h, P, ncl, mode, nullptr, mark_static, io);
     } catch (...) {
         cudaStreamEndCapture(s, &graph);
         if (graph) cudaGraphDestroy(graph);
@@ -1353,10 +1380,11 @@ void assemble_criteria(const ekg_heart *h, const double *crit2, bool done, doubl
 TuneChoice tune_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, int reps,
                      double *builtin_ms);
 
-// Queues one device pass from the current staging buffer (h->cur): plan, upload, the pass (a graph
-// replay) and the copies of its outputs (ECG to ecg_host; criterion values and the error word to
-// the pending slot's pinned buffers).  pend[h->cur].done marks the pass and its copies complete.
+// Queues one device pass from the current staging buffer (h->cur): plan, the pass with the copies of its
+// inputs and of its criterion values and error word (one graph replay), and a larger ECG's copies to
+// ecg_host.  pend[h->cur].done marks the pass and its copies complete.
 // The pass's kernels wait for the previous pass's copies to the host (they overwrite its outputs).
+constexpr size_t SMALL_ECG_BYTES = 128 << 10;
 void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, double *ecg_host,
                  int n_crit_leads, int mode) {
     HeartDev &D = h->dev;
@@ -1369,18 +1397,23 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
         for (cudaEvent_t *e : {&h->static_done, &h->moved_done, &h->copies_done, &h->pass_end})
             EKG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
-    if (!pd.done) {
-        EKG_CUDA(cudaEventCreateWithFlags(&pd.done, cudaEventDisableTiming));
-        EKG_CUDA(cudaMallocHost(&pd.err, sizeof(uint32_t)));
+    if (!pd.done) EKG_CUDA(cudaEventCreateWithFlags(&pd.done, cudaEventDisableTiming));
+    const size_t L = D.nleads, S = n_sims, T = D.steps;
+    // a small ECG comes with the criteria in the pass's own copy to pinned memory and is handed over from
+    // there: the copy into pageable memory makes the driver wait for the pass and copy twice by itself
+    const size_t ecg_off = out_ecg_offset(n_sims, n_crit_leads);
+    const bool small = ecg_host && S * L * T * 8 <= SMALL_ECG_BYTES;
+    const size_t need = ecg_off + (small ? S * L * T : 0);
+    if (pd.out_cap < need) {
+        if (pd.out) cudaFreeHost(pd.out);
+        pd.out = nullptr;
+        pd.out_cap = 0;
+        EKG_CUDA(cudaMallocHost(&pd.out, need * sizeof(double)));
+        pd.out_cap = need;
     }
-    const size_t need = (size_t)n_sims * std::max(1, n_crit_leads) * 2;
-    if (pd.crit2_cap < need) {
-        if (pd.crit2) cudaFreeHost(pd.crit2);
-        pd.crit2 = nullptr;
-        pd.crit2_cap = 0;
-        EKG_CUDA(cudaMallocHost(&pd.crit2, need * sizeof(double)));
-        pd.crit2_cap = need;
-    }
+    pd.ecg = small ? ecg_host : nullptr;
+    pd.ecg_off = ecg_off;
+    pd.ecg_n = S * L * T;
     if (h->eng->tune && n_sims > 1) {
         // tune a new pass shape on its first pass (the choice is kept for the heart)
         const PassPlan Pt = plan_pass(h, n_sims, layer_k, leads);
@@ -1388,30 +1421,34 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
             tune_pass(h, n_sims, layer_k, leads, 3, nullptr);
     }
     const PassPlan P = plan_pass(h, n_sims, layer_k, leads);
-    upload_inputs(h, P, layer_k, leads);
+    upload_inputs(h, P, layer_k, leads, n_crit_leads, false);
     if (h->copies_pending) EKG_CUDA(cudaStreamWaitEvent(s, h->copies_done, 0));
-    const size_t L = D.nleads, S = n_sims, T = D.steps;
+    h->copies_pending = false;
+    PassIO io;
+    io.in = true;
+    io.out = pd.out;
+    io.out_n = need;
+    if (small || !ecg_host) {
+        run_pass(h, P, n_crit_leads, mode, false, io);
+        EKG_CUDA(cudaEventRecord(pd.done, s));
+        return;
+    }
     // batched form: the static-lead rows of the ECG are final early, so their copy to the host runs
     // on the copy stream while the moved-lead part is computed
-    const bool split = ecg_host && P.batch && P.nmove < (int)L;
-    run_pass(h, P, n_crit_leads, mode, split);
+    const bool split = P.batch && P.nmove < (int)L;
+    run_pass(h, P, n_crit_leads, mode, split, io);
     if (split) {
         const size_t nm = P.nmove;
         EKG_CUDA(cudaStreamWaitEvent(h->copy_stream, h->static_done, 0));
-        EKG_CUDA(cudaMemcpy2DAsync(ecg_host + nm * T, L * T * 8, E.ecg.p + nm * T, L * T * 8, (L - nm) * T * 8, S,
+        EKG_CUDA(cudaMemcpy2DAsync(ecg_host + nm * T, L * T * 8, E.ecg + nm * T, L * T * 8, (L - nm) * T * 8, S,
                                    cudaMemcpyDeviceToHost, h->copy_stream));
-    }
-    EKG_CUDA(cudaMemcpyAsync(pd.err, E.err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    if (n_crit_leads > 0)
-        EKG_CUDA(cudaMemcpyAsync(pd.crit2, E.crit.p, S * n_crit_leads * 2 * 8, cudaMemcpyDeviceToHost, s));
-    if (split) {
         if (P.nmove > 0) {
             EKG_CUDA(cudaStreamWaitEvent(h->copy_stream, h->moved_done, 0));
-            EKG_CUDA(cudaMemcpy2DAsync(ecg_host, L * T * 8, E.ecg.p, L * T * 8, (size_t)P.nmove * T * 8, S,
+            EKG_CUDA(cudaMemcpy2DAsync(ecg_host, L * T * 8, E.ecg, L * T * 8, (size_t)P.nmove * T * 8, S,
                                        cudaMemcpyDeviceToHost, h->copy_stream));
         }
-    } else if (ecg_host) {
-        EKG_CUDA(cudaMemcpyAsync(ecg_host, E.ecg.p, S * L * T * 8, cudaMemcpyDeviceToHost, s));
+    } else {
+        EKG_CUDA(cudaMemcpyAsync(ecg_host, E.ecg, S * L * T * 8, cudaMemcpyDeviceToHost, s));
     }
     // done = the heart's stream and the copy stream both past this pass
     EKG_CUDA(cudaEventRecord(h->pass_end, s));
@@ -1421,6 +1458,17 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
     h->copies_pending = true;
 }
 
+// Clears a slot's error word once it is reported (no pass of the slot is in flight then).
+void clear_error(ekg_heart *h, int slot) {
+    if (h->ev.out.p) cudaMemsetAsync(reinterpret_cast<uint32_t *>(h->ev.out.p) + slot, 0, sizeof(uint32_t), h->stream);
+}
+// The error word of passes run outside the pending slots (benchmark, autotuner), cleared if set.
+bool take_error(ekg_heart *h) {
+    EKG_CUDA(cudaMemcpy(h->err_host, h->ev.err, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    if (*h->err_host) clear_error(h, h->cur);
+    return *h->err_host != 0;
+}
+
 // Hands over a pending batched evaluation: waits for its pass, checks the device error word and
 // writes the criteria and violations to the caller's buffers.
 void complete_pending(ekg_heart *h, int slot) {
@@ -1428,11 +1476,16 @@ void complete_pending(ekg_heart *h, int slot) {
     if (!pd.busy) return;
     pd.busy = false;
     EKG_CUDA(cudaEventSynchronize(pd.done));
-    if (*pd.err) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (error word " + std::to_string(*pd.err) + ")"};
+    const uint32_t err = reinterpret_cast<const uint32_t *>(pd.out)[slot];
+    if (err) {
+        clear_error(h, slot);
+        throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (error word " + std::to_string(err) + ")"};
+    }
+    if (pd.ecg) std::memcpy(pd.ecg, pd.out + pd.ecg_off, pd.ecg_n * sizeof(double));
     if (!pd.criteria) return;
     const int nl = h->dev.nlayers, ncl = h->es.n_crit_leads;
     for (int s = 0; s < pd.n_sims; ++s) {
-        assemble_criteria(h, &pd.crit2[(size_t)s * ncl * 2], pd.done_flags[s] != 0, pd.acrit[s], pd.approx[s],
+        assemble_criteria(h, pd.out + 1 + (size_t)s * ncl * 2, pd.done_flags[s] != 0, pd.acrit[s], pd.approx[s],
                           pd.endo_epi[s], pd.criteria + (size_t)s * h->es.n_criteria);
         pd.violation[s] = pd.viol[s];
     }
@@ -1464,8 +1517,8 @@ void benchmark(ekg_heart *h, int n_sims, const double *layer_k, const double *le
     EKG_CUDA(cudaSetDevice(h->eng->device));
     cudaStream_t s = h->stream;
     const PassPlan P = plan_pass(h, n_sims, layer_k, leads);
-    upload_inputs(h, P, layer_k, leads);
     const int ncl = h->has_eval ? h->es.n_crit_leads : 0;
+    upload_inputs(h, P, layer_k, leads, ncl, true);
     const int mode = h->has_eval ? h->es.comparison_mode : 2;
     // the passes as an evaluation runs them (graph replays, see run_pass); the second warm-up pass
     // captures the graph
@@ -1540,8 +1593,7 @@ void benchmark(ekg_heart *h, int n_sims, const double *layer_k, const double *le
     for (auto &e : tm.ev) cudaEventDestroy(e);
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
-    EKG_CUDA(cudaMemcpy(h->err_host, h->ev.err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    if (*h->err_host) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out"};
+    if (take_error(h)) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out"};
 }
 
 // Times every candidate launch shape of the batched form for a pass of n_sims simulations with these
@@ -1579,7 +1631,7 @@ TuneChoice tune_pass(ekg_heart *h, int n_sims, const double *layer_k, const doub
     for (TuneChoice &c : cands) {
         h->tune_force = &c;
         const PassPlan P = plan_pass(h, n_sims, layer_k, leads);
-        upload_inputs(h, P, layer_k, leads);
+        upload_inputs(h, P, layer_k, leads, ncl, true);
         compute(h, P, ncl, mode, nullptr);
         EKG_CUDA(cudaEventRecord(a, s));
         for (int r = 0; r < reps; ++r) compute(h, P, ncl, mode, nullptr);
@@ -1587,8 +1639,7 @@ TuneChoice tune_pass(ekg_heart *h, int n_sims, const double *layer_k, const doub
         EKG_CUDA(cudaEventSynchronize(b));
         float ms = 0;
         EKG_CUDA(cudaEventElapsedTime(&ms, a, b));
-        EKG_CUDA(cudaMemcpy(h->err_host, h->ev.err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-        if (*h->err_host) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (autotuner)"};
+        if (take_error(h)) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (autotuner)"};
         c.ms = ms / reps;
         const int bN = batch_tile_rows(P0.two_bases, P0.rows_used);
         const bool builtin = c.tile_rows == bN && c.op_small == (n_sims <= small_operand_sims() ? 1 : 0) &&
