@@ -212,10 +212,49 @@ __global__ void __launch_bounds__(CA_THREADS, 3)
     }
 }
 
-__global__ void k_ca_init(size_t n, const uint8_t *__restrict__ layers, const uint8_t *__restrict__ start,
-                          u64 *__restrict__ at) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        at[i] = layers[i] ? (start[i] ? 2 * 0x3ff0000000000000ULL + 1 : 2 * INF_BITS) : 0;
+// The caller's grid: layers stripped of the stimulus sign, the header, and with `at` the entries before
+// round 0 and the stimulus tiles in its list.
+__global__ void __launch_bounds__(256) k_ca_grid(int nz, int ny, int nx, int nty, int ntx, const int32_t *__restrict__ grid,
+                                                 uint8_t *__restrict__ lay, GridHeader *__restrict__ hdr,
+                                                 u64 *__restrict__ at, TileLists T) {
+    __shared__ uint32_t s_present[8];
+    if (threadIdx.x < 8) s_present[threadIdx.x] = 0;
+    __syncthreads();
+    const size_t n = (size_t)nz * ny * nx;
+    int bad = 0, starts = 0, vox = 0, last = 0;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const int32_t v = grid[i];
+        // widened before the negation, so that INT32_MIN is rejected rather than overflowing
+        const int64_t a = v < 0 ? -(int64_t)v : (int64_t)v;
+        if (a > 254) {
+            bad = 1;
+            continue;
+        }
+        lay[i] = (uint8_t)a;
+        vox += a != 0;
+        if (a && (int)a != last) {
+            last = (int)a;
+            atomicOr(&s_present[last >> 5], 1u << (last & 31));
+        }
+        if (v < 0) ++starts;
+        if (at) {
+            at[i] = a ? (v < 0 ? 2 * 0x3ff0000000000000ULL + 1 : 2 * INF_BITS) : 0;
+            if (v < 0) {
+                const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
+                tile_append(T, ((z / TS) * nty + (y / TS)) * ntx + (x / TS), 0);
+            }
+        }
+    }
+    starts = __reduce_add_sync(0xffffffffu, starts);
+    vox = __reduce_add_sync(0xffffffffu, vox);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (starts) atomicAdd(&hdr->nstart, starts);
+        if (vox) atomicAdd(&hdr->nvox, vox);
+        if (bad) atomicOr(&hdr->bad, 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 && s_present[threadIdx.x]) atomicOr(&hdr->present[threadIdx.x], s_present[threadIdx.x]);
 }
 
 // entries -> times; unreachable voxels keep excitationDelay 0
@@ -228,8 +267,8 @@ __global__ void k_ca_finish(size_t n, u64 *__restrict__ at) {
 
 }  // namespace
 
-// The lists over `ctrl` (CA_CTRL_WORDS words) and its words before round 0: the stimulus (time 1.0)
-// pending in n_start tiles.
+// The lists over `ctrl` (CA_CTRL_WORDS words), and its words before round 0, when the stimulus tiles are yet
+// to be appended: the earliest pending time is the stimulus', 1.0.
 static TileLists tile_lists(int32_t *ctrl, uint32_t *flags, int32_t *list, int cap) {
     TileLists T;
     T.counts = ctrl;
@@ -239,12 +278,7 @@ static TileLists tile_lists(int32_t *ctrl, uint32_t *flags, int32_t *list, int c
     T.cap = cap;
     return T;
 }
-static void first_round(int32_t (&ctrl)[CA_CTRL_WORDS], int32_t n_start) {
-    std::fill(ctrl, ctrl + CA_CTRL_WORDS, 0);
-    ctrl[0] = n_start;
-    ctrl[4] = 0x3ff00000;  // high word of 1.0
-    ctrl[5] = ctrl[6] = -1;
-}
+static const int32_t FIRST_ROUND[CA_CTRL_WORDS] = {0, 0, 0, 0, 0x3ff00000 /* high word of 1.0 */, -1, -1};
 
 // The width of a round, 5 of the largest lag between present layers: in a narrower one the rounds' fixed
 // cost shows (launch, staging, write-back), in a wider one the wave leaves the tile and its successors
@@ -286,25 +320,38 @@ static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, 
     }
 }
 
-CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const uint8_t *d_start,
-                const std::vector<int32_t> &start_tiles, const std::vector<double> &lag_h,
-                const std::vector<char> &present, int nl1, const double *d_lag, double *d_at, int round_cap,
-                int sm_count) {
+static int tile_count(int nz, int ny, int nx) {
+    return ((nz + TS - 1) / TS) * ((ny + TS - 1) / TS) * ((nx + TS - 1) / TS);
+}
+// scratch: control words, flags, two lists
+static TileLists scratch_lists(void *scratch, int ntiles) {
+    int32_t *p = static_cast<int32_t *>(scratch);
+    const size_t nflag = (size_t)(ntiles + 3) / 4;
+    return tile_lists(p, reinterpret_cast<uint32_t *>(p + CA_CTRL_WORDS), p + CA_CTRL_WORDS + nflag, ntiles);
+}
+size_t ca_scratch_bytes(int nz, int ny, int nx) {
+    const size_t nt = (size_t)tile_count(nz, ny, nx);
+    return (CA_CTRL_WORDS + (nt + 3) / 4 + 2 * nt) * sizeof(int32_t);
+}
+
+void ca_grid(cudaStream_t s, int nz, int ny, int nx, const int32_t *d_grid, uint8_t *d_lay, GridHeader *d_hdr,
+             double *d_at, void *scratch) {
+    const int nt = tile_count(nz, ny, nx), nty = (ny + TS - 1) / TS, ntx = (nx + TS - 1) / TS;
+    const TileLists T = scratch_lists(scratch, nt);
+    EKG_CUDA(cudaMemsetAsync(T.flags, 0, (size_t)(nt + 3) / 4 * sizeof(int32_t), s));
+    EKG_CUDA(cudaMemsetAsync(d_hdr, 0, sizeof(GridHeader), s));
+    // the kernel appends the stimulus tiles
+    EKG_CUDA(cudaMemcpyAsync(T.counts, FIRST_ROUND, sizeof(FIRST_ROUND), cudaMemcpyHostToDevice, s));
+    k_ca_grid<<<1216, 256, 0, s>>>(nz, ny, nx, nty, ntx, d_grid, d_lay, d_hdr, reinterpret_cast<u64 *>(d_at), T);
+    EKG_CUDA(cudaGetLastError());
+}
+
+CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const std::vector<double> &lag_h,
+                const std::vector<char> &present, int nl1, const double *d_lag, double *d_at, void *scratch,
+                int round_cap, int sm_count) {
     CaResult res;
-    const int ntz = (nz + TS - 1) / TS, nty = (ny + TS - 1) / TS, ntx = (nx + TS - 1) / TS;
-    const int ntiles = ntz * nty * ntx;
-    const size_t n = (size_t)nz * ny * nx, nflag = (size_t)(ntiles + 3) / 4;
-    DBuf<int32_t> buf;  // control words, flags, two lists
-    buf.alloc(CA_CTRL_WORDS + nflag + 2 * (size_t)ntiles);
-    const TileLists T = tile_lists(buf.p, reinterpret_cast<uint32_t *>(buf.p + CA_CTRL_WORDS),
-                                   buf.p + CA_CTRL_WORDS + nflag, ntiles);
-    const int32_t n_start = (int32_t)start_tiles.size();
-    EKG_CUDA(cudaMemsetAsync(T.flags, 0, nflag * sizeof(int32_t), s));
-    int32_t ctrl[CA_CTRL_WORDS];
-    first_round(ctrl, n_start);
-    EKG_CUDA(cudaMemcpyAsync(buf.p, ctrl, sizeof(ctrl), cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(T.list, start_tiles.data(), start_tiles.size() * sizeof(int32_t),
-                             cudaMemcpyHostToDevice, s));
+    const size_t n = (size_t)nz * ny * nx;
+    const TileLists T = scratch_lists(scratch, tile_count(nz, ny, nx));
     struct Events {
         cudaEvent_t a = nullptr, b = nullptr;
         ~Events() {
@@ -316,8 +363,6 @@ CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers,
     EKG_CUDA(cudaEventCreate(&ev.b));
     EKG_CUDA(cudaEventRecord(ev.a, s));
     u64 *entries = reinterpret_cast<u64 *>(d_at);
-    k_ca_init<<<1024, 256, 0, s>>>(n, d_layers, d_start, entries);
-    EKG_CUDA(cudaGetLastError());
     // every round settles at least the voxels with the earliest pending time for good
     const int cap = round_cap > 0 ? round_cap : (int)std::min<size_t>(n, INT32_MAX / 2) + 64;
     res.rounds = run_rounds(s, nz, ny, nx, d_layers, d_lag, nl1, round_window(lag_h.data(), nl1, present.data()),
@@ -465,9 +510,8 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
             }
         EKG_CUDA(cudaMemcpy(sc->lag, lag, (size_t)nl1 * nl1 * 3 * sizeof(double), cudaMemcpyHostToDevice));
         const TileLists T = tile_lists(sc->ctrl, sc->flag, sc->list[0], NOALLOC_MAX_TILES);
-        int32_t ctrl[CA_CTRL_WORDS];
-        first_round(ctrl, 0);  // k_na_init appends the stimulus tiles
-        EKG_CUDA(cudaMemcpy(sc->ctrl, ctrl, sizeof(ctrl), cudaMemcpyHostToDevice));
+        // k_na_init appends the stimulus tiles
+        EKG_CUDA(cudaMemcpy(sc->ctrl, FIRST_ROUND, sizeof(FIRST_ROUND), cudaMemcpyHostToDevice));
         u64 *entries = reinterpret_cast<u64 *>(d_at);
         k_na_init<<<1024, 256, 0, s>>>(nz, ny, nx, nty, ntx, d_layers, entries, T);
         EKG_CUDA(cudaGetLastError());

@@ -17,6 +17,7 @@ struct ekg_engine {
     int contract = 0;
     bool batched = true;  // separable batched form for multi-simulation passes (EKG_BATCHED=0 disables)
     int batch_ctas = 0;   // target CTAs of the moved-lead GEMM (0 = one wave)
+    int sm_count = 152;
     bool graphs = true;   // replay repeated passes as CUDA graphs (EKG_GRAPHS=0 disables)
     // rounds after which the activation-time relaxation gives up with EKG_ERR_CA_NOT_CONVERGED
     // (0 = the default bound from the grid size; EKG_CA_ROUND_CAP sets it, e.g. to test that error)
@@ -116,7 +117,6 @@ struct ekg_heart {
     // the moved-lead operand kernel and GEMM (fork and join by events; captured into the graphs)
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_op = nullptr, ev_join = nullptr;
-    uint32_t *err_host = nullptr;     // pinned copy of the kernels' error word
     // device passes captured as CUDA graphs, keyed by everything their launches depend on
     struct PassGraph {
         std::vector<uint64_t> sig;
@@ -188,7 +188,6 @@ struct ekg_heart {
         if (aux_stream) cudaStreamDestroy(aux_stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         if (stream) cudaStreamDestroy(stream);
-        if (err_host) cudaFreeHost(err_host);
     }
     std::mutex mu;
     int nz = 0, ny = 0, nx = 0, nhood = 0;
@@ -200,10 +199,11 @@ struct ekg_heart {
     std::vector<double> leads0;       // loaded lead positions (z,y,x)
     std::vector<double> lead_uv;      // their displacement frames [n][u, v]
     std::vector<double> at_host;      // activation time per cell (copied from the device on first use)
-    std::vector<uint8_t> layer_host;  // layer id per cell (stimulus flag stripped)
     std::vector<int64_t> ap_index_ref;    // reference AP numbering per cell (built on demand)
-    std::vector<int32_t> vox_cell;        // cell of each voxel, voxels in AP order
-    std::vector<int32_t> vox_group_start; // [naps + 1] first voxel of each AP
+    ekg::Arena cells_mem, mem;  // behind the arrays per cell, and behind the others of the heart
+    ekg::DBuf<uint8_t> layers_dev;        // layer id per cell (stimulus flag stripped)
+    ekg::DBuf<int32_t> vox_cell_dev;      // cell of each voxel, voxels in AP order
+    ekg::DBuf<int32_t> vox_start_dev;     // [naps] first voxel of each AP
     ekg::HeartDev dev;
     ekg::EvalDev ev;
     ekg::DBuf<double> at_cells;       // device activation times per cell

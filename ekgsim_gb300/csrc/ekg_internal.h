@@ -83,11 +83,12 @@ template <class T>
 struct DBuf {
     T *p = nullptr;
     size_t n = 0;
+    bool own = true;  // false: a part of an Arena
     DBuf() = default;
     DBuf(const DBuf &) = delete;
     DBuf &operator=(const DBuf &) = delete;
     ~DBuf() { release(); }
-    DBuf(DBuf &&o) noexcept : p(o.p), n(o.n) {
+    DBuf(DBuf &&o) noexcept : p(o.p), n(o.n), own(o.own) {
         o.p = nullptr;
         o.n = 0;
     }
@@ -96,15 +97,23 @@ struct DBuf {
             release();
             p = o.p;
             n = o.n;
+            own = o.own;
             o.p = nullptr;
             o.n = 0;
         }
         return *this;
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p && own) cudaFree(p);
         p = nullptr;
         n = 0;
+        own = true;
+    }
+    void view(T *q, size_t count) {
+        release();
+        p = q;
+        n = count;
+        own = false;
     }
     void alloc(size_t count) {
         if (count == n && p) return;
@@ -121,18 +130,51 @@ struct DBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
+// One allocation cut into 256-byte aligned parts: cudaMalloc and cudaFree cost 10 to 20 us each (and
+// cudaFree waits for the device), so arrays that live and die together share one.
+struct Arena {
+    DBuf<uint8_t> mem;
+    size_t used = 0;
+    static size_t part(size_t bytes) { return (bytes + 255) / 256 * 256; }
+    void reserve(size_t bytes) {
+        mem.alloc(bytes);
+        used = 0;
+    }
+    template <class T>
+    T *take(size_t count) {
+        T *q = reinterpret_cast<T *>(mem.p + used);
+        used += part(count * sizeof(T));
+        if (used > mem.n) throw Error{EKG_ERR_DEVICE, "arena too small"};
+        return q;
+    }
+    template <class T>
+    void place(DBuf<T> &b, size_t count) {
+        b.view(take<T>(count), count);
+    }
+};
+
 // ------------------------------------------------------------------ CA (ca.cu)
 struct CaResult {
     int rounds = 0;  // rounds that had a tile
     float ms = 0.f;
 };
-// layers_u8: stripped layer per cell; start flags in `is_start`; lag: [nl1][nl1][3] FP64 with
-// lag[s][d][k-1] = T[s][d] * sqrt(k) (lag_h the same on the host, present[layer] != 0 where the heart has
-// the layer).  at_out: FP64 per cell (0 for empty / unreachable).
-CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const uint8_t *d_start,
-                const std::vector<int32_t> &start_tiles, const std::vector<double> &lag_h,
-                const std::vector<char> &present, int nl1, const double *d_lag, double *d_at, int round_cap,
-                int sm_count);
+// What a layer grid holds: bit a of `present` for layer a, layer ids out of range, stimulus voxels,
+// non-empty voxels.
+struct GridHeader {
+    uint32_t present[8];
+    int32_t bad, nstart, nvox;
+};
+// bytes of the relaxation's device scratch (lists and flags of its tiles)
+size_t ca_scratch_bytes(int nz, int ny, int nx);
+// One pass over the caller's grid (0 empty, L > 0 layer, -L stimulus voxel of layer L): stripped layers
+// to d_lay, the header to d_hdr, and with d_at the relaxation's start (d_at, scratch) for ca_run.
+void ca_grid(cudaStream_t s, int nz, int ny, int nx, const int32_t *d_grid, uint8_t *d_lay, GridHeader *d_hdr,
+             double *d_at, void *scratch);
+// lag: [nl1][nl1][3] FP64 with lag[s][d][k-1] = T[s][d] * sqrt(k) (lag_h the same on the host,
+// present[layer] != 0 where the heart has the layer).  d_at: FP64 per cell (0 for empty / unreachable).
+CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers, const std::vector<double> &lag_h,
+                const std::vector<char> &present, int nl1, const double *d_lag, double *d_at, void *scratch,
+                int round_cap, int sm_count);
 
 // ------------------------------------------------------------------ ECG kernels (ecg.cu)
 // Heart-resident device arrays used by the simulation kernels.
@@ -147,7 +189,7 @@ struct HeartDev {
     DBuf<double> at;        // [apad]
     DBuf<int32_t> a_layer;  // [apad] layer index 0-based (pad: layer of its chunk)
     DBuf<int64_t> a_vox_begin;  // [apad + 1] voxel ranges (voxels sorted by AP)
-    // per voxel (sorted by AP)
+    // per voxel (sorted by AP); the first three only while the heart is set up
     DBuf<int32_t> vox_zyx;  // [nvox] packed z<<20 | y<<10 | x  (each < 1024)
     DBuf<uint32_t> vox_nb;  // [nvox] bits 0..25: in-neighbour mask, (unused high bits)
     DBuf<uint32_t> vox_nbo; // [nvox] out-neighbour mask
@@ -181,23 +223,34 @@ struct DedupResult {
     int64_t nvox = 0, naps = 0, apad = 0;
     std::vector<int> pl_layer, pfirst, pcount;  // per present layer: id (1-based), first AP, APs
     std::vector<int64_t> pbase;                  // per present layer: first padded AP slot
-    DBuf<int> cell;                              // [nvox] cell of each sorted voxel
-    DBuf<int> gstart;                            // [naps (+1)] first sorted voxel of each AP
-    DBuf<uint64_t> key;                          // [nvox] activation-time bits of each sorted voxel
-    DBuf<uint8_t> vl;                            // [nvox] layer of each sorted voxel
+    // in the scratch arena
+    int *cell = nullptr;      // [nvox] cell of each sorted voxel
+    int *gstart = nullptr;    // [naps (+1)] first sorted voxel of each AP
+    uint64_t *key = nullptr;  // [nvox] activation-time bits of each sorted voxel
+    uint8_t *vl = nullptr;    // [nvox] layer of each sorted voxel
+    // the sort's other buffers, free for the stage order
+    uint64_t *key2 = nullptr;
+    uint8_t *vl2 = nullptr;
+    int *cell2 = nullptr, *hist = nullptr, *totals = nullptr, *base = nullptr, *tsum = nullptr;
+    unsigned long long *n_interior = nullptr;
 };
+size_t setup_scratch_bytes(int64_t n_cells, int64_t nvox);
 void setup_voxels_device(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_lay, const double *d_at_cells,
-                         int nl, DedupResult &r);
-// at / at_hilo / a_layer [apad], a_vb [apad + 1]
-void setup_ap_arrays_device(cudaStream_t s, const DedupResult &r, const double *d_at_cells, double *at,
-                            float2 *at_hilo, int32_t *a_layer, int64_t *a_vb);
-// per-voxel records of the dipole kernels; returns the number of voxels flagged interior
+                         int nl, int64_t nvox, Arena &scratch, DedupResult &r);
+// at / at_hilo / a_layer [apad], a_vb [apad + 1]; the tables (setup_ap_tables) are on the device
+size_t setup_ap_tables(const DedupResult &r, uint8_t *host);  // writes them (host not null), returns their bytes
+void setup_ap_arrays_device(cudaStream_t s, const DedupResult &r, const uint8_t *d_tables, const double *d_at_cells,
+                            double *at, float2 *at_hilo, int32_t *a_layer, int64_t *a_vb);
+// per-voxel records of the dipole kernels; the number of voxels flagged interior goes to r.n_interior
+void setup_voxel_records_device(cudaStream_t s, const DedupResult &r, int nz, int ny, int nx, const uint8_t *d_lay,
+                                const HeartDev &D, int few_max, int32_t *vzyx, uint32_t *vin, uint32_t *vout,
+                                float4 *vpos, float4 *vosum);
 // Bounding box of each 32-AP stage's voxel positions (empty stages: an inverted box).
 void setup_stage_boxes_device(cudaStream_t s, int64_t apad, const int64_t *a_vox_begin, const float4 *vox_pos,
                               float4 *stage_box);
-int64_t setup_voxel_records_device(cudaStream_t s, const DedupResult &r, int nz, int ny, int nx, const uint8_t *d_lay,
-                                   const HeartDev &D, int few_max, int32_t *vzyx, uint32_t *vin, uint32_t *vout,
-                                   float4 *vpos, float4 *vosum);
+// Stages by descending voxel count, ties by index (the field kernels' item order).  Uses the sort's
+// buffers of r: the voxel lists are not valid afterwards.
+void setup_stage_order_device(cudaStream_t s, DedupResult &r, const int64_t *a_vox_begin, int32_t *stage_order);
 
 // Per-evaluation scratch (sized for n_sims simulations).
 struct EvalDev {

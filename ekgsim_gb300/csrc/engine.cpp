@@ -237,48 +237,37 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
         }
     }
 
-    // layers, stimulus, validation: in parts on the host pool (per part its largest layer, present
-    // layers, first out-of-range cell and stimulus cells in order)
-    std::vector<uint8_t> lay(n), st(n);
-    const size_t vparts = (size_t)std::min<int64_t>(64, std::max<int64_t>(1, n / 65536));
-    struct Part {
-        int nl = 0;
-        int64_t bad = -1;
-        std::vector<int64_t> starts;
-        char present[256] = {0};
-    };
-    std::vector<Part> parts(vparts);
-    HostPool::get().run(vparts, [&](size_t pb, size_t pe) {
-        for (size_t q = pb; q < pe; ++q) {
-            Part &P = parts[q];
-            for (int64_t i = n * (int64_t)q / (int64_t)vparts; i < n * (int64_t)(q + 1) / (int64_t)vparts; ++i) {
-                const int32_t v = d->layers[i];
-                // widened before the negation, so that INT32_MIN is rejected rather than overflowing
-                const int64_t a = v < 0 ? -(int64_t)v : (int64_t)v;
-                if (a > 254) {
-                    if (P.bad < 0) P.bad = i;
-                    continue;
-                }
-                lay[i] = (uint8_t)a;
-                st[i] = v < 0;
-                if (v < 0) P.starts.push_back(i);
-                P.nl = std::max(P.nl, (int)a);
-                P.present[a] = 1;
-            }
-        }
-    });
+    // the grid goes to the device as it is, where one pass strips and validates it and prepares the relaxation
+    const bool loaded = d->activation_in != nullptr;
+    EKG_CHECK(n < ((int64_t)1 << 31), EKG_ERR_BAD_INPUT, "grid too large");
+    EKG_CUDA(cudaSetDevice(h->eng->device));
+    if (!h->stream) EKG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+    h->sm_count = h->eng->sm_count;
+    cudaStream_t s = h->stream;
+    h->cells_mem.reserve(Arena::part(n) + Arena::part(n * 8));
+    h->cells_mem.place(h->layers_dev, n);
+    h->cells_mem.place(h->at_cells, n);
+    Arena first;  // until the relaxation is done
+    first.reserve(Arena::part(n * 4) + Arena::part(ca_scratch_bytes(d->nz, d->ny, d->nx)) + Arena::part(sizeof(GridHeader)));
+    int32_t *d_grid = first.take<int32_t>(n);
+    uint8_t *ca_scratch = first.take<uint8_t>(ca_scratch_bytes(d->nz, d->ny, d->nx));
+    GridHeader *d_hdr = first.take<GridHeader>(1);
+    EKG_CUDA(cudaMemcpyAsync(d_grid, d->layers, n * 4, cudaMemcpyHostToDevice, s));
+    ca_grid(s, d->nz, d->ny, d->nx, d_grid, h->layers_dev.p, d_hdr, loaded ? nullptr : h->at_cells.p, ca_scratch);
+    GridHeader hdr;
+    EKG_CUDA(cudaMemcpyAsync(&hdr, d_hdr, sizeof(hdr), cudaMemcpyDeviceToHost, s));
+    EKG_CUDA(cudaStreamSynchronize(s));
+    EKG_CHECK(!hdr.bad, EKG_ERR_BAD_INPUT, "layer ids must be at most 254");
     int nl = 0;
-    int64_t nstart = 0;
+    const int64_t nstart = hdr.nstart;
     std::vector<char> present(256, 0);
-    for (const Part &P : parts) {
-        EKG_CHECK(P.bad < 0, EKG_ERR_BAD_INPUT, "layer ids must be at most 254");
-        nl = std::max(nl, P.nl);
-        nstart += (int64_t)P.starts.size();
-        for (int a = 0; a < 256; ++a) present[a] = present[a] || P.present[a];
-    }
+    for (int a = 1; a < 256; ++a)
+        if ((hdr.present[a >> 5] >> (a & 31)) & 1u) {
+            present[a] = 1;
+            nl = a;
+        }
     // a loaded sequence replaces the automaton (simlib/sim_lib.h:224-231): the stimulus and the
     // conduction matrix are not used then
-    const bool loaded = d->activation_in != nullptr;
     EKG_CHECK(loaded || nstart > 0, EKG_ERR_NO_START, "Could not find starting point for excitation sequence");
     EKG_CHECK(nl >= 1, EKG_ERR_BAD_INPUT, "model has no non-empty voxel");
     D.nlayers = nl;
@@ -287,7 +276,7 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
     std::vector<double> lag((size_t)nl1 * nl1 * 3, 0.0);
     if (loaded) {
         for (int64_t i = 0; i < n; ++i)
-            if (lay[i]) {
+            if (d->layers[i] != 0) {
                 const double v = d->activation_in[i];
                 EKG_CHECK(std::isfinite(v) && v >= 0, EKG_ERR_BAD_INPUT,
                           "loaded activation times of non-empty cells must be finite and non-negative");
@@ -311,73 +300,36 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
                     lag[((size_t)s * nl1 + t) * 3 + (k - 1)] = l;
                 }
     }
-    std::vector<int32_t> start_tiles;
-    {
-        const int ntx = (d->nx + 7) / 8, nty = (d->ny + 7) / 8;
-        std::vector<char> seen((size_t)ntx * nty * ((d->nz + 7) / 8), 0);
-        for (const Part &P : parts)
-            for (const int64_t i : P.starts) {
-                const int64_t z = i / ((int64_t)d->ny * d->nx), y = (i / d->nx) % d->ny, x = i % d->nx;
-                const int64_t tile = ((z / 8) * nty + (y / 8)) * ntx + (x / 8);
-                if (!seen[tile]) {
-                    seen[tile] = 1;
-                    start_tiles.push_back((int32_t)tile);
-                }
-            }
-    }
-
-    h->layer_host.assign(lay.begin(), lay.end());
-    // activation times on the device
-    EKG_CUDA(cudaSetDevice(h->eng->device));
-    if (!h->stream) EKG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-    if (!h->aux_stream) {
-        EKG_CUDA(cudaStreamCreateWithFlags(&h->aux_stream, cudaStreamNonBlocking));
-        for (cudaEvent_t *e : {&h->ev_fork, &h->ev_op, &h->ev_join})
-            EKG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    }
-    if (!h->err_host) EKG_CUDA(cudaMallocHost(&h->err_host, sizeof(uint32_t)));
-    EKG_CUDA(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->eng->device));
-    h->ev.basis_err.alloc(1);
-    cudaStream_t s = h->stream;
-    // activation times (the layer grid stays on the device for the de-duplication)
-    DBuf<uint8_t> dl;
-    dl.alloc(n);
-    EKG_CUDA(cudaMemcpyAsync(dl.p, lay.data(), n, cudaMemcpyHostToDevice, s));
+    // the sort's scratch, the lag table and the records that only the set-up reads
+    const int64_t nv = hdr.nvox;
+    h->nvox = nv;
+    D.nvox = nv;
+    Arena scratch;
+    scratch.reserve(setup_scratch_bytes(n, nv) + Arena::part(lag.size() * 8) + 3 * Arena::part(nv * 4));
     if (loaded) {
         // -0.0 keys like +0.0 in the reference's std::map (simlib/simulator.cpp:570-590)
         std::vector<double> at_in(d->activation_in, d->activation_in + n);
         for (double &v : at_in)
             if (v == 0.0) v = 0.0;
-        h->at_cells.alloc(n);
         EKG_CUDA(cudaMemcpyAsync(h->at_cells.p, at_in.data(), n * 8, cudaMemcpyHostToDevice, s));
         h->ca_rounds = 0;
         h->ca_ms = 0;
         EKG_CUDA(cudaStreamSynchronize(s));
     } else {
-        DBuf<uint8_t> ds;
-        DBuf<double> dlag;
-        ds.alloc(n);
-        dlag.alloc(lag.size());
-        h->at_cells.alloc(n);
-        EKG_CUDA(cudaMemcpyAsync(ds.p, st.data(), n, cudaMemcpyHostToDevice, s));
-        EKG_CUDA(cudaMemcpyAsync(dlag.p, lag.data(), lag.size() * 8, cudaMemcpyHostToDevice, s));
-        const CaResult r = ca_run(s, d->nz, d->ny, d->nx, dl.p, ds.p, start_tiles, lag, present, nl1, dlag.p,
-                                  h->at_cells.p, h->eng->ca_round_cap, h->sm_count);
+        double *d_lag = scratch.take<double>(lag.size());
+        EKG_CUDA(cudaMemcpyAsync(d_lag, lag.data(), lag.size() * 8, cudaMemcpyHostToDevice, s));
+        const CaResult r = ca_run(s, d->nz, d->ny, d->nx, h->layers_dev.p, lag, present, nl1, d_lag, h->at_cells.p,
+                                  ca_scratch, h->eng->ca_round_cap, h->sm_count);
         h->ca_rounds = r.rounds;
         h->ca_ms = r.ms;
-        EKG_CUDA(cudaStreamSynchronize(s));
     }
-    h->at_host.clear();  // copied to the host on first use (ensure_at_host)
 
     // de-duplicate (layer, at) pairs on the device (setup.cu): voxels sorted by (layer, at bits,
     // cell), equal (layer, at) runs are the APs.  The reference numbers APs by first appearance in
     // raster order (simlib/simulator.cpp:570-590); that numbering is derived on demand.
-    EKG_CHECK(n < ((int64_t)1 << 31), EKG_ERR_BAD_INPUT, "grid too large");
     DedupResult dd;
-    setup_voxels_device(s, d->nz, d->ny, d->nx, dl.p, h->at_cells.p, nl, dd);
-    const int64_t nv = dd.nvox, na = dd.naps, apad = dd.apad;
-    h->nvox = nv;
-    D.nvox = nv;
+    setup_voxels_device(s, d->nz, d->ny, d->nx, h->layers_dev.p, h->at_cells.p, nl, nv, scratch, dd);
+    const int64_t na = dd.naps, apad = dd.apad, nst = apad / 32;
     h->naps = na;
     D.naps = na;
     EKG_CHECK(apad < (int64_t)1 << 31, EKG_ERR_BAD_INPUT, "too many distinct activation times");
@@ -399,58 +351,6 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
     D.nchunks = (int)c0.size();
     D.chunk_max = 0;
     for (size_t k = 0; k < c0.size(); ++k) D.chunk_max = std::max(D.chunk_max, c1[k] - c0[k]);
-    D.at.alloc(apad);
-    D.at_hilo.alloc(apad);
-    D.a_layer.alloc(apad);
-    D.a_vox_begin.alloc(apad + 1);
-    D.vox_zyx.alloc(nv);
-    D.vox_nb.alloc(nv);
-    D.vox_nbo.alloc(nv);
-    D.vox_pos.alloc(nv);
-    D.vox_out.alloc(nv);
-    D.chunk_a0.alloc(c0.size());
-    D.chunk_a1.alloc(c0.size());
-    D.chunk_layer.alloc(c0.size());
-    D.difs.alloc(3 * D.nnb);
-    D.t.alloc(steps);
-    D.t_hilo.alloc(steps);
-    setup_ap_arrays_device(s, dd, h->at_cells.p, D.at.p, D.at_hilo.p, D.a_layer.p, D.a_vox_begin.p);
-    // absent neighbours up to which the closed form minus their terms is cheaper than the sum over
-    // the present ones (the 8 body diagonals have a cheaper direct sum)
-    const int few_max = D.nhood == EKG_NHOOD_3D4 ? 2 : D.nnb / 2;
-    D.n_interior = setup_voxel_records_device(s, dd, d->nz, d->ny, d->nx, dl.p, D, few_max, D.vox_zyx.p, D.vox_nb.p,
-                                              D.vox_nbo.p, D.vox_pos.p, D.vox_out.p);
-    D.stage_box.alloc((size_t)2 * (apad / 32));
-    setup_stage_boxes_device(s, apad, D.a_vox_begin.p, D.vox_pos.p, D.stage_box.p);
-    {
-        // work items of the moved-lead field kernels: stages with the most voxels first
-        // (longest-first), ties by index
-        const int64_t nst = apad / 32;
-        std::vector<int64_t> vb(apad + 1);
-        EKG_CUDA(cudaMemcpyAsync(vb.data(), D.a_vox_begin.p, vb.size() * 8, cudaMemcpyDeviceToHost, s));
-        EKG_CUDA(cudaStreamSynchronize(s));
-        std::vector<int32_t> order(nst);
-        for (int64_t st = 0; st < nst; ++st) order[st] = (int32_t)st;
-        std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-            return vb[32 * (a + 1)] - vb[32 * a] > vb[32 * (b + 1)] - vb[32 * b];
-        });
-        D.stage_order.alloc(nst);
-        EKG_CUDA(cudaMemcpy(D.stage_order.p, order.data(), nst * 4, cudaMemcpyHostToDevice));
-    }
-    // host copies of the sorted voxel cells and AP starts, for the reference's AP numbering
-    h->vox_cell.resize(nv);
-    h->vox_group_start.resize(na + 1);
-    EKG_CUDA(cudaMemcpyAsync(h->vox_cell.data(), dd.cell.p, nv * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    EKG_CUDA(cudaMemcpyAsync(h->vox_group_start.data(), dd.gstart.p, na * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    h->ap_index_ref.clear();
-    std::vector<float2> th(steps);
-    for (int64_t i = 0; i < steps; ++i) {
-        const float hi = (float)h->t[i];
-        th[i] = make_float2(hi, (float)(h->t[i] - (double)hi));
-    }
-    EKG_CUDA(cudaMemcpyAsync(D.chunk_a0.p, c0.data(), c0.size() * 4, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(D.chunk_a1.p, c1.data(), c0.size() * 4, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(D.chunk_layer.p, cl.data(), c0.size() * 4, cudaMemcpyHostToDevice, s));
     // chunk range of each layer (a layer's chunks are contiguous)
     std::vector<int32_t> lc0v(nl, 0), lc1v(nl, 0);
     for (size_t k = 0; k < cl.size(); ++k) {
@@ -458,29 +358,84 @@ void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {
         if (lc0v[L] == lc1v[L]) lc0v[L] = (int32_t)k;
         lc1v[L] = (int32_t)k + 1;
     }
-    D.layer_c0.alloc(nl);
-    D.layer_c1.alloc(nl);
-    EKG_CUDA(cudaMemcpyAsync(D.layer_c0.p, lc0v.data(), nl * 4, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(D.layer_c1.p, lc1v.data(), nl * 4, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(D.difs.p, D.nb_dif, 3 * D.nnb, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(D.t.p, h->t.data(), steps * 8, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(D.t_hilo.p, th.data(), steps * 8, cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaStreamSynchronize(s));
-    h->vox_group_start[na] = (int32_t)nv;
+    std::vector<float2> th(steps);
+    for (int64_t i = 0; i < steps; ++i) {
+        const float hi = (float)h->t[i];
+        th[i] = make_float2(hi, (float)(h->t[i] - (double)hi));
+    }
+    // the heart's arrays, in one allocation; the small ones that the host fills come first and travel
+    // in one copy
+    const size_t nch = c0.size(), tables = setup_ap_tables(dd, nullptr);
+    auto P = [](size_t bytes) { return Arena::part(bytes); };
+    h->mem.reserve(P(nch * 4) * 3 + P(nl * 4) * 2 + P(3 * D.nnb) + P(steps * 8) * 2 + P(h->leads0.size() * 8) + P(tables) +
+                   P(apad * 8) * 2 + P(apad * 4) + P((apad + 1) * 8) + P(nv * 16) * 2 + P(2 * nst * 16) + P(nst * 4) +
+                   P((size_t)D.nleads * apad * 4) + P(nv * 4) + P(na * 4));
+    h->mem.place(D.chunk_a0, nch);
+    h->mem.place(D.chunk_a1, nch);
+    h->mem.place(D.chunk_layer, nch);
+    h->mem.place(D.layer_c0, nl);
+    h->mem.place(D.layer_c1, nl);
+    h->mem.place(D.difs, 3 * D.nnb);
+    h->mem.place(D.t, steps);
+    h->mem.place(D.t_hilo, steps);
+    h->mem.place(h->leads0_dev, h->leads0.size());
+    uint8_t *d_tables = h->mem.take<uint8_t>(tables);
+    std::vector<uint8_t> blob(h->mem.used);
+    auto put = [&](const void *dev, const void *src, size_t bytes) {
+        std::memcpy(blob.data() + (static_cast<const uint8_t *>(dev) - h->mem.mem.p), src, bytes);
+    };
+    put(D.chunk_a0.p, c0.data(), nch * 4);
+    put(D.chunk_a1.p, c1.data(), nch * 4);
+    put(D.chunk_layer.p, cl.data(), nch * 4);
+    put(D.layer_c0.p, lc0v.data(), nl * 4);
+    put(D.layer_c1.p, lc1v.data(), nl * 4);
+    put(D.difs.p, D.nb_dif, 3 * D.nnb);
+    put(D.t.p, h->t.data(), steps * 8);
+    put(D.t_hilo.p, th.data(), steps * 8);
+    put(h->leads0_dev.p, h->leads0.data(), h->leads0.size() * 8);
+    setup_ap_tables(dd, blob.data() + (d_tables - h->mem.mem.p));
+    EKG_CUDA(cudaMemcpyAsync(h->mem.mem.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, s));
+    h->mem.place(D.at, apad);
+    h->mem.place(D.at_hilo, apad);
+    h->mem.place(D.a_layer, apad);
+    h->mem.place(D.a_vox_begin, apad + 1);
+    h->mem.place(D.vox_pos, nv);
+    h->mem.place(D.vox_out, nv);
+    h->mem.place(D.stage_box, 2 * nst);
+    h->mem.place(D.stage_order, nst);
+    h->mem.place(h->W0, (size_t)D.nleads * apad);
+    h->mem.place(h->vox_cell_dev, nv);
+    h->mem.place(h->vox_start_dev, na);
+    scratch.place(D.vox_zyx, nv);
+    scratch.place(D.vox_nb, nv);
+    scratch.place(D.vox_nbo, nv);
+    setup_ap_arrays_device(s, dd, d_tables, h->at_cells.p, D.at.p, D.at_hilo.p, D.a_layer.p, D.a_vox_begin.p);
+    // absent neighbours up to which the closed form minus their terms is cheaper than the sum over
+    // the present ones (the 8 body diagonals have a cheaper direct sum)
+    const int few_max = D.nhood == EKG_NHOOD_3D4 ? 2 : D.nnb / 2;
+    setup_voxel_records_device(s, dd, d->nz, d->ny, d->nx, h->layers_dev.p, D, few_max, D.vox_zyx.p, D.vox_nb.p,
+                               D.vox_nbo.p, D.vox_pos.p, D.vox_out.p);
+    unsigned long long n_interior = 0;
+    EKG_CUDA(cudaMemcpyAsync(&n_interior, dd.n_interior, sizeof(n_interior), cudaMemcpyDeviceToHost, s));
+    setup_stage_boxes_device(s, apad, D.a_vox_begin.p, D.vox_pos.p, D.stage_box.p);
+    // the sorted voxel cells and AP starts, for the reference's AP numbering (fetched on demand)
+    EKG_CUDA(cudaMemcpyAsync(h->vox_cell_dev.p, dd.cell, nv * 4, cudaMemcpyDeviceToDevice, s));
+    EKG_CUDA(cudaMemcpyAsync(h->vox_start_dev.p, dd.gstart, na * 4, cudaMemcpyDeviceToDevice, s));
+    // work items of the moved-lead field kernels: stages with the most voxels first (longest-first), ties
+    // by index
+    setup_stage_order_device(s, dd, D.a_vox_begin.p, D.stage_order.p);
     // resident lead field for the loaded lead positions
-    h->leads0_dev.alloc(3 * D.nleads);
-    EKG_CUDA(cudaMemcpyAsync(h->leads0_dev.p, h->leads0.data(), h->leads0.size() * 8, cudaMemcpyHostToDevice, s));
-    h->W0.alloc((size_t)D.nleads * apad);
     launch_lead_field(s, D, h->leads0_dev.p, D.nleads, D.nleads, 1, h->W0.p, D.nleads);
     EKG_CUDA(cudaStreamSynchronize(s));
+    D.n_interior = (int64_t)n_interior;
+    D.vox_zyx.release();
+    D.vox_nb.release();
+    D.vox_nbo.release();
     h->setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
 int64_t heart_device_bytes(const ekg_heart *h) {
-    const HeartDev &D = h->dev;
-    int64_t b = D.at.bytes() + D.at_hilo.bytes() + D.a_layer.bytes() + D.a_vox_begin.bytes() + D.vox_zyx.bytes() +
-                D.vox_nb.bytes() + D.vox_nbo.bytes() + D.chunk_a0.bytes() * 3 + D.t.bytes() + D.t_hilo.bytes() +
-                h->W0.bytes() + h->at_cells.bytes() + D.vox_pos.bytes() + D.vox_out.bytes() + D.stage_box.bytes();
+    int64_t b = (int64_t)h->cells_mem.mem.bytes() + (int64_t)h->mem.mem.bytes();
     const EvalDev &E = h->ev;
     b += (int64_t)h->stg[0].dev.bytes() + (int64_t)h->stg[1].dev.bytes() + E.layer_c.bytes() + E.F.bytes() + E.k0w.bytes() + E.W.bytes() +
          E.Wp.bytes() + E.partial.bytes() + E.out.bytes() + E.ecg_ff.bytes() + E.coef.bytes() + E.targets.bytes() +
@@ -534,10 +489,8 @@ void ensure_general_capacity(ekg_heart *h, int n_sims) {
     const HeartDev &D = h->dev;
     const size_t S = (size_t)n_sims;
     const size_t nw = S * D.nleads * D.apad, np = S * D.nchunks * D.nleads * D.steps;
-    if (E.W.n < nw) {
-        E.W.alloc(nw);
-        E.Wp.alloc(nw);
-    }
+    if (E.W.n < nw) E.W.alloc(nw);
+    if (!band_contraction(h) && E.Wp.n < nw) E.Wp.alloc(nw);
     if (E.work.n < 1) E.work.alloc(1);
     if (band_contraction(h)) {
         if (E.band.n < np) E.band.alloc(np);
@@ -774,13 +727,15 @@ void ensure_basis(ekg_heart *h, const std::vector<double> &key) {
         A.layer_c = lc.p;
         A.F = ones.p;
         A.partial = part.p;
+        h->ev.basis_err.alloc(1);
         A.err = h->ev.basis_err.p;
         EKG_CUDA(cudaMemsetAsync(h->ev.basis_err.p, 0, 4, s));
         launch_contract_umma_args(s, A);
         launch_reduce_layers(s, D.steps, rows, nl, B.lc0.p, B.lc1.p, part.p, basis == 0 ? B.Q1.p : B.Q2.p);
-        EKG_CUDA(cudaMemcpyAsync(h->err_host, h->ev.basis_err.p, 4, cudaMemcpyDeviceToHost, s));
+        uint32_t err = 0;
+        EKG_CUDA(cudaMemcpyAsync(&err, h->ev.basis_err.p, 4, cudaMemcpyDeviceToHost, s));
         EKG_CUDA(cudaStreamSynchronize(s));
-        if (*h->err_host) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (basis build)"};
+        if (err) throw Error{EKG_ERR_TIMEOUT, "a bounded device wait ran out (basis build)"};
     }
     build_band(h, key, at_h, al);
     B.J = J;
@@ -1116,11 +1071,16 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     // (measured: other placements of the small kernels, such as the criteria of the static leads
     // beside the GEMM, lengthen the pass)
     const bool fork = P.batch && nmove > 0;
-    cudaStream_t sx = fork ? h->aux_stream : s;
     if (fork) {
+        if (!h->aux_stream) {
+            EKG_CUDA(cudaStreamCreateWithFlags(&h->aux_stream, cudaStreamNonBlocking));
+            for (cudaEvent_t *e : {&h->ev_fork, &h->ev_op, &h->ev_join})
+                EKG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        }
         EKG_CUDA(cudaEventRecord(h->ev_fork, s));
-        EKG_CUDA(cudaStreamWaitEvent(sx, h->ev_fork, 0));
+        EKG_CUDA(cudaStreamWaitEvent(h->aux_stream, h->ev_fork, 0));
     }
+    cudaStream_t sx = fork ? h->aux_stream : s;
     launch_layer_factors(sx, D, in.layer_k, in.cpre, n_sims, E.F.p, E.Ff.p, E.layer_c.p,
                          P.batch ? h->bs.d_centre.p : nullptr, P.batch ? h->bs.d_scale.p : nullptr, P.J,
                          P.batch ? E.coef.p : nullptr);
@@ -1392,11 +1352,6 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
     cudaStream_t s = h->stream;
     ekg_heart::Pending &pd = h->pend[h->cur];
     EKG_CUDA(cudaSetDevice(h->eng->device));
-    if (!h->copy_stream) {
-        EKG_CUDA(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-        for (cudaEvent_t *e : {&h->static_done, &h->moved_done, &h->copies_done, &h->pass_end})
-            EKG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    }
     if (!pd.done) EKG_CUDA(cudaEventCreateWithFlags(&pd.done, cudaEventDisableTiming));
     const size_t L = D.nleads, S = n_sims, T = D.steps;
     // a small ECG comes with the criteria in the pass's own copy to pinned memory and is handed over from
@@ -1433,6 +1388,11 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
         EKG_CUDA(cudaEventRecord(pd.done, s));
         return;
     }
+    if (!h->copy_stream) {
+        EKG_CUDA(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+        for (cudaEvent_t *e : {&h->static_done, &h->moved_done, &h->copies_done, &h->pass_end})
+            EKG_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    }
     // batched form: the static-lead rows of the ECG are final early, so their copy to the host runs
     // on the copy stream while the moved-lead part is computed
     const bool split = P.batch && P.nmove < (int)L;
@@ -1464,9 +1424,10 @@ void clear_error(ekg_heart *h, int slot) {
 }
 // The error word of passes run outside the pending slots (benchmark, autotuner), cleared if set.
 bool take_error(ekg_heart *h) {
-    EKG_CUDA(cudaMemcpy(h->err_host, h->ev.err, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    if (*h->err_host) clear_error(h, h->cur);
-    return *h->err_host != 0;
+    uint32_t err = 0;
+    EKG_CUDA(cudaMemcpy(&err, h->ev.err, sizeof(err), cudaMemcpyDeviceToHost));
+    if (err) clear_error(h, h->cur);
+    return err != 0;
 }
 
 // Hands over a pending batched evaluation: waits for its pass, checks the device error word and
@@ -1955,6 +1916,7 @@ int ekg_engine_create(int device, ekg_engine **out) {
         if (const char *v = std::getenv("EKG_TUNE")) e->tune = std::string(v) == "1";
         if (const char *v = std::getenv("EKG_TUNE_CACHE")) e->tune_cache = v;
         EKG_CUDA(cudaSetDevice(device));
+        EKG_CUDA(cudaDeviceGetAttribute(&e->sm_count, cudaDevAttrMultiProcessorCount, device));
         EKG_CUDA(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
         *out = e.release();
     });
@@ -2036,8 +1998,9 @@ int ekg_heart_activation(ekg_heart *h, double *at_out) {
     return guard([&] {
         EKG_CHECK(h && at_out, EKG_ERR_BAD_INPUT, "null argument");
         std::lock_guard<std::mutex> lk(h->mu);
-        ensure_at_host(h);
-        std::copy(h->at_host.begin(), h->at_host.end(), at_out);
+        EKG_CUDA(cudaSetDevice(h->eng->device));
+        EKG_CUDA(cudaMemcpyAsync(at_out, h->at_cells.p, h->ncell * 8, cudaMemcpyDeviceToHost, h->stream));
+        EKG_CUDA(cudaStreamSynchronize(h->stream));
     });
 }
 
@@ -2046,9 +2009,15 @@ int ekg_heart_activation(ekg_heart *h, double *at_out) {
 void ensure_ap_ref(ekg_heart *h) {
     if (!h->ap_index_ref.empty() || h->ncell == 0) return;
     const int64_t n = h->ncell, na = h->naps;
+    // cell of each voxel (voxels in AP order) and first voxel of each AP
+    std::vector<int32_t> cell(h->nvox), start(na + 1, (int32_t)h->nvox);
+    EKG_CUDA(cudaSetDevice(h->eng->device));
+    EKG_CUDA(cudaMemcpyAsync(cell.data(), h->vox_cell_dev.p, cell.size() * 4, cudaMemcpyDeviceToHost, h->stream));
+    EKG_CUDA(cudaMemcpyAsync(start.data(), h->vox_start_dev.p, na * 4, cudaMemcpyDeviceToHost, h->stream));
+    EKG_CUDA(cudaStreamSynchronize(h->stream));
     std::vector<int64_t> g_of_cell(n, -1);
     for (int64_t g = 0; g < na; ++g)
-        for (int64_t i = h->vox_group_start[g]; i < h->vox_group_start[g + 1]; ++i) g_of_cell[h->vox_cell[i]] = g;
+        for (int64_t i = start[g]; i < start[g + 1]; ++i) g_of_cell[cell[i]] = g;
     std::vector<int64_t> g2ref(na, -1);
     int64_t next = 0;
     h->ap_index_ref.assign(n, -1);
@@ -2273,7 +2242,9 @@ int ekg_heart_cell_ap(ekg_heart *h, int64_t index, int32_t *layer_out, double *a
         ensure_at_host(h);
         for (int64_t i = 0; i < h->ncell; ++i)
             if (h->ap_index_ref[i] == index) {
-                *layer_out = h->layer_host[i];
+                uint8_t layer = 0;
+                EKG_CUDA(cudaMemcpy(&layer, h->layers_dev.p + i, 1, cudaMemcpyDeviceToHost));
+                *layer_out = layer;
                 *at_out = h->at_host[i];
                 return;
             }

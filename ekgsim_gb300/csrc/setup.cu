@@ -8,7 +8,9 @@
 // runs of equal keys are the APs.  Then the per-AP arrays in the padded per-layer K layout and the
 // per-voxel records of the dipole kernels are written by one thread per AP slot / voxel.  The
 // results are the arrays a host sort by (layer, time bits, cell) gives, element for element.
+#include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 #include "ekg_internal.h"
@@ -110,19 +112,6 @@ __global__ void __launch_bounds__(ST) k_compact(F f, int64_t n, const int *__res
         if (flags & (1 << k)) out[pos++] = (int)(base + k);
 }
 
-template <class F>
-int compact(cudaStream_t s, F f, int64_t n, DBuf<int> &tsum, int *out, int *host_total) {
-    const int nt = (int)((n + STILE - 1) / STILE);
-    if (tsum.n < (size_t)nt + 1) tsum.alloc((size_t)nt + 1);
-    k_tile_counts<<<nt, ST, 0, s>>>(f, n, tsum.p);
-    k_scan_counts<<<1, ST, 0, s>>>(tsum.p, nt);
-    k_compact<<<nt, ST, 0, s>>>(f, n, tsum.p, out);
-    EKG_CUDA(cudaGetLastError());
-    EKG_CUDA(cudaMemcpyAsync(host_total, tsum.p + nt, sizeof(int), cudaMemcpyDeviceToHost, s));
-    EKG_CUDA(cudaStreamSynchronize(s));
-    return *host_total;
-}
-
 // ---- stable LSD radix sort of (layer, time bits) with the cell as payload, 8-bit digits
 // pass p < 8: byte p of the time bits; pass 8: the layer.  One element per thread, tiles of ST.
 __device__ __forceinline__ int digit(int pass, uint64_t key, uint8_t lay) {
@@ -207,13 +196,24 @@ __global__ void k_gather_keys(int nv, const int *__restrict__ cell, const double
     vl[i] = lay[c];
 }
 
-// first AP of each layer (APs are ordered by layer): lfirst[L] (-1 when the layer has none)
-__global__ void k_layer_first(int na, const int *__restrict__ gstart, const uint8_t *__restrict__ vl,
-                              int *__restrict__ lfirst) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= na) return;
+// out[0] = the number of APs (*na); out[L] = first AP of layer L (APs are ordered by layer; the others keep
+// what they held)
+__global__ void k_layer_first(const int *__restrict__ na, const int *__restrict__ gstart, const uint8_t *__restrict__ vl,
+                              int *__restrict__ out) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, n = *na;
+    if (a == 0) out[0] = n;
+    if (a >= n) return;
     const uint8_t L = vl[gstart[a]];
-    if (a == 0 || vl[gstart[a - 1]] != L) lfirst[L] = a;
+    if (a == 0 || vl[gstart[a - 1]] != L) out[L] = a;
+}
+
+// stage order: sort key (most voxels first) and payload of each 32-AP stage
+__global__ void k_stage_keys(int nst, uint32_t top, const int64_t *__restrict__ a_vb, uint64_t *__restrict__ key,
+                             int *__restrict__ val) {
+    const int st = blockIdx.x * blockDim.x + threadIdx.x;
+    if (st >= nst) return;
+    key[st] = top - (uint32_t)(a_vb[(int64_t)st * 32 + 32] - a_vb[(int64_t)st * 32]);
+    val[st] = st;
 }
 
 // per padded AP slot p: its layer (present layer k with pbase[k] <= p < pbase[k + 1]), the AP's
@@ -310,84 +310,75 @@ __global__ void k_voxel_records(int nv, VoxelGeom g, const int *__restrict__ cel
 
 }  // namespace
 
+// Sorts n (key, layer, payload) triples by the digit passes listed; the pointers are left at the sorted
+// buffers (first) and the other ones.
+static void sort_passes(cudaStream_t s, int n, int first, int passes, uint64_t *&key, uint64_t *&key2, uint8_t *&lay,
+                        uint8_t *&lay2, int *&val, int *&val2, int *hist, int *totals, int *base) {
+    const int nblk = (n + ST - 1) / ST;
+    for (int pass = first; pass < first + passes; ++pass) {
+        k_digit_hist<<<nblk, ST, 0, s>>>(pass, n, key, lay, nblk, hist);
+        k_digit_scan<<<256, ST, 0, s>>>(hist, nblk, totals);
+        k_digit_base<<<1, ST, 0, s>>>(totals, base);
+        k_digit_scatter<<<nblk, ST, 0, s>>>(pass, n, key, lay, val, nblk, hist, base, key2, lay2, val2);
+        EKG_CUDA(cudaGetLastError());
+        std::swap(key, key2);
+        std::swap(lay, lay2);
+        std::swap(val, val2);
+    }
+}
+
+// elements the sort's buffers hold: the voxels, or the stages of the padded APs
+static size_t sort_capacity(int64_t nvox) { return (size_t)std::max<int64_t>(nvox, nvox / 32 + 2 * 256 + 2); }
+
+size_t setup_scratch_bytes(int64_t n_cells, int64_t nvox) {
+    const size_t m = sort_capacity(nvox), tiles = (size_t)(n_cells + STILE - 1) / STILE + 1;
+    return 2 * (Arena::part(m * 8) + Arena::part(m) + Arena::part(m * 4)) + Arena::part((m + 1) * 4) +
+           Arena::part((m + ST - 1) / ST * 256 * 4) + 2 * Arena::part(256 * 4) + Arena::part(tiles * 4) +
+           Arena::part(257 * 4) + Arena::part(8);
+}
+
 void setup_voxels_device(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_lay, const double *d_at_cells,
-                         int nl, DedupResult &r) {
+                         int nl, int64_t nvox, Arena &scratch, DedupResult &r) {
     const int64_t n = (int64_t)nz * ny * nx;
-    int *pinned = nullptr;
-    EKG_CUDA(cudaMallocHost(&pinned, 8 * sizeof(int)));
-    struct Free {
-        int *p;
-        ~Free() { cudaFreeHost(p); }
-    } free_pinned{pinned};
-    DBuf<int> tsum;
-    // 1. voxels in raster order
-    DBuf<int> cellA, cellB;
-    const int nv = [&] {
-        // an upper bound for the list: count first
-        const int nt = (int)((n + STILE - 1) / STILE);
-        tsum.alloc((size_t)nt + 1);
-        k_tile_counts<<<nt, ST, 0, s>>>(IsVoxel{d_lay}, n, tsum.p);
-        k_scan_counts<<<1, ST, 0, s>>>(tsum.p, nt);
-        EKG_CUDA(cudaGetLastError());
-        EKG_CUDA(cudaMemcpyAsync(pinned, tsum.p + nt, sizeof(int), cudaMemcpyDeviceToHost, s));
-        EKG_CUDA(cudaStreamSynchronize(s));
-        const int c = pinned[0];
-        cellA.alloc((size_t)std::max(c, 1));
-        k_compact<<<nt, ST, 0, s>>>(IsVoxel{d_lay}, n, tsum.p, cellA.p);
-        EKG_CUDA(cudaGetLastError());
-        return c;
-    }();
+    const int nv = (int)nvox;
+    const size_t m = sort_capacity(nvox);
+    r.key = scratch.take<uint64_t>(m);
+    r.key2 = scratch.take<uint64_t>(m);
+    r.vl = scratch.take<uint8_t>(m);
+    r.vl2 = scratch.take<uint8_t>(m);
+    r.cell = scratch.take<int>(m);
+    r.cell2 = scratch.take<int>(m);
+    r.gstart = scratch.take<int>(m + 1);
+    r.hist = scratch.take<int>((m + ST - 1) / ST * 256);
+    r.totals = scratch.take<int>(256);
+    r.base = scratch.take<int>(256);
+    r.tsum = scratch.take<int>((size_t)(n + STILE - 1) / STILE + 1);
+    int *info = scratch.take<int>(257);
+    r.n_interior = scratch.take<unsigned long long>(1);
     r.nvox = nv;
-    if (nv == 0) return;
+    // 1. voxels in raster order
+    const int nt = (int)((n + STILE - 1) / STILE);
+    k_tile_counts<<<nt, ST, 0, s>>>(IsVoxel{d_lay}, n, r.tsum);
+    k_scan_counts<<<1, ST, 0, s>>>(r.tsum, nt);
+    k_compact<<<nt, ST, 0, s>>>(IsVoxel{d_lay}, n, r.tsum, r.cell);
     // 2. stable radix sort by (layer, time bits); payload = cell
-    DBuf<uint64_t> keyA, keyB;
-    DBuf<uint8_t> layA, layB;
-    keyA.alloc(nv);
-    keyB.alloc(nv);
-    layA.alloc(nv);
-    layB.alloc(nv);
-    cellB.alloc(nv);
-    {
-        const int g = (nv + 255) / 256;
-        k_gather_keys<<<g, 256, 0, s>>>(nv, cellA.p, d_at_cells, d_lay, keyA.p, layA.p);
-        EKG_CUDA(cudaGetLastError());
-    }
-    const int nblk = (nv + ST - 1) / ST;
-    DBuf<int> hist, totals, base;
-    hist.alloc((size_t)256 * nblk);
-    totals.alloc(256);
-    base.alloc(256);
-    uint64_t *ki = keyA.p, *ko = keyB.p;
-    uint8_t *li = layA.p, *lo = layB.p;
-    int *vi = cellA.p, *vo = cellB.p;
-    for (int pass = 0; pass < 9; ++pass) {
-        k_digit_hist<<<nblk, ST, 0, s>>>(pass, nv, ki, li, nblk, hist.p);
-        k_digit_scan<<<256, ST, 0, s>>>(hist.p, nblk, totals.p);
-        k_digit_base<<<1, ST, 0, s>>>(totals.p, base.p);
-        k_digit_scatter<<<nblk, ST, 0, s>>>(pass, nv, ki, li, vi, nblk, hist.p, base.p, ko, lo, vo);
-        EKG_CUDA(cudaGetLastError());
-        std::swap(ki, ko);
-        std::swap(li, lo);
-        std::swap(vi, vo);
-    }
-    // after an odd number of passes the sorted arrays are the B buffers
-    DBuf<uint64_t> &key = ki == keyA.p ? keyA : keyB;
-    DBuf<uint8_t> &vl = li == layA.p ? layA : layB;
-    DBuf<int> &cell = vi == cellA.p ? cellA : cellB;
-    // 3. runs of equal (layer, time): the APs
-    DBuf<int> gstart;
-    gstart.alloc((size_t)nv + 1);
-    const int na = compact(s, StartsRun{vl.p, key.p}, nv, tsum, gstart.p, pinned);
-    r.naps = na;
-    // 4. first AP of each layer
-    DBuf<int> lfirst;
-    lfirst.alloc(256);
-    EKG_CUDA(cudaMemsetAsync(lfirst.p, 0xff, 256 * sizeof(int), s));
-    k_layer_first<<<(na + 255) / 256, 256, 0, s>>>(na, gstart.p, vl.p, lfirst.p);
+    k_gather_keys<<<(nv + 255) / 256, 256, 0, s>>>(nv, r.cell, d_at_cells, d_lay, r.key, r.vl);
     EKG_CUDA(cudaGetLastError());
-    std::vector<int> lf(256);
-    EKG_CUDA(cudaMemcpyAsync(lf.data(), lfirst.p, 256 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    sort_passes(s, nv, 0, 9, r.key, r.key2, r.vl, r.vl2, r.cell, r.cell2, r.hist, r.totals, r.base);
+    // 3. runs of equal (layer, time): the APs
+    const int nt2 = (nv + STILE - 1) / STILE;
+    k_tile_counts<<<nt2, ST, 0, s>>>(StartsRun{r.vl, r.key}, nv, r.tsum);
+    k_scan_counts<<<1, ST, 0, s>>>(r.tsum, nt2);
+    k_compact<<<nt2, ST, 0, s>>>(StartsRun{r.vl, r.key}, nv, r.tsum, r.gstart);
+    // 4. their number and the first one of each layer
+    EKG_CUDA(cudaMemsetAsync(info, 0xff, 257 * sizeof(int), s));
+    k_layer_first<<<(nv + 255) / 256, 256, 0, s>>>(r.tsum + nt2, r.gstart, r.vl, info);
+    EKG_CUDA(cudaGetLastError());
+    int lf[257];
+    EKG_CUDA(cudaMemcpyAsync(lf, info, sizeof(lf), cudaMemcpyDeviceToHost, s));
     EKG_CUDA(cudaStreamSynchronize(s));
+    const int na = lf[0];
+    r.naps = na;
     // present layers in order with their AP ranges and padded (multiple of 64) bases
     r.pl_layer.clear();
     r.pfirst.clear();
@@ -409,37 +400,34 @@ void setup_voxels_device(cudaStream_t s, int nz, int ny, int nx, const uint8_t *
             pad += (int64_t)(next - lf[L] + 63) / 64 * 64;
         }
     r.apad = pad;
-    // keep the sorted voxel list and run starts for the remaining steps and the host copies
-    r.cell = std::move(cell);
-    r.gstart = std::move(gstart);
-    r.key = std::move(key);
-    r.vl = std::move(vl);
 }
 
-void setup_ap_arrays_device(cudaStream_t s, const DedupResult &r, const double *d_at_cells, double *at, float2 *at_hilo,
-                            int32_t *a_layer, int64_t *a_vb) {
-    const int npl = (int)r.pl_layer.size();
-    DBuf<int> pl, pf, pc;
-    DBuf<int64_t> pb;
-    pl.alloc(npl);
-    pf.alloc(npl);
-    pc.alloc(npl);
-    pb.alloc(npl);
-    EKG_CUDA(cudaMemcpyAsync(pl.p, r.pl_layer.data(), npl * sizeof(int), cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(pf.p, r.pfirst.data(), npl * sizeof(int), cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(pc.p, r.pcount.data(), npl * sizeof(int), cudaMemcpyHostToDevice, s));
-    EKG_CUDA(cudaMemcpyAsync(pb.p, r.pbase.data(), npl * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+// bases first (8 bytes), then layers, first APs, counts
+size_t setup_ap_tables(const DedupResult &r, uint8_t *host) {
+    const size_t npl = r.pl_layer.size();
+    if (host) {
+        std::memcpy(host, r.pbase.data(), npl * 8);
+        std::memcpy(host + npl * 8, r.pl_layer.data(), npl * 4);
+        std::memcpy(host + npl * 12, r.pfirst.data(), npl * 4);
+        std::memcpy(host + npl * 16, r.pcount.data(), npl * 4);
+    }
+    return npl * 20;
+}
+
+void setup_ap_arrays_device(cudaStream_t s, const DedupResult &r, const uint8_t *d_tables, const double *d_at_cells,
+                            double *at, float2 *at_hilo, int32_t *a_layer, int64_t *a_vb) {
+    const size_t npl = r.pl_layer.size();
     const int64_t slots = r.apad + 1;
-    k_ap_arrays<<<(unsigned)((slots + 255) / 256), 256, 0, s>>>(r.apad, npl, pl.p, pb.p, pf.p, pc.p, (int)r.naps,
-                                                                (int)r.nvox, r.gstart.p, r.cell.p, d_at_cells, at,
-                                                                at_hilo, a_layer, a_vb);
+    k_ap_arrays<<<(unsigned)((slots + 255) / 256), 256, 0, s>>>(
+        r.apad, (int)npl, reinterpret_cast<const int *>(d_tables + npl * 8), reinterpret_cast<const int64_t *>(d_tables),
+        reinterpret_cast<const int *>(d_tables + npl * 12), reinterpret_cast<const int *>(d_tables + npl * 16), (int)r.naps,
+        (int)r.nvox, r.gstart, r.cell, d_at_cells, at, at_hilo, a_layer, a_vb);
     EKG_CUDA(cudaGetLastError());
-    EKG_CUDA(cudaStreamSynchronize(s));  // the small tables above are freed on return
 }
 
-int64_t setup_voxel_records_device(cudaStream_t s, const DedupResult &r, int nz, int ny, int nx, const uint8_t *d_lay,
-                                   const HeartDev &D, int few_max, int32_t *vzyx, uint32_t *vin, uint32_t *vout,
-                                   float4 *vpos, float4 *vosum) {
+void setup_voxel_records_device(cudaStream_t s, const DedupResult &r, int nz, int ny, int nx, const uint8_t *d_lay,
+                                const HeartDev &D, int few_max, int32_t *vzyx, uint32_t *vin, uint32_t *vout,
+                                float4 *vpos, float4 *vosum) {
     VoxelGeom g;
     g.nz = nz;
     g.ny = ny;
@@ -451,17 +439,25 @@ int64_t setup_voxel_records_device(cudaStream_t s, const DedupResult &r, int nz,
     g.cz = D.centre[0];
     g.cy = D.centre[1];
     g.cx = D.centre[2];
-    DBuf<unsigned long long> cnt;
-    cnt.alloc(1);
-    EKG_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned long long), s));
+    EKG_CUDA(cudaMemsetAsync(r.n_interior, 0, sizeof(unsigned long long), s));
     const int nv = (int)r.nvox;
-    k_voxel_records<<<(nv + 255) / 256, 256, 0, s>>>(nv, g, r.cell.p, d_lay, r.vl.p, r.key.p, vzyx, vin, vout, vpos,
-                                                     vosum, cnt.p);
+    k_voxel_records<<<(nv + 255) / 256, 256, 0, s>>>(nv, g, r.cell, d_lay, r.vl, r.key, vzyx, vin, vout, vpos, vosum,
+                                                     r.n_interior);
     EKG_CUDA(cudaGetLastError());
-    unsigned long long h = 0;
-    EKG_CUDA(cudaMemcpyAsync(&h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-    EKG_CUDA(cudaStreamSynchronize(s));
-    return (int64_t)h;
+}
+
+// Keys top - voxels ascend as the voxel counts descend; the sort is stable, so ties keep their index
+// order.  As many 8-bit digits as a count can have.
+void setup_stage_order_device(cudaStream_t s, DedupResult &r, const int64_t *a_vox_begin, int32_t *stage_order) {
+    const int nst = (int)(r.apad / 32);
+    if (nst <= 0) return;
+    int digits = 1;
+    while (digits < 4 && (r.nvox >> (8 * digits))) ++digits;
+    const uint32_t top = digits == 4 ? 0xffffffffu : (1u << (8 * digits)) - 1u;
+    k_stage_keys<<<(nst + 255) / 256, 256, 0, s>>>(nst, top, a_vox_begin, r.key, r.cell);
+    EKG_CUDA(cudaGetLastError());
+    sort_passes(s, nst, 0, digits, r.key, r.key2, r.vl, r.vl2, r.cell, r.cell2, r.hist, r.totals, r.base);
+    EKG_CUDA(cudaMemcpyAsync(stage_order, r.cell, (size_t)nst * 4, cudaMemcpyDeviceToDevice, s));
 }
 
 // ------------------------------------------------------------------ stage bounding boxes
