@@ -255,6 +255,7 @@ void setup_stage_order_device(cudaStream_t s, DedupResult &r, const int64_t *a_v
 // Per-evaluation scratch (sized for n_sims simulations).
 struct EvalDev {
     int cap_sims = 0;
+    Arena mem, general;     // behind the buffers of every pass, and of the per-simulation form
     DBuf<float> layer_c;    // [S][nl][4]: k1*log2e, k4*log2e, 1-k3, k3 (FP32 H constants)
     DBuf<double> F;         // [S][nl][steps]
     DBuf<float> Ff;         // [S][nl][steps] the same in FP32 (batched form)

@@ -459,13 +459,17 @@ void ensure_eval_capacity(ekg_heart *h, int n_sims) {
     const HeartDev &D = h->dev;
     if (E.cap_sims >= n_sims) return;
     const size_t S = (size_t)n_sims;
-    E.layer_c.alloc(S * D.nlayers * 4);
-    E.F.alloc(S * D.nlayers * D.steps);
-    E.Ff.alloc(S * D.nlayers * D.steps);
-    E.k0w.alloc(S * D.nleads);
-    E.out.alloc(out_ecg_offset(n_sims, std::max(1, D.nleads)) + S * D.nleads * D.steps);
+    const size_t nf = S * D.nlayers * D.steps, ne = S * D.nleads * D.steps;
+    const size_t no = out_ecg_offset(n_sims, std::max(1, D.nleads)) + ne;
+    E.mem.reserve(Arena::part(S * D.nlayers * 16) + Arena::part(nf * 8) + Arena::part(nf * 4) + Arena::part(S * D.nleads * 8) +
+                  Arena::part(no * 8) + Arena::part(ne * 8));
+    E.mem.place(E.layer_c, S * D.nlayers * 4);
+    E.mem.place(E.F, nf);
+    E.mem.place(E.Ff, nf);
+    E.mem.place(E.k0w, S * D.nleads);
+    E.mem.place(E.out, no);
+    E.mem.place(E.ecg_ff, ne);
     EKG_CUDA(cudaMemsetAsync(E.out.p, 0, sizeof(double), h->stream));  // the error words
-    E.ecg_ff.alloc(S * D.nleads * D.steps);
     E.cap_sims = n_sims;
 }
 // Places a pass's results in EvalDev::out.
@@ -489,16 +493,21 @@ void ensure_general_capacity(ekg_heart *h, int n_sims) {
     const HeartDev &D = h->dev;
     const size_t S = (size_t)n_sims;
     const size_t nw = S * D.nleads * D.apad, np = S * D.nchunks * D.nleads * D.steps;
-    if (E.W.n < nw) E.W.alloc(nw);
-    if (!band_contraction(h) && E.Wp.n < nw) E.Wp.alloc(nw);
-    if (E.work.n < 1) E.work.alloc(1);
     if (band_contraction(h)) {
-        if (E.band.n < np) E.band.alloc(np);
-        if (E.csum.n < S * D.nchunks * D.nleads) E.csum.alloc(S * D.nchunks * D.nleads);
-        if (E.cinfo.n < S * D.nchunks) E.cinfo.alloc(S * D.nchunks);
-    } else if (E.partial.n < np) {
-        E.partial.alloc(np);
+        if (E.W.n >= nw && E.band.n >= np && E.cinfo.n >= S * D.nchunks && E.csum.n >= S * D.nchunks * D.nleads) return;
+        E.general.reserve(Arena::part(nw * 4) + Arena::part(np * 4) + Arena::part(S * D.nchunks * D.nleads * 8) +
+                          Arena::part(S * D.nchunks * 16) + Arena::part(4));
+        E.general.place(E.W, nw);
+        E.general.place(E.band, np);
+        E.general.place(E.csum, S * D.nchunks * D.nleads);
+        E.general.place(E.cinfo, S * D.nchunks);
+        E.general.place(E.work, 1);
+        return;
     }
+    if (E.W.n < nw) E.W.alloc(nw);
+    if (E.Wp.n < nw) E.Wp.alloc(nw);
+    if (E.work.n < 1) E.work.alloc(1);
+    if (E.partial.n < np) E.partial.alloc(np);
 }
 
 // Device pass for n_sims simulations, split into upload / compute / download so the benchmark
