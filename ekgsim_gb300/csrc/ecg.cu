@@ -243,14 +243,107 @@ __global__ void __launch_bounds__(CC_T) k_contract_cuda(int steps, int nleads, i
 // W'[l][a] = W[l][a] exp(k5 at_a) is formed here (the FP32 operations of the lead-field kernel's
 // W'), with W the moved rows' field Wm [S][L][apad] for l < wrows and the resident field
 // W0 [L][apad] for the others.
-constexpr int CB_THREADS = 256, CB_LB = 16, CB_CAP = CONTRACT_BAND_CAP;
+//
+// What bounds it: FP32 issue, and the shared-memory reads of W' in the band.  A block is 128 threads of
+// which each takes two band steps, so that a row of W' read serves both; the steps' APs are dealt to
+// CB_SLICES / rows slices as if 256 threads took one step each, which fixes the order of the sums.
+constexpr int CB_THREADS = 128, CB_WARPS = CB_THREADS / 32, CB_SLICES = 256, CB_LB = 16, CB_CAP = CONTRACT_BAND_CAP;
 // dynamic shared memory of a block with NLB leads: W' [CB_CAP][NLB], the activation times, the
-// band passes' partial sums [CB_THREADS][NLB + 1]; five blocks per SM fit up to 12 leads
+// band passes' partial sums of half the leads [CB_SLICES][NLB / 2 + 1]
 constexpr size_t cb_smem_bytes(int nlb) {
-    return (size_t)CB_CAP * nlb * 4 + (size_t)CB_CAP * 8 + (size_t)CB_THREADS * (nlb + 1) * 4;
+    return (size_t)CB_CAP * nlb * 4 + (size_t)CB_CAP * 8 + (size_t)CB_SLICES * (nlb / 2 + 1) * 4;
+}
+// number of leading steps for which f holds (f holds for a prefix of the steps): 32 probes at a time
+template <class Pred>
+__device__ __forceinline__ int prefix_steps(int steps, int lane, Pred f) {
+    int lo = 0, n = steps;  // the first step without f lies in [lo, lo + n]
+    while (n > 0) {
+        const int stride = (n + 31) / 32, t = lo + lane * stride;
+        const int k = __popc(__ballot_sync(0xffffffffu, lane * stride < n && f(t)));
+        if (stride == 1) return lo + k;
+        if (k == 0) return lo;
+        const int from = (k - 1) * stride + 1;  // behind the last probe that holds
+        n = min(n, k * stride) - from;
+        lo += from;
+    }
+    return lo;
+}
+// sums over a warp of 2 G values per lane (v[0 .. G) and v[G .. 2 G)) by recursive halving: at each level a
+// lane keeps half of its values (chosen by one lane bit) and adds its partner's copy of them.  Every
+// value is added over the lanes in the order of the xor tree 16, 8, 4, 2, 1.  Returns the lane's value;
+// its index is in idx (lanes that share one hold the same value).
+template <int G>
+__device__ __forceinline__ float warp_sums(float (&v)[2 * G], int lane, int &idx) {
+    idx = 0;
+    int o = 16;
+#pragma unroll
+    for (int n = G; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+            const float keep = up ? v[j + n] : v[j], give = up ? v[j] : v[j + n];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        idx += up ? n : 0;
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+// S0, S1 of G leads from lh: per virtual warp of 32 slices (slice i: APs i, i + 256) a warp sum each;
+// g: the APs' factors, negative where there is none
+template <int NLB, int G>
+__device__ __forceinline__ void steady_sums(int lh, int warp, int lane, const float (*s_w)[NLB],
+                                            const float (&g)[CB_CAP / CB_THREADS], float (*s_part)[CB_SLICES / 32][NLB]) {
+#pragma unroll
+    for (int q = 0; q < CB_SLICES / CB_THREADS; ++q) {
+        const int vw = warp + q * CB_WARPS;
+        float v[2 * G];
+#pragma unroll
+        for (int l = 0; l < 2 * G; ++l) v[l] = 0.f;
+#pragma unroll
+        for (int h = 0; h < CB_CAP / CB_SLICES; ++h) {
+            const int i = vw * 32 + lane + h * CB_SLICES;
+            const float gi = g[q + h * (CB_SLICES / CB_THREADS)];
+            if (!(gi >= 0.f)) continue;
+#pragma unroll
+            for (int l = 0; l < G; l += 4) {
+                const float4 w = *reinterpret_cast<const float4 *>(&s_w[i][lh + l]);
+                v[l] = fmaf(w.x, gi, v[l]);
+                v[l + 1] = fmaf(w.y, gi, v[l + 1]);
+                v[l + 2] = fmaf(w.z, gi, v[l + 2]);
+                v[l + 3] = fmaf(w.w, gi, v[l + 3]);
+                v[G + l] += w.x;
+                v[G + l + 1] += w.y;
+                v[G + l + 2] += w.z;
+                v[G + l + 3] += w.w;
+            }
+        }
+        int idx;
+        const float x = warp_sums<G>(v, lane, idx);
+        s_part[idx / G][vw][lh + idx % G] = x;  // lanes that share a value write the same
+    }
+}
+// two steps' sums over a slice of the APs (sl, sl + nsl, ...); H(i, k): H of AP i at step k
+template <int NLB, class H>
+__device__ __forceinline__ void band_sums(float (&acc)[2][NLB], int sl, int nsl, int na, const float (*s_w)[NLB], H h_of) {
+    for (int i = sl; i < na; i += nsl) {
+        const float h[2] = {h_of(i, 0), h_of(i, 1)};
+#pragma unroll
+        for (int l = 0; l < NLB; l += 4) {
+            const float4 w = *reinterpret_cast<const float4 *>(&s_w[i][l]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                acc[k][l] = fmaf(w.x, h[k], acc[k][l]);
+                acc[k][l + 1] = fmaf(w.y, h[k], acc[k][l + 1]);
+                acc[k][l + 2] = fmaf(w.z, h[k], acc[k][l + 2]);
+                acc[k][l + 3] = fmaf(w.w, h[k], acc[k][l + 3]);
+            }
+        }
+    }
 }
 template <int NLB>
-__global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 5 : 4) k_contract_band(
+__global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 6 : 4) k_contract_band(
     int steps, int nleads, int64_t apad, int nl, const float2 *__restrict__ t_hilo, const float2 *__restrict__ at_hilo,
     const double *__restrict__ at, const int32_t *__restrict__ chunk_a0, const int32_t *__restrict__ chunk_a1,
     const int32_t *__restrict__ chunk_layer, const float *__restrict__ Wm, int wrows, const float *__restrict__ W0,
@@ -259,9 +352,10 @@ __global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 5 : 4) k_contract_band
     extern __shared__ __align__(16) uint8_t cb_smem[];
     float(*s_w)[NLB] = reinterpret_cast<float(*)[NLB]>(cb_smem);  // W'[a][l] of the chunk
     float2 *s_at = reinterpret_cast<float2 *>(cb_smem + (size_t)CB_CAP * NLB * 4);
-    float(*s_red)[NLB + 1] = reinterpret_cast<float(*)[NLB + 1]>(s_at + CB_CAP);  // [slice * rows + step]
-    __shared__ float s_ext[2][CB_THREADS / 32];
-    __shared__ float s_part[2][CB_THREADS / 32][(NLB + 7) / 8 * 8];
+    constexpr int HL = NLB / 2;
+    float(*s_red)[HL + 1] = reinterpret_cast<float(*)[HL + 1]>(s_at + CB_CAP);  // [slice * rows + step]
+    __shared__ float s_ext[2][CB_WARPS];
+    __shared__ float s_part[2][CB_SLICES / 32][NLB];
     __shared__ float s_sum[2][NLB];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c = blockIdx.x;
@@ -274,22 +368,27 @@ __global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 5 : 4) k_contract_band
 
     // the chunk: activation times, W' transposed to [a][l], the extreme finite activation times
     float amin = INFINITY, amax = -INFINITY;
+#pragma unroll 2
     for (int i = tid; i < na; i += CB_THREADS) {
+        // every load of the AP is issued before the first is used (a row's source by its address, not by
+        // a branch around the load: those put 12 round trips to L2 in a row, half of the kernel's time)
+        float w[NLB];
+#pragma unroll
+        for (int l = 0; l < NLB; ++l) {
+            const int lg = l0 + min(l, nlh - 1);
+            const float *row = lg < wrows ? Wm + ((size_t)s * nleads + lg) * apad : W0 + (size_t)lg * apad;
+            w[l] = row[a0 + i];
+        }
         const float2 a2 = at_hilo[a0 + i];
+        const double ad = at[a0 + i];
         s_at[i] = a2;
         if (isfinite(a2.x)) {
             amin = fminf(amin, a2.x);
             amax = fmaxf(amax, a2.x);
         }
-        const double ad = at[a0 + i];
         const float f = isinf(ad) ? 0.f : expf((float)(k5 * ad));
-        float w[NLB];
 #pragma unroll
-        for (int l = 0; l < NLB; ++l) {
-            const int lg = l0 + l;
-            w[l] = l >= nlh ? 0.f
-                            : (lg < wrows ? Wm[((size_t)s * nleads + lg) * apad + a0 + i] : W0[(size_t)lg * apad + a0 + i]) * f;
-        }
+        for (int l = 0; l < NLB; ++l) w[l] = l < nlh ? w[l] * f : 0.f;
 #pragma unroll
         for (int l = 0; l < NLB; l += 4)
             *reinterpret_cast<float4 *>(&s_w[i][l]) = make_float4(w[l], w[l + 1], w[l + 2], w[l + 3]);
@@ -305,83 +404,49 @@ __global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 5 : 4) k_contract_band
     }
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < CB_THREADS / 32; ++w) {
+    for (int w = 0; w < CB_WARPS; ++w) {
         amin = fminf(amin, s_ext[0][w]);
         amax = fmaxf(amax, s_ext[1][w]);
     }
     const bool any_finite = amin <= amax;
     const bool classify = any_finite && kc.x > 0.f && kc.y >= 0.f;
-    int nzero = 0, nsteady = 0;
-    for (int tb = 0; tb < steps; tb += CB_THREADS) {
-        const int t = tb + tid;
-        bool z = false, st = false;
-        if (t < steps && classify) {
+    // both conditions are monotone in the step's time
+    int tb0 = any_finite ? 0 : steps, tb1 = steps;  // band steps [tb0, tb1)
+    if (classify) {
+        tb0 = prefix_steps(steps, lane, [&](int t) {
             const float tt = t_hilo[t].x;
-            z = kc.x * (amin - tt) >= 30.5f && (kc.x - kc.y) * (amin - tt) >= 30.5f;
-            st = kc.x * (tt - amax) >= 26.5f;
-        }
-        nzero += __syncthreads_count(z);
-        nsteady += __syncthreads_count(st);
+            return kc.x * (amin - tt) >= 30.5f && (kc.x - kc.y) * (amin - tt) >= 30.5f;
+        });
+        tb1 = prefix_steps(steps, lane, [&](int t) { return !(kc.x * (t_hilo[t].x - amax) >= 26.5f); });
     }
-    if (!any_finite) nzero = steps;
-    const int tb0 = nzero, tb1 = steps - nsteady;  // band steps [tb0, tb1)
     if (lb == 0 && tid == 0) cinfo[(size_t)s * nchunks + c] = make_int4(tb0, tb1, __float_as_int(amax), 0);
 
-    if (nsteady > 0) {
-        // S0, S1 per lead: each thread its APs, then a shuffle and a shared-memory reduction (eight
-        // leads at a time, which keeps the accumulators in registers)
-#pragma unroll 1
-        for (int lh = 0; lh < NLB; lh += 8) {
-            float u0[8], u1[8];
+    if (tb1 < steps) {
+        // the steady run's sums per lead: S0 = sum W' 2^(-k4'(amax - at)), S1 = sum W'
+        float g[CB_CAP / CB_THREADS];
 #pragma unroll
-            for (int l = 0; l < 8; ++l) u0[l] = u1[l] = 0.f;
-            for (int i = tid; i < na; i += CB_THREADS) {
-                const float2 a2 = s_at[i];
-                if (!isfinite(a2.x)) continue;
-                const float g = ex2_approx(-kc.y * ((amax - a2.x) - a2.y));
-#pragma unroll
-                for (int l = 0; l < 8; ++l) {
-                    const float w = lh + l < NLB ? s_w[i][lh + l] : 0.f;
-                    u0[l] = fmaf(w, g, u0[l]);
-                    u1[l] += w;
-                }
-            }
-            // the 16 warp sums by recursive halving: at each level a lane keeps half of its values
-            // (chosen by one lane bit) and adds its partner's copy of them; 16 shuffles instead of 80
-            float v[16];
-#pragma unroll
-            for (int l = 0; l < 8; ++l) {
-                v[l] = u0[l];
-                v[8 + l] = u1[l];
-            }
-#pragma unroll
-            for (int o = 16, n = 8; o > 1; o >>= 1, n >>= 1) {
-                const bool up = lane & o;
-#pragma unroll
-                for (int j = 0; j < n; ++j) {
-                    const float keep = up ? v[j + n] : v[j], give = up ? v[j] : v[j + n];
-                    v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-                }
-            }
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-            // lane holds value 8 b4 + 4 b3 + 2 b2 + b1 (b_i its lane bits): (S0 or S1, lead)
-            const int idx = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
-            if (!(lane & 1)) s_part[idx >> 3][warp][lh + (idx & 7)] = v[0];
+        for (int q = 0; q < CB_CAP / CB_THREADS; ++q) {
+            const int i = tid + q * CB_THREADS;
+            g[q] = -1.f;
+            if (i < na && isfinite(s_at[i].x)) g[q] = ex2_approx(-kc.y * ((amax - s_at[i].x) - s_at[i].y));
         }
+#pragma unroll
+        for (int lh = 0; lh + 8 <= NLB; lh += 8) steady_sums<NLB, 8>(lh, warp, lane, s_w, g, s_part);
+        if constexpr (NLB % 8) steady_sums<NLB, 4>(NLB / 8 * 8, warp, lane, s_w, g, s_part);
         __syncthreads();
         if (tid < 2 * NLB) {
             const int k = tid / NLB, l = tid % NLB;
             float v = 0.f;
-            for (int w = 0; w < CB_THREADS / 32; ++w) v += s_part[k][w][l];
+            for (int w = 0; w < CB_SLICES / 32; ++w) v += s_part[k][w][l];
             s_sum[k][l] = v;
         }
         __syncthreads();
         if (tid < nlh) csum[((size_t)s * nchunks + c) * nleads + l0 + tid] = make_float2(s_sum[0][tid], s_sum[1][tid]);
     }
 
-    // band: passes of 32, 16 or 8 steps (the fewest steps that cover the run), lane = step.  The
+    // band: passes of 32, 16 or 8 steps (the fewest steps that cover the run), two steps per thread.  The
     // chunk's APs are dealt round-robin to 256 / rows slices (slice j takes APs j, j + nsl, ...);
-    // the 8 lanes of a quarter warp share one slice, so the W' reads are broadcasts.
+    // lanes that share a slice read the same W' rows.
     // With T the chunk's first (smallest) activation time the two exponentials separate,
     //     2^(-k' (t - at)) = 2^(-k' (t - T)) 2^(k' (at - T)),
     // one factor per step and one per AP (replacing the AP time in shared memory), which leaves one
@@ -407,53 +472,59 @@ __global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 5 : 4) k_contract_band
     }
     for (int tb = tb0; tb < tb1;) {
         const int rem = tb1 - tb;
-        const int rows = rem > 24 ? 32 : (rem > 8 ? 16 : 8);
-        const int nsl = CB_THREADS / rows, r = lane & (rows - 1), sl = warp * (32 / rows) + lane / rows;
-        const float2 th = t_hilo[min(tb + r, steps - 1)];
-        float acc[NLB];
+        const int rows = rem > 24 ? 32 : (rem > 8 ? 16 : 8), half = rows / 2;
+        const int nsl = CB_SLICES / rows, r = lane & (half - 1), sl = warp * (32 / half) + lane / half;
+        float2 th[2];
+        float acc[2][NLB];
 #pragma unroll
-        for (int l = 0; l < NLB; ++l) acc[l] = 0.f;
+        for (int k = 0; k < 2; ++k) {
+            th[k] = t_hilo[min(tb + r + k * half, steps - 1)];
+#pragma unroll
+            for (int l = 0; l < NLB; ++l) acc[k][l] = 0.f;
+        }
         if (sep) {
-            const float d = (th.x - T.x) + (th.y - T.y);
-            const float E1 = ex2_approx(-kc.x * d), E4 = ex2_approx(-kc.y * d);
-            for (int i = sl; i < na; i += nsl) {
-                const float2 g = s_g[i];
-                const float sg = rcp_approx(fmaf(E1, g.x, 1.0f));
-                const float hv = sg * fmaf(kc.z, E4 * g.y, kc.w);
-                const float h = sg == 0.f ? 0.f : hv;
+            float E1[2], E4[2];
 #pragma unroll
-                for (int l = 0; l < NLB; l += 4) {
-                    const float4 w = *reinterpret_cast<const float4 *>(&s_w[i][l]);
-                    acc[l] = fmaf(w.x, h, acc[l]);
-                    acc[l + 1] = fmaf(w.y, h, acc[l + 1]);
-                    acc[l + 2] = fmaf(w.z, h, acc[l + 2]);
-                    acc[l + 3] = fmaf(w.w, h, acc[l + 3]);
-                }
+            for (int k = 0; k < 2; ++k) {
+                const float d = (th[k].x - T.x) + (th[k].y - T.y);
+                E1[k] = ex2_approx(-kc.x * d);
+                E4[k] = ex2_approx(-kc.y * d);
             }
+            // 0 where the sigmoid underflows; the other factor stays finite there but for a k4 near or above k1
+            // and times far before the chunk's, and only then the product has to be replaced
+            if (ex2_approx(-kc.y * ((t_hilo[tb].x - T.x) + (t_hilo[tb].y - T.y))) < 0x1p60f && fabsf(kc.z) < 0x1p3f)
+                band_sums<NLB>(acc, sl, nsl, na, s_w, [&](int i, int k) {
+                    const float2 g = s_g[i];
+                    return rcp_approx(fmaf(E1[k], g.x, 1.0f)) * fmaf(kc.z, E4[k] * g.y, kc.w);
+                });
+            else
+                band_sums<NLB>(acc, sl, nsl, na, s_w, [&](int i, int k) {
+                    const float2 g = s_g[i];
+                    const float sg = rcp_approx(fmaf(E1[k], g.x, 1.0f));
+                    const float hv = sg * fmaf(kc.z, E4[k] * g.y, kc.w);
+                    return sg == 0.f ? 0.f : hv;
+                });
         } else {
-            for (int i = sl; i < na; i += nsl) {
+            band_sums<NLB>(acc, sl, nsl, na, s_w, [&](int i, int k) {
                 const float2 a2 = s_at[i];
-                const float h = h_value(((th.x - a2.x) + (th.y - a2.y)), kc);
+                return h_value(((th[k].x - a2.x) + (th[k].y - a2.y)), kc);
+            });
+        }
 #pragma unroll
-                for (int l = 0; l < NLB; l += 4) {
-                    const float4 w = *reinterpret_cast<const float4 *>(&s_w[i][l]);
-                    acc[l] = fmaf(w.x, h, acc[l]);
-                    acc[l + 1] = fmaf(w.y, h, acc[l + 1]);
-                    acc[l + 2] = fmaf(w.z, h, acc[l + 2]);
-                    acc[l + 3] = fmaf(w.w, h, acc[l + 3]);
-                }
+        for (int lh = 0; lh < NLB; lh += HL) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int l = 0; l < HL; ++l) s_red[sl * rows + r + k * half][l] = acc[k][lh + l];
+            __syncthreads();
+            for (int i = tid; i < rows * HL; i += CB_THREADS) {
+                const int l = i / rows, rr = i % rows, t = tb + rr;
+                float v = 0.f;
+                for (int w = 0; w < nsl; ++w) v += s_red[w * rows + rr][l];
+                if (t < tb1 && lh + l < nlh) out[(size_t)(lh + l) * steps + t] = v;
             }
+            __syncthreads();
         }
-#pragma unroll
-        for (int l = 0; l < NLB; ++l) s_red[sl * rows + r][l] = acc[l];
-        __syncthreads();
-        for (int i = tid; i < rows * NLB; i += CB_THREADS) {
-            const int l = i / rows, rr = i % rows, t = tb + rr;
-            float v = 0.f;
-            for (int w = 0; w < nsl; ++w) v += s_red[w * rows + rr][l];
-            if (t < tb1 && l < nlh) out[(size_t)l * steps + t] = v;
-        }
-        __syncthreads();
         tb += rows;
     }
 }
