@@ -45,7 +45,7 @@ using namespace ptx;
 namespace {
 
 constexpr int BM = 128, BKT = 64;
-constexpr int LF_THREADS = 128;  // threads of the moved-lead operand kernel
+constexpr int LF_THREADS = 128, LF_BLOCKS = 8;  // threads of the moved-lead operand kernel, its blocks per SM
 
 __device__ __forceinline__ float ex2a(float x) {
     float y;
@@ -429,7 +429,7 @@ constexpr int LF_ROWS = 4;  // rows per thread
 constexpr int LF_VCAP = 256;  // voxel records of a stage staged in shared memory
 static_assert(LF_THREADS >= BST + BST / 8 + 1, "the stage tables are loaded one entry per thread");
 template <bool DIAG, int ROWS, bool SPLIT, bool K0>
-__global__ void __launch_bounds__(LF_THREADS, 8) k_batch_lead_field(
+__global__ void __launch_bounds__(LF_THREADS, LF_BLOCKS) k_batch_lead_field(
     int nlog, int nst, int ngr, int ksplit_arg, int *__restrict__ work, InteriorField ic, const int64_t *__restrict__ a_vox_begin,
     const float4 *__restrict__ vox_pos, const float4 *__restrict__ vox_out, int nnb, const int8_t *__restrict__ difs,
     const float2 *__restrict__ at_hilo, const int32_t *__restrict__ a_layer, const float *__restrict__ k5l, int nl,
@@ -1292,7 +1292,7 @@ __global__ void __launch_bounds__(128) k_sim_lead_field(
 // rows the block's warps split the stage's four 8-AP chunks: ksplit groups of LF_THREADS / ksplit
 // threads, group g taking chunks g, g + ksplit, ... of the item's stage.
 template <bool DIAG, int ROWS>
-__global__ void __launch_bounds__(LF_THREADS, 8) k_sim_lead_field_rows(
+__global__ void __launch_bounds__(LF_THREADS, LF_BLOCKS) k_sim_lead_field_rows(
     int nst, int ngr, int ksplit, int *__restrict__ work, InteriorField ic, const int64_t *__restrict__ a_vox_begin,
     const float4 *__restrict__ vox_pos, const float4 *__restrict__ vox_out, int nnb, const int8_t *__restrict__ difs,
     const double *__restrict__ leads, int lead_stride, double cz, double cy, double cx, int nmove, int n_sims,
@@ -1426,6 +1426,29 @@ void launch_sim_lead_field(cudaStream_t s, const HeartDev &h, const double *d_le
     EKG_CUDA(cudaGetLastError());
 }
 
+namespace {
+// rows per thread and chunk split of the operand kernel by the rows: a warp covers 32 lanes x rows, so few
+// rows take one row per thread, and the block's warps split a stage's four 8-AP chunks when the rows fill
+// fewer than all of them (measured at 160^3 against four rows per thread and four groups: 32
+// simulations x 2 moved leads 0.208 against 0.288 ms per pass, 128 simulations 0.457 against 0.508)
+struct OperandSplit {
+    int rows_t, ksplit, ngr;  // ngr: row groups, a block's item is a stage of one group
+};
+OperandSplit operand_split(int rows_used) {
+    OperandSplit o{4, 1, 1};
+    if (rows_used <= 32) o.rows_t = 1, o.ksplit = 4;
+    else if (rows_used <= 64) o.rows_t = 1, o.ksplit = 2;
+    else if (rows_used <= 128) o.rows_t = 1, o.ksplit = 1;
+    else if (rows_used <= 256) o.rows_t = 4, o.ksplit = 2;
+    const int grows = LF_THREADS / o.ksplit * o.rows_t;
+    o.ngr = (rows_used + grows - 1) / grows;
+    return o;
+}
+}  // namespace
+bool batch_operand_fills(const HeartDev &h, int rows_used, int sm_count) {
+    return h.apad / BST * operand_split(rows_used).ngr >= (int64_t)LF_BLOCKS * sm_count;
+}
+
 void launch_batch_lead_field(cudaStream_t s, const HeartDev &h, int tile_rows, bool small, int blocks_per_sm,
                              const float *k5l,
                              const float4 *hconst, const float4 *lrel, int nmove, int n_sims, const BandArgs &B,
@@ -1460,17 +1483,8 @@ void launch_batch_lead_field(cudaStream_t s, const HeartDev &h, int tile_rows, b
         EKG_CUDA(cudaGetLastError());
         return;
     }
-    // rows per thread and chunk split by the rows: a warp covers 32 lanes x rows, so few rows take
-    // one row per thread, and the block's warps split a stage's four 8-AP chunks when the rows fill
-    // fewer than all of them (measured at 160^3 against four rows per thread and four groups: 32
-    // simulations x 2 moved leads 0.208 against 0.288 ms per pass, 128 simulations 0.457 against 0.508)
-    int rows_t = 4, ksplit = 1;
-    if (rows_used <= 32) rows_t = 1, ksplit = 4;
-    else if (rows_used <= 64) rows_t = 1, ksplit = 2;
-    else if (rows_used <= 128) rows_t = 1, ksplit = 1;
-    else if (rows_used <= 256) rows_t = 4, ksplit = 2;
-    const int grows = LF_THREADS / ksplit * rows_t;
-    const int ngr = (rows_used + grows - 1) / grows;
+    const OperandSplit split = operand_split(rows_used);
+    const int rows_t = split.rows_t, ksplit = split.ksplit, ngr = split.ngr;
     EKG_CUDA(cudaMemsetAsync(work, 0, sizeof(int), s));
     auto go = [&](auto kern) {
         static int per_sm = 0;

@@ -372,6 +372,8 @@ void launch_reduce_layers(cudaStream_t s, int steps, int rows, int nl, const int
 void launch_static_combine(cudaStream_t s, const HeartDev &h, int J, int Jb, int nmove, int n_sims, const float *F,
                            const float *coef, const double *k3, const float *Q1, const float *Q2, double *ecg,
                            float2 *ecg_ff, const double *cst = nullptr);
+// whether the operand kernel's items (stages x row groups) are at least one wave of its blocks
+bool batch_operand_fills(const HeartDev &h, int rows_used, int sm_count);
 void launch_batch_lead_field(cudaStream_t s, const HeartDev &h, int tile_rows, bool small, int blocks_per_sm,
                              const float *k5l,
                              const float4 *hconst, const float4 *lrel, int nmove, int n_sims, const BandArgs &B,

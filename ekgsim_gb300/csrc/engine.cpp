@@ -1078,8 +1078,14 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     // operand kernel, which needs neither) and the steady-sum reduction (beside the band GEMM) run on the
     // auxiliary stream, joined before the band reduction
     // (measured: other placements of the small kernels, such as the criteria of the static leads
-    // beside the GEMM, lengthen the pass)
-    const bool fork = P.batch && nmove > 0;
+    // beside the GEMM, lengthen the pass).  Without static leads only the layer factors can be hidden, and
+    // their blocks, which start first, unbalance an operand grid that is less than one wave (64^3, two
+    // moved leads, us per pass beside each other / in a row: 17 simulations 84 / 91, 32 105 / 102,
+    // 100 186 / 168, 200 272 / 244); a fuller one deals its items as blocks come free (96^3, 12 moved
+    // leads: 40 simulations 381 / 390, 256 1035 / 1097)
+    const bool fork = P.batch && nmove > 0 &&
+                      (nmove < (int)L || n_sims * D.nlayers <= h->sm_count / 2 ||
+                       batch_operand_fills(D, P.rows_used, h->sm_count));
     if (fork) {
         if (!h->aux_stream) {
             EKG_CUDA(cudaStreamCreateWithFlags(&h->aux_stream, cudaStreamNonBlocking));
