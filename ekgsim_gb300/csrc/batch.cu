@@ -121,17 +121,22 @@ __global__ void k_reduce_layers(int steps, int rows, int nl, const int32_t *__re
 // per layer in FP32 (the basis is stored in FP32), the sum over layers in float-float; written as
 // FP64 and as float-float.  Block = 128 steps of one static lead for SC_SIMS simulations: a
 // thread loads the basis rows of its step once per layer and applies them to every simulation of
-// the group (coefficients broadcast from shared memory).  With few simulations a layer is a handful of
-// operations behind a load, so the coefficients of SC_LAYERS layers are staged at once and the next
-// layer's basis rows are on their way while one is summed.
+// the group (coefficients broadcast from shared memory, four at a time).  With few simulations a layer
+// is a handful of operations behind a load, so the coefficients of SC_LAYERS layers are staged at once and
+// the next layer's basis rows are on their way while one is summed.  Bound by FP32 issue, so the number of
+// terms is compiled in and a layer's factors of the 16 simulations are loaded together: the band GEMM,
+// which finds no room beside these blocks, waits for them where there are many (256^3, ten layers, 64
+// simulations x 62 static leads: 224 us, now 141; 160^3, 256 x 10: 74, now 57).
 constexpr int SC_SIMS = 16, SC_LAYERS = 8;
-__global__ void __launch_bounds__(128) k_static_combine(int steps, int nleads, int nl, int J, int Jb, int nmove,
+template <int JP>  // terms per sum: J, or the next size that is compiled (further coefficients are 0)
+__global__ void __launch_bounds__(128, 4) k_static_combine(int steps, int nleads, int nl, int J, int Jb, int nmove,
                                                         int n_sims, const float *__restrict__ F,
                                                         const float *__restrict__ coef, const double *__restrict__ k3,
                                                         const float *__restrict__ Q1, const float *__restrict__ Q2,
                                                         double *__restrict__ ecg, float2 *__restrict__ ecg_ff,
                                                         const double *__restrict__ cst) {
-    __shared__ float s_c[SC_LAYERS][SC_SIMS][11];  // [layer][simulation][j < J: coefficient, 10: k3]
+    constexpr int CW = (JP + 4) / 4 * 4;  // [j < J: coefficient, JP: k3]
+    __shared__ __align__(16) float s_c[SC_LAYERS][SC_SIMS][CW];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int l = nmove + blockIdx.y, s0 = blockIdx.z * SC_SIMS;
     const int ns = min(SC_SIMS, n_sims - s0);
@@ -141,11 +146,11 @@ __global__ void __launch_bounds__(128) k_static_combine(int steps, int nleads, i
     float2 acc[SC_SIMS];
 #pragma unroll
     for (int i = 0; i < SC_SIMS; ++i) acc[i] = make_float2(0.f, 0.f);
-    float n1[10], n2[10];  // the next layer's basis rows
+    float n1[JP], n2[JP];  // the next layer's basis rows
     auto fetch = [&](int L) {
         const size_t q0 = ((size_t)L * rows + (size_t)l * Jb) * steps + tc;
 #pragma unroll
-        for (int j = 0; j < 10; ++j) {  // J <= 10 (the basis order)
+        for (int j = 0; j < JP; ++j) {
             n1[j] = j < J ? Q1[q0 + (size_t)j * steps] : 0.f;
             n2[j] = j < J ? Q2[q0 + (size_t)j * steps] : 0.f;
         }
@@ -154,32 +159,38 @@ __global__ void __launch_bounds__(128) k_static_combine(int steps, int nleads, i
     for (int L0 = 0; L0 < nl; L0 += SC_LAYERS) {
         const int nL = min(SC_LAYERS, nl - L0);
         __syncthreads();
-        for (int k = threadIdx.x; k < nL * ns * 11; k += blockDim.x) {
-            const int Lk = k / (ns * 11), i = (k / 11) % ns, j = k % 11;
+        for (int k = threadIdx.x; k < nL * ns * CW; k += blockDim.x) {
+            const int Lk = k / (ns * CW), i = (k / CW) % ns, j = k % CW;
             const size_t sl = (size_t)(s0 + i) * nl + L0 + Lk;
-            s_c[Lk][i][j] = j < J ? coef[sl * J + j] : (j == 10 ? (float)k3[sl] : 0.f);
+            s_c[Lk][i][j] = j < J ? coef[sl * J + j] : (j == JP ? (float)k3[sl] : 0.f);
         }
         __syncthreads();
+#pragma unroll 1
         for (int Lk = 0; Lk < nL; ++Lk) {
-            float q1[10], q2[10];
+            const int L = L0 + Lk;
+            float q1[JP], q2[JP], f[SC_SIMS];
 #pragma unroll
-            for (int j = 0; j < 10; ++j) {
+            for (int j = 0; j < JP; ++j) {
                 q1[j] = n1[j];
                 q2[j] = n2[j];
             }
-            const int L = L0 + Lk;
+#pragma unroll
+            for (int i = 0; i < SC_SIMS; ++i) f[i] = i < ns ? F[((size_t)(s0 + i) * nl + L) * steps + tc] : 0.f;
             if (L + 1 < nl) fetch(L + 1);
 #pragma unroll
             for (int i = 0; i < SC_SIMS; ++i)
                 if (i < ns) {
+                    float c[CW];
+#pragma unroll
+                    for (int j = 0; j < CW; j += 4)
+                        *reinterpret_cast<float4 *>(&c[j]) = *reinterpret_cast<const float4 *>(&s_c[Lk][i][j]);
                     float v1 = 0.f, v2 = 0.f;
 #pragma unroll
-                    for (int j = 0; j < 10; ++j)
-                        if (j < J) {
-                            v1 = fmaf(s_c[Lk][i][j], q1[j], v1);
-                            v2 = fmaf(s_c[Lk][i][j], q2[j], v2);
-                        }
-                    acc[i] = ff_add_f(acc[i], F[((size_t)(s0 + i) * nl + L) * steps + tc] * fmaf(s_c[Lk][i][10], v2 - v1, v1));
+                    for (int j = 0; j < JP; ++j) {
+                        v1 = fmaf(c[j], q1[j], v1);
+                        v2 = fmaf(c[j], q2[j], v2);
+                    }
+                    acc[i] = ff_add_f(acc[i], f[i] * fmaf(c[JP], v2 - v1, v1));
                 }
         }
     }
@@ -1205,8 +1216,13 @@ void launch_static_combine(cudaStream_t s, const HeartDev &h, int J, int Jb, int
                            float2 *ecg_ff, const double *cst) {
     if (nmove >= h.nleads) return;
     dim3 grid((unsigned)((h.steps + 127) / 128), (unsigned)(h.nleads - nmove), (unsigned)((n_sims + SC_SIMS - 1) / SC_SIMS));
-    k_static_combine<<<grid, 128, 0, s>>>(h.steps, h.nleads, h.nlayers, J, Jb, nmove, n_sims, F, coef, k3, Q1, Q2,
-                                          ecg, ecg_ff, cst);
+    auto go = [&](auto kern) {
+        kern<<<grid, 128, 0, s>>>(h.steps, h.nleads, h.nlayers, J, Jb, nmove, n_sims, F, coef, k3, Q1, Q2, ecg, ecg_ff,
+                                  cst);
+    };
+    if (J <= 6) go(k_static_combine<6>);
+    else if (J <= 8) go(k_static_combine<8>);
+    else go(k_static_combine<10>);
     EKG_CUDA(cudaGetLastError());
 }
 

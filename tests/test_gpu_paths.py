@@ -116,3 +116,68 @@ def test_few_simulations_operand(engine, kind, sims, moved, nhood):
         ref = O.run(layer, at, lk, move_leads(leads, genes[i, 12:].reshape(-1, 2)), nhood, 0.0, 150.0, 1.0)
         assert rel_l2(ecg[i], ref) <= ECG_TOL, i
     h.close()
+
+
+def small_heart(engine, n, n_leads, steps, free, seed):
+    from ekgsim_gb300.engine import Heart
+    spec = synth.small_spec(n, n_leads=n_leads, seed=seed)
+    grid, tm = synth.ellipsoid_heart(spec), synth.transfer_matrix(3, spec.delays)
+    rng = np.random.Generator(np.random.PCG64(seed))
+    leads = synth.leads(spec, rng)[:, ::-1].copy()
+    h = Heart.create(engine, grid, tm, leads, "3D4", 0.0, float(steps), 1.0)
+    h.set_eval([synth.BASE_AP] * 3, synth.K_MIN, synth.K_MAX, free, list(synth.analytic_target(n_leads, steps, 3)),
+               mid_position=0.6)
+    return h, O.activation(grid, tm), leads, rng
+
+
+def check_sims(h, act, leads, rng, sims, moved, free, steps):
+    from ekgsim_gb300.engine import layer_aps, move_leads
+    at, layer = act
+    nk, nl = 3 * len(free), len(leads)
+    lo, hi = np.array(synth.K_MIN)[free], np.array(synth.K_MAX)[free]
+    genes = np.zeros((sims, nk + 2 * nl))
+    genes[:, :nk] = np.tile(lo, 3) + np.tile(hi - lo, 3) * rng.random((sims, nk))
+    genes[:, nk:nk + 2 * moved] = rng.uniform(-15, 15, size=(sims, 2 * moved))
+    ecg = h.eval_batch(genes, want_ecg=True)[2]
+    for i in {0, sims // 2, sims - 1}:
+        lk = layer_aps(h._cfg, 3, genes[i, :nk])[0]
+        ref = O.run(layer, at, lk, move_leads(leads, genes[i, nk:].reshape(-1, 2)), "3D4", 0.0, float(steps), 1.0)
+        assert rel_l2(ecg[i], ref) <= ECG_TOL, i
+
+
+@pytest.mark.parametrize("n_leads,steps", [(1, 61), (4, 300), (5, 97), (12, 257), (13, 64), (17, 129)])
+def test_band_contraction_leads(engine, n_leads, steps):
+    """Upstrokes that differ per simulation: every compiled number of leads per block, a block with few of its
+    leads, steps that are no multiple of a pass or of the probes of a run's end."""
+    free = [1, 5, 6, 7, 8]
+    h, act, leads, rng = small_heart(engine, 22, n_leads, steps, free, seed=n_leads)
+    check_sims(h, act, leads, rng, 9, min(2, n_leads), free, steps)
+    h.close()
+
+
+@pytest.mark.parametrize("sims,moved,steps", [
+    (3, 2, 1400),    # as many steady entries per layer as there can be
+    (467, 3, 300),   # outputs of the steady sums: thousands, no multiple of a warp's four
+    (33, 1, 128),    # a group of 16 simulations with one of them
+])
+def test_steady_sums_and_static_leads(engine, sims, moved, steps):
+    """Batched passes with moved and static leads: the steady sums' two passes, the static leads' groups."""
+    free = [5, 6, 7, 8]
+    h, act, leads, rng = small_heart(engine, 20, 5, steps, free, seed=sims)
+    check_sims(h, act, leads, rng, sims, moved, free, steps)
+    h.close()
+
+
+def test_fresh_result_pages(engine):
+    """Results into memory that was never touched, at an odd offset in its pages: what goes into touched memory."""
+    import mmap
+    from ekgsim_gb300 import _lib as L
+    h, act, leads, rng = small_heart(engine, 40, 2, 50, [5, 6, 7, 8], seed=1)
+    want = h.activation()
+    fresh = mmap.mmap(-1, want.nbytes + 4096)
+    base = ctypes.addressof(ctypes.c_char.from_buffer(fresh))
+    L.check(L.load().ekg_heart_activation(h._h, ctypes.cast(base + 1000, ctypes.POINTER(ctypes.c_double))))
+    got = np.frombuffer(ctypes.string_at(base, len(fresh)), dtype=np.uint8)
+    assert np.array_equal(got[1000:1000 + want.nbytes], want.reshape(-1).view(np.uint8))
+    assert not got[:1000].any() and not got[1000 + want.nbytes:].any()
+    h.close()
