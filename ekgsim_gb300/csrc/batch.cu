@@ -730,61 +730,98 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
 // Steady sums per (row', layer, entry): U[row'][L][e] = sum over the layer's stages [ls0, ls1)
 // below the entry's prefix end of (P1[st][row'].x, G_e[st] P1[st][row'].y) (U0, U1),
 // G_e[st] = gtab[goff[L][e] + st - ls0[L]].  Two passes in a fixed order: k_band_u sums BU_PARTS
-// consecutive parts of the stage range in FP32 (a few stages each), block per (part, 128 rows,
-// layer), thread per row, all entries from one read of P1 (small blocks that fit beside the band
-// GEMM's CTAs, which they run next to); k_band_u2 adds the parts in FP64, one warp per output.
-// Up: [parts][rows][nl][max_ent]; U stored in FP32.  The prefix ends ascend with e.
-constexpr int BU_PARTS = 128;
-__global__ void __launch_bounds__(128, 8) k_band_u(int rows_used, int nl, int max_ent,
-                                                   const int32_t *__restrict__ nent, const int32_t *__restrict__ esplit,
-                                                   const int32_t *__restrict__ ls0, const int32_t *__restrict__ ls1,
-                                                   const int64_t *__restrict__ goff, const float *__restrict__ gtab,
-                                                   const float2 *__restrict__ P1, float2 *__restrict__ Up) {
+// consecutive parts of the stage range in FP32 (a few stages each), a warp per (part, 32 rows, layer),
+// thread per row, all entries from one read of P1, BU_AHEAD stages' values loaded at once; k_band_u2 adds
+// the parts in FP64.  Up: [parts][rows][nl][max_ent]; U stored in FP32.  The prefix ends ascend with e.
+// Both run beside the band GEMM, but the GEMM's ten warps leave no registers for another block (168 a
+// thread; at 152 they share an SM and the GEMM takes 115 us instead of 102), so they live on the SMs that
+// it leaves or ends on: one-warp blocks are placed there soonest (160^3, 256 simulations x 2 moved leads:
+// the sums are ready 20 us behind the GEMM with 128-thread blocks and a warp per output in k_band_u2, now
+// 12; where the GEMM is short the second pass is the longer one: 96^3, 17 simulations: 25 us to 6).
+constexpr int BU_PARTS = 128, BU_AHEAD = 4, BU_THREADS = 32;
+template <int ME>  // entries a layer has at most
+__global__ void __launch_bounds__(BU_THREADS, 32) k_band_u(int rows_used, int nl, int max_ent,
+                                                    const int32_t *__restrict__ nent, const int32_t *__restrict__ esplit,
+                                                    const int32_t *__restrict__ ls0, const int32_t *__restrict__ ls1,
+                                                    const int64_t *__restrict__ goff, const float *__restrict__ gtab,
+                                                    const float2 *__restrict__ P1, float2 *__restrict__ Up) {
     const int p = blockIdx.x, L = blockIdx.z;
     const int rr = blockIdx.y * blockDim.x + threadIdx.x;
     if (rr >= rows_used) return;
-    const int ne = nent[L], n = ls1[L] - ls0[L];
-    const int g0 = ls0[L] + (int)((int64_t)n * p / BU_PARTS), g1 = ls0[L] + (int)((int64_t)n * (p + 1) / BU_PARTS);
-    int ge[MAXE];
-    const float *gt[MAXE];  // entry e's factor of stage g: gt[e][g - g0]
+    const int ne = nent[L], l0 = ls0[L], n = ls1[L] - l0;
+    const int g0 = l0 + (int)((int64_t)n * p / BU_PARTS), g1 = l0 + (int)((int64_t)n * (p + 1) / BU_PARTS);
+    int ge[ME], gt[ME];  // entry e: end of its prefix; its factor of stage g: gtab[gt[e] + g]
+    int gend = g0;
 #pragma unroll
-    for (int e = 0; e < MAXE; ++e) {
-        ge[e] = e < ne ? min(g1, esplit[L * MAXE + e]) : g0;
-        gt[e] = gtab + (e < ne ? goff[L * MAXE + e] + (g0 - ls0[L]) : 0);
+    for (int e = 0; e < ME; ++e) {
+        const int end = esplit[L * MAXE + e], off = (int)goff[L * MAXE + e];
+        ge[e] = e < ne ? min(g1, end) : g0;
+        gt[e] = off - l0;
+        gend = max(gend, ge[e]);
     }
-    const int gend = ne > 0 ? ge[ne - 1] : g0;
-    float a[MAXE], b[MAXE];
+    float a[ME], b[ME];
 #pragma unroll
-    for (int e = 0; e < MAXE; ++e) a[e] = b[e] = 0.f;
-    for (int g = g0; g < gend; ++g) {
-        const float2 v = P1[(size_t)g * rows_used + rr];
+    for (int e = 0; e < ME; ++e) a[e] = b[e] = 0.f;
+    for (int g = g0; g < gend; g += BU_AHEAD) {
+        float2 v[BU_AHEAD];
 #pragma unroll
-        for (int e = 0; e < MAXE; ++e)
-            if (g < ge[e]) {
-                a[e] += v.x;
-                b[e] = fmaf(gt[e][g - g0], v.y, b[e]);
-            }
+        for (int k = 0; k < BU_AHEAD; ++k) v[k] = P1[(size_t)min(g + k, gend - 1) * rows_used + rr];
+#pragma unroll
+        for (int e = 0; e < ME; ++e) {
+            float w[BU_AHEAD];
+#pragma unroll
+            for (int k = 0; k < BU_AHEAD; ++k) w[k] = g + k < ge[e] ? gtab[gt[e] + g + k] : 0.f;
+#pragma unroll
+            for (int k = 0; k < BU_AHEAD; ++k)
+                if (g + k < ge[e]) {
+                    a[e] += v[k].x;
+                    b[e] = fmaf(w[k], v[k].y, b[e]);
+                }
+        }
     }
 #pragma unroll
-    for (int e = 0; e < MAXE; ++e)
+    for (int e = 0; e < ME; ++e)
         if (e < ne) Up[(((size_t)p * rows_used + rr) * nl + L) * max_ent + e] = make_float2(a[e], b[e]);
 }
 
-__global__ void __launch_bounds__(256) k_band_u2(int64_t n_out, const float2 *__restrict__ Up, float2 *__restrict__ U) {
-    const int lane = threadIdx.x & 31;
-    const int64_t i = blockIdx.x * 8 + (threadIdx.x >> 5);  // one warp per output
-    if (i >= n_out) return;
-    double a = 0.0, b = 0.0;
-    for (int p = lane; p < BU_PARTS; p += 32) {
-        const float2 v = Up[p * n_out + i];
-        a += (double)v.x;
-        b += (double)v.y;
+// A warp takes O outputs (4 where there are many): lane p adds parts p, p + 32, ..., then 2 O values per lane
+// are added over the lanes by recursive halving (in the order of an xor tree), which takes 9 FP64 additions
+// for four outputs instead of 40.  Bound by the FP64 pipe.
+template <int O>
+__global__ void __launch_bounds__(32) k_band_u2(int64_t n_out, const float2 *__restrict__ Up, float2 *__restrict__ U) {
+    const int lane = threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * O;
+    float2 v[O][BU_PARTS / 32];
+#pragma unroll
+    for (int q = 0; q < O; ++q)
+#pragma unroll
+        for (int k = 0; k < BU_PARTS / 32; ++k) v[q][k] = Up[(lane + k * 32) * n_out + min(i + q, n_out - 1)];
+    double x[2 * O];
+#pragma unroll
+    for (int q = 0; q < O; ++q) {
+        x[q] = (double)v[q][0].x;
+        x[O + q] = (double)v[q][0].y;
+#pragma unroll
+        for (int k = 1; k < BU_PARTS / 32; ++k) {
+            x[q] += (double)v[q][k].x;
+            x[O + q] += (double)v[q][k].y;
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
+    int idx = 0, d = 16;
+#pragma unroll
+    for (int n = O; n >= 1; n >>= 1, d >>= 1) {
+        const bool up = lane & d;
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+            const double keep = up ? x[j + n] : x[j], give = up ? x[j] : x[j + n];
+            x[j] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+        }
+        idx += up ? n : 0;
     }
-    if (lane == 0) U[i] = make_float2((float)a, (float)b);
+#pragma unroll
+    for (; d >= 1; d >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], d);
+    // value idx: S0 of output idx, or S1 of output idx - O; lanes that share one write the same
+    if (i + idx % O < n_out) reinterpret_cast<float *>(U)[(i + idx % O) * 2 + idx / O] = (float)x[0];
 }
 
 // ------------------------------------------------------------------ batch GEMM
@@ -1675,10 +1712,15 @@ void launch_w0_layer_sums(cudaStream_t s, const HeartDev &h, const float *W0, do
 int band_u_parts() { return BU_PARTS; }
 
 void launch_band_u(cudaStream_t s, const BandArgs &A) {
-    k_band_u<<<dim3(BU_PARTS, (unsigned)((A.rows_used + 127) / 128), (unsigned)A.nl), 128, 0, s>>>(
-        A.rows_used, A.nl, A.max_ent, A.nent, A.esplit, A.ls0, A.ls1, A.goff, A.gtab, A.P1, A.Up);
+    const dim3 grid(BU_PARTS, (unsigned)((A.rows_used + BU_THREADS - 1) / BU_THREADS), (unsigned)A.nl);
+    auto go = [&](auto kern) {
+        kern<<<grid, BU_THREADS, 0, s>>>(A.rows_used, A.nl, A.max_ent, A.nent, A.esplit, A.ls0, A.ls1, A.goff, A.gtab, A.P1, A.Up);
+    };
+    if (A.max_ent <= 4) go(k_band_u<4>);
+    else go(k_band_u<MAXE>);
     const int64_t n = (int64_t)A.rows_used * A.nl * A.max_ent;
-    k_band_u2<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(n, A.Up, A.U);
+    if (n >= 4096) k_band_u2<4><<<(unsigned)((n + 3) / 4), 32, 0, s>>>(n, A.Up, A.U);
+    else k_band_u2<1><<<(unsigned)n, 32, 0, s>>>(n, A.Up, A.U);
     EKG_CUDA(cudaGetLastError());
 }
 
