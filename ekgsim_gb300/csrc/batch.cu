@@ -1438,7 +1438,6 @@ void launch_sim_lead_field_rows(cudaStream_t s, const HeartDev &h, const double 
     const int nst = (int)(h.apad / BST);
     const int items = nst * ngr;
     const int grid = std::max(1, std::min(items, sm_count * 8));
-    EKG_CUDA(cudaMemsetAsync(work, 0, sizeof(int), s));
     auto go = [&](auto kern) {
         kern<<<grid, LF_THREADS, 0, s>>>(nst, ngr, ksplit, work, ic, h.a_vox_begin.p, h.vox_pos.p, h.vox_out.p, h.nnb,
                                          h.difs.p, d_leads, lead_stride, h.centre[0], h.centre[1], h.centre[2], nmove,
@@ -1538,7 +1537,6 @@ void launch_batch_lead_field(cudaStream_t s, const HeartDev &h, int tile_rows, b
     }
     const OperandSplit split = operand_split(rows_used);
     const int rows_t = split.rows_t, ksplit = split.ksplit, ngr = split.ngr;
-    EKG_CUDA(cudaMemsetAsync(work, 0, sizeof(int), s));
     auto go = [&](auto kern) {
         static int per_sm = 0;
         if (!per_sm) EKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, LF_THREADS, 0));

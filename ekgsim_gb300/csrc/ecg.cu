@@ -846,9 +846,59 @@ __global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, 
     }
 }
 
+// ------------------------------------------------------------------ a pass's inputs and results
+// Copies between page-locked host memory and the device by a kernel of the pass itself: between two
+// kernels a copy or memset node costs its hand-over to the copy engine and back, 3 to 9 us of a pass that
+// takes 30 to 100 (64^3, one simulation: evaluation 64 us with copy nodes, 56.5 without; 96^3, 17
+// simulations: 126, 112).  k_pass_in also clears the item counter that the pass's operand kernel takes from.
+constexpr int PIO_THREADS = 256, PIO_UNROLL = 4;
+template <class T>
+__device__ __forceinline__ void pass_copy(const T *__restrict__ src, T *__restrict__ dst, int64_t n) {
+    const int64_t stride = (int64_t)gridDim.x * PIO_THREADS;
+    for (int64_t i = (int64_t)blockIdx.x * PIO_THREADS + threadIdx.x; i < n; i += stride * PIO_UNROLL) {
+        T v[PIO_UNROLL];
+#pragma unroll
+        for (int k = 0; k < PIO_UNROLL; ++k)
+            if (i + k * stride < n) v[k] = src[i + k * stride];
+#pragma unroll
+        for (int k = 0; k < PIO_UNROLL; ++k)
+            if (i + k * stride < n) dst[i + k * stride] = v[k];
+    }
+}
+__global__ void __launch_bounds__(PIO_THREADS) k_pass_in(const uint4 *src, uint4 *dst, int64_t n, int *work) {
+    if (work && blockIdx.x == 0 && threadIdx.x == 0) *work = 0;
+    pass_copy(src, dst, n);
+}
+__global__ void __launch_bounds__(PIO_THREADS) k_pass_out(const double *src, double *dst, int64_t n) {
+    pass_copy(src, dst, n);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
+// up to these sizes by kernel, larger ones by the copy engine
+constexpr size_t PASS_IN_MAX = 1 << 20, PASS_OUT_MAX = 1 << 18;
+static unsigned pass_blocks(size_t n) {
+    return (unsigned)std::max<size_t>(1, (n + PIO_THREADS - 1) / PIO_THREADS);
+}
+void launch_pass_in(cudaStream_t s, const uint8_t *host, uint8_t *dev, size_t bytes, int *work) {
+    const bool copy = bytes > PASS_IN_MAX;
+    if (copy) EKG_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s));
+    const size_t n = copy ? 0 : bytes / 16;
+    if (n == 0 && !work) return;
+    k_pass_in<<<std::min(152u, pass_blocks(n)), PIO_THREADS, 0, s>>>(reinterpret_cast<const uint4 *>(host),
+                                                                    reinterpret_cast<uint4 *>(dev), (int64_t)n, work);
+    EKG_CUDA(cudaGetLastError());
+}
+void launch_pass_out(cudaStream_t s, const double *dev, double *host, size_t n) {
+    if (n == 0) return;
+    if (n * sizeof(double) > PASS_OUT_MAX) {
+        EKG_CUDA(cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+        return;
+    }
+    k_pass_out<<<std::min(152u, pass_blocks(n)), PIO_THREADS, 0, s>>>(dev, host, (int64_t)n);
+    EKG_CUDA(cudaGetLastError());
+}
 void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads, int nleads_in, int lead_stride,
                        int n_sims, float *d_W, int w_lead_stride) {
     dim3 grid((unsigned)((h.apad + 127) / 128), (unsigned)nleads_in, (unsigned)n_sims);

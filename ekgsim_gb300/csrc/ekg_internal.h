@@ -284,6 +284,10 @@ struct EvalDev {
 
 void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads, int nleads_in, int lead_stride,
                        int n_sims, float *d_W, int w_lead_stride);
+// a pass's staged inputs from page-locked memory (16-byte aligned, a multiple of 16 bytes) and its item counter
+// cleared; its first n result values to page-locked memory
+void launch_pass_in(cudaStream_t s, const uint8_t *host, uint8_t *dev, size_t bytes, int *work);
+void launch_pass_out(cudaStream_t s, const double *dev, double *host, size_t n);
 void launch_layer_factors(cudaStream_t s, const HeartDev &h, const double *d_layer_k, const double *d_cpre,
                           int n_sims, double *d_F, float *d_Ff, float *d_layer_c, const double *d_centre = nullptr,
                           const double *d_scale = nullptr, int J = 0, float *d_coef = nullptr);

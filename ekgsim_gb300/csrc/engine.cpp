@@ -1097,7 +1097,7 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     int launches = 0;
     if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[0], s));
     const ekg_heart::Staging &sg = h->stg[h->cur];
-    if (io.in && sg.used) EKG_CUDA(cudaMemcpyAsync(sg.dev.p, sg.host, sg.used, cudaMemcpyHostToDevice, s));
+    launch_pass_in(s, sg.host, sg.dev.p, io.in ? sg.used : 0, P.batch ? h->bs.work.p : E.work.p);
     const ekg_heart::PassInputs &in = h->in();
     // batched form with moved leads: the layer factors and the static combine (beside the moved-lead
     // operand kernel, which needs neither) and the steady-sum reduction (beside the band GEMM) run on the
@@ -1147,7 +1147,8 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
         }
         static_part();
         if (nmove > 0) {
-            if (P.rows_used < P.rows) EKG_CUDA(cudaMemsetAsync(B.Bt.p, 0, (size_t)P.rows * D.apad * 4, s));
+            // (the tile's rows past rows_used keep what is there: a row of B only enters its own column of
+            // the product, and those columns are not read)
             BandArgs U;
             U.n_sims = n_sims;
             U.nmove = nmove;
@@ -1287,7 +1288,7 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
                         E.targets_ff.p, E.target_len.p, E.target_off.p, E.crit);
         ++launches;
     }
-    if (io.out_n) EKG_CUDA(cudaMemcpyAsync(io.out, E.out.p, io.out_n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    launch_pass_out(s, E.out.p, io.out, io.out_n);
     if (tm && tm->on) EKG_CUDA(cudaEventRecord(tm->ev[3], s));
     g_launch_count = launches;
 }

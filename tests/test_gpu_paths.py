@@ -159,6 +159,7 @@ def test_band_contraction_leads(engine, n_leads, steps):
     (3, 2, 1400),    # as many steady entries per layer as there can be
     (467, 3, 300),   # outputs of the steady sums: thousands, no multiple of a warp's four
     (33, 1, 128),    # a group of 16 simulations with one of them
+    (4000, 1, 64),   # inputs and criteria too large for the pass's own copies
 ])
 def test_steady_sums_and_static_leads(engine, sims, moved, steps):
     """Batched passes with moved and static leads: the steady sums' two passes, the static leads' groups."""
