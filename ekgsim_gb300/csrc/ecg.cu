@@ -121,41 +121,56 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
 // passes, where the FP64 pow/log would be one block's latency), else NULL.  With them the steps are cut
 // into blocks too (grid.y): a pass of one simulation has only as many (sim, layer) pairs as layers, whose
 // five steps a thread, one behind the other, took 7.7 us (three layers, 600 steps).
-__global__ void k_layer_factors(int nl, int steps, const double *__restrict__ t, const double *__restrict__ layer_k,
-                                const double *__restrict__ cpre, int n_sims, double *__restrict__ F,
-                                float *__restrict__ Ff, float *__restrict__ layer_c, const double *__restrict__ centre,
-                                const double *__restrict__ scale, int J, float *__restrict__ coef) {
-    const int64_t sl = blockIdx.x;  // sim * nl + layer
-    const double *k = layer_k + sl * 9;
-    __shared__ double c;
-    if (threadIdx.x == 0) {
-        c = cpre ? cpre[sl] : log(pow(2.0, k[7] / k[6]) - 1);
-    }
-    if (threadIdx.x == 0 && blockIdx.y == 0) {
-        const double L2E = 1.4426950408889634;
-        reinterpret_cast<float4 *>(layer_c)[sl] =
-            make_float4((float)(k[1] * L2E), (float)(k[4] * L2E), (float)(1.0 - k[3]), (float)k[3]);
-    } else if (threadIdx.x == 32 && blockIdx.y == 0 && coef) {
-        // Taylor coefficients of the static-lead basis: coef[sl][j] = exp(k5 c_L) (k5 s_L)^j / j!
-        const int L = (int)(sl % nl);
-        const double x = k[5] * scale[L];
-        double e = exp(k[5] * centre[L]);
-        for (int j = 0; j < J; ++j) {
-            coef[sl * J + j] = (float)e;
-            e *= x / (j + 1);
+//
+// Without them a block takes up to FACTOR_PAIRS pairs, a lane per pair for the FP64 constants (logarithm,
+// powers, the coefficients' quotients: chains of some 300 FP64 instructions, which cost the FP64 pipe the
+// same for one lane as for 32).  Beside the moved-lead operand kernel (which takes every register it finds)
+// the pairs are dealt to one block per SM: with a block per pair they filled the chip, and the operand,
+// 20 times as long, waited (160^3, 256 simulations x 3 layers: 26 us, FP64-bound).
+constexpr int FACTOR_PAIRS = 32;
+__global__ void __launch_bounds__(128) k_layer_factors(
+    int nl, int steps, const double *__restrict__ t, const double *__restrict__ layer_k, const double *__restrict__ cpre,
+    int64_t pairs, int per, double *__restrict__ F, float *__restrict__ Ff, float *__restrict__ layer_c,
+    const double *__restrict__ centre, const double *__restrict__ scale, int J, float *__restrict__ coef) {
+    const int64_t p0 = (int64_t)blockIdx.x * per;  // pair = sim * nl + layer
+    const int np = (int)min((int64_t)per, pairs - p0);
+    __shared__ double c[FACTOR_PAIRS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane < np) {
+        const int64_t sl = p0 + lane;
+        const double *k = layer_k + sl * 9;
+        if (warp == 0) {
+            c[lane] = cpre ? cpre[sl] : log(pow(2.0, k[7] / k[6]) - 1);
+        } else if (warp == 1 && blockIdx.y == 0 && coef) {
+            // Taylor coefficients of the static-lead basis: coef[sl][j] = exp(k5 c_L) (k5 s_L)^j / j!
+            const int L = (int)(sl % nl);
+            const double x = k[5] * scale[L];
+            double e = exp(k[5] * centre[L]);
+            for (int j = 0; j < J; ++j) {
+                coef[sl * J + j] = (float)e;
+                e *= x / (j + 1);
+            }
+        } else if (warp == 2 && blockIdx.y == 0) {
+            const double L2E = 1.4426950408889634;
+            reinterpret_cast<float4 *>(layer_c)[sl] =
+                make_float4((float)(k[1] * L2E), (float)(k[4] * L2E), (float)(1.0 - k[3]), (float)k[3]);
         }
     }
     __syncthreads();
-    const float r = (float)(k[6] / k[7]);
-    for (int step = blockIdx.y * blockDim.x + threadIdx.x; step < steps; step += gridDim.y * blockDim.x) {
-        const double tt = t[step];
-        const float u = (float)fma(-k[7], tt - k[8], c);
-        const float sp = u > 0.f ? u + log1pf(expf(-u)) : log1pf(expf(u));
-        const float R = -expm1f(-r * sp);
-        const float e5 = expf((float)(-k[5] * tt));
-        const double f = k[2] * (double)e5 * (double)R;
-        F[sl * steps + step] = f;
-        Ff[sl * steps + step] = (float)f;
+    for (int i = 0; i < np; ++i) {
+        const int64_t sl = p0 + i;
+        const double *k = layer_k + sl * 9;
+        const float r = (float)(k[6] / k[7]);
+        for (int step = blockIdx.y * blockDim.x + threadIdx.x; step < steps; step += gridDim.y * blockDim.x) {
+            const double tt = t[step];
+            const float u = (float)fma(-k[7], tt - k[8], c[i]);
+            const float sp = u > 0.f ? u + log1pf(expf(-u)) : log1pf(expf(u));
+            const float R = -expm1f(-r * sp);
+            const float e5 = expf((float)(-k[5] * tt));
+            const double f = k[2] * (double)e5 * (double)R;
+            F[sl * steps + step] = f;
+            Ff[sl * steps + step] = (float)f;
+        }
     }
 }
 
@@ -909,10 +924,12 @@ void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads,
 
 void launch_layer_factors(cudaStream_t s, const HeartDev &h, const double *d_layer_k, const double *d_cpre,
                           int n_sims, double *d_F, float *d_Ff, float *d_layer_c, const double *d_centre,
-                          const double *d_scale, int J, float *d_coef) {
-    const dim3 grid((unsigned)((int64_t)n_sims * h.nlayers), d_cpre ? (unsigned)((h.steps + 127) / 128) : 1u);
-    k_layer_factors<<<grid, 128, 0, s>>>(
-        h.nlayers, h.steps, h.t.p, d_layer_k, d_cpre, n_sims, d_F, d_Ff, d_layer_c, d_centre, d_scale, J, d_coef);
+                          const double *d_scale, int J, float *d_coef, int max_blocks) {
+    const int64_t pairs = (int64_t)n_sims * h.nlayers;
+    const int per = d_cpre ? 1 : (int)std::min<int64_t>(FACTOR_PAIRS, (pairs + max_blocks - 1) / max_blocks);
+    const dim3 grid((unsigned)((pairs + per - 1) / per), d_cpre ? (unsigned)((h.steps + 127) / 128) : 1u);
+    k_layer_factors<<<grid, 128, 0, s>>>(h.nlayers, h.steps, h.t.p, d_layer_k, d_cpre, pairs, per, d_F, d_Ff, d_layer_c,
+                                         d_centre, d_scale, J, d_coef);
     EKG_CUDA(cudaGetLastError());
 }
 

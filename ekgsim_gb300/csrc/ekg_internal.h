@@ -289,8 +289,8 @@ void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads,
 void launch_pass_in(cudaStream_t s, const uint8_t *host, uint8_t *dev, size_t bytes, int *work);
 void launch_pass_out(cudaStream_t s, const double *dev, double *host, size_t n);
 void launch_layer_factors(cudaStream_t s, const HeartDev &h, const double *d_layer_k, const double *d_cpre,
-                          int n_sims, double *d_F, float *d_Ff, float *d_layer_c, const double *d_centre = nullptr,
-                          const double *d_scale = nullptr, int J = 0, float *d_coef = nullptr);
+                          int n_sims, double *d_F, float *d_Ff, float *d_layer_c, const double *d_centre,
+                          const double *d_scale, int J, float *d_coef, int max_blocks);
 // per-simulation form: W and (Wp not null) W' = W exp(k5 at) of the moved rows from the lead
 // positions, and with static_rows W' of the other rows from the resident field W0 (batch.cu)
 void launch_sim_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads, int nmove, int lead_stride,

@@ -1105,8 +1105,8 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     // (measured: other placements of the small kernels, such as the criteria of the static leads
     // beside the GEMM, lengthen the pass).  Without static leads only the layer factors can be hidden, and
     // their blocks, which start first, unbalance an operand grid that is less than one wave (64^3, two
-    // moved leads, us per pass beside each other / in a row: 17 simulations 84 / 91, 32 105 / 102,
-    // 100 186 / 168, 200 272 / 244); a fuller one deals its items as blocks come free (96^3, 12 moved
+    // moved leads, us per pass beside each other / in a row: 9 simulations 73 / 84, 32 92 / 88,
+    // 100 180 / 153, 200 285 / 225); a fuller one deals its items as blocks come free (96^3, 12 moved
     // leads: 40 simulations 381 / 390, 256 1035 / 1097)
     const bool fork = P.batch && nmove > 0 &&
                       (nmove < (int)L || n_sims * D.nlayers <= h->sm_count / 2 ||
@@ -1123,7 +1123,7 @@ void compute(ekg_heart *h, const PassPlan &P, int n_crit_leads, int mode, PassTi
     cudaStream_t sx = fork ? h->aux_stream : s;
     launch_layer_factors(sx, D, in.layer_k, in.cpre, n_sims, E.F.p, E.Ff.p, E.layer_c.p,
                          P.batch ? h->bs.d_centre.p : nullptr, P.batch ? h->bs.d_scale.p : nullptr, P.J,
-                         P.batch ? E.coef.p : nullptr);
+                         P.batch ? E.coef.p : nullptr, h->sm_count);
     ++launches;
     if (P.batch) {
         BatchState &B = h->bs;
