@@ -698,19 +698,27 @@ __device__ __forceinline__ double warp_max(double v) {
 // Block-wide reductions for the criteria (NT threads): a warp butterfly, then lane 0 of each warp
 // in warp order, so every thread gets the same value in a fixed order.  `red` is shared scratch of
 // NT / 32 entries.
-template <int NT>
-__device__ __forceinline__ double block_sum_ff(float2 v, float2 *red) {
+// K sums at once, in place
+template <int NT, int K>
+__device__ __forceinline__ void block_sums_ff(float2 (&v)[K], float2 (*red)[3]) {
     constexpr int CR_WARPS = NT / 32;
-    for (int o = 16; o > 0; o >>= 1) {
-        const float2 w = make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
-        v = ff_add(v, w);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            v[k] = ff_add(v[k], make_float2(__shfl_xor_sync(0xffffffffu, v[k].x, o), __shfl_xor_sync(0xffffffffu, v[k].y, o)));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k) red[threadIdx.x >> 5][k] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        float2 t = red[0][k];
+#pragma unroll
+        for (int w = 1; w < CR_WARPS; ++w) t = ff_add(t, red[w][k]);
+        v[k] = t;
     }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float2 t = red[0];
-    for (int k = 1; k < CR_WARPS; ++k) t = ff_add(t, red[k]);
-    return ff_to_double(t);
 }
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *red) {
@@ -737,11 +745,17 @@ __device__ __forceinline__ double block_minmax(double v, bool is_max, double *re
 __device__ __forceinline__ bool ff_greater(float2 a, float2 b) { return a.x > b.x || (a.x == b.x && a.y > b.y); }
 
 // One block of NT threads per (simulation, criterion lead): threads stride over the steps, sums
-// combined in a fixed order (one warp per pair when there are many pairs, four for few).  Pearson, vector correlation and RMS accumulate in float-float (about
-// 48 significant bits) on the FP32 pipe, reading the float-float copies of the ECG and targets;
-// the few closing operations (means, square roots, quotients) are FP64.  devFromLinear stays FP64
+// combined in a fixed order (one warp per pair when there are many pairs, four for few).  Pearson, vector
+// correlation and RMS accumulate in float-float (about 48 significant bits) on the FP32 pipe, reading the
+// float-float copies of the ECG and targets; the closing operations are FP64.  devFromLinear stays FP64
 // throughout.  Writes the criterion value and the argmax (first maximum) of the lead.
-template <int NT>
+// Bound by the FP64 pipe (an instruction costs it the same for one lane as for 32) and, with few pairs, by
+// latency: the sums of a pass over the steps are reduced together, the number of steps cancels out of the
+// closing quotient, which is one rsqrt, and with few pairs a thread keeps its steps in registers (64^3, one
+// simulation x 2 leads: 6.2 us, now 4.2; 160^3, 256 x 12: 21, now 15.7, where registers or two warps per
+// pair give 19.5).
+constexpr int CRIT_STEPS = 1024;  // steps that a block keeps in registers
+template <int NT, int PER>
 __global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, int i1, int n_sims, int mode,
                                                          const double *__restrict__ ecg,
                                                          const float2 *__restrict__ ecg_ff,
@@ -751,6 +765,7 @@ __global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, 
                                                          const double *__restrict__ toff, int crit_stride,
                                                          double *__restrict__ crit) {
     constexpr int CR_THREADS = NT, CR_WARPS = NT / 32;
+    __shared__ float2 reds[CR_WARPS][3];
     __shared__ float2 redf[CR_WARPS];
     __shared__ double redd[CR_WARPS];
     __shared__ int redi[CR_WARPS];
@@ -759,50 +774,69 @@ __global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, 
     const int i = i0 + (int)(blockIdx.x % ni), s = (int)(blockIdx.x / ni);
     const size_t row = ((size_t)s * nleads + i) * steps;
     const float2 *af = ecg_ff + row;
+    float2 xs[PER ? PER : 1], ys[PER ? PER : 1];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) xs[q] = tid + q * NT < steps ? af[tid + q * NT] : make_float2(0.f, 0.f);
     int64_t off = 0;
     for (int j = 0; j < i; ++j) off += tlen[j];
     const float2 *bf = targets_ff + off;
     const int64_t nb = tlen[i];
     const int64_t len = steps < nb ? steps : nb;
-    const double inv = 1.0 / (double)len;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) ys[q] = tid + q * NT < len ? bf[tid + q * NT] : make_float2(0.f, 0.f);
+    // f(x, y) of the thread's steps below len, in order
+    auto each = [&](auto f) {
+        if constexpr (PER > 0) {
+#pragma unroll
+            for (int q = 0; q < PER; ++q)
+                if (tid + q * NT < len) f(xs[q], ys[q]);
+        } else {
+            for (int64_t j = tid; j < len; j += NT) f(af[j], bf[j]);
+        }
+    };
+    const float2 zero = make_float2(0.f, 0.f);
     double value = 0.0;
     if (mode == 2) {
-        float2 sa = make_float2(0.f, 0.f), sb = sa;
-        for (int64_t j = tid; j < len; j += CR_THREADS) {
-            sa = ff_add(sa, af[j]);
-            sb = ff_add(sb, bf[j]);
-        }
-        const float2 ma = ff_neg(ff_from_double(block_sum_ff<NT>(sa, redf) * inv));
-        const float2 mb = ff_neg(ff_from_double(block_sum_ff<NT>(sb, redf) * inv));
-        float2 va = make_float2(0.f, 0.f), vb = va, cv = va;
-        for (int64_t j = tid; j < len; j += CR_THREADS) {
-            const float2 x = ff_add(af[j], ma), y = ff_add(bf[j], mb);
-            va = ff_add(va, ff_mul(x, x));
-            vb = ff_add(vb, ff_mul(y, y));
-            cv = ff_add(cv, ff_mul(x, y));
-        }
-        const double dva = block_sum_ff<NT>(va, redf) * inv, dvb = block_sum_ff<NT>(vb, redf) * inv;
-        const double dcv = block_sum_ff<NT>(cv, redf) / (double)len;
-        value = 1.0 - dcv / (sqrt(dva) * sqrt(dvb));
+        // 1 - cov / (sigma_a sigma_b); the number of steps cancels, and an error of a mean enters the sums
+        // with its square
+        float2 m[2] = {zero, zero};
+        each([&](float2 x, float2 y) {
+            m[0] = ff_add(m[0], x);
+            m[1] = ff_add(m[1], y);
+        });
+        block_sums_ff<NT>(m, reds);
+        const float n = (float)len, rn = 1.0f / n;
+        const float2 ninv = make_float2(-rn, -rn * fmaf(-rn, n, 1.0f));
+        const float2 ma = ff_mul(m[0], ninv), mb = ff_mul(m[1], ninv);
+        float2 v[3] = {zero, zero, zero};
+        each([&](float2 xx, float2 yy) {
+            const float2 x = ff_add(xx, ma), y = ff_add(yy, mb);
+            v[0] = ff_add(v[0], ff_mul(x, x));
+            v[1] = ff_add(v[1], ff_mul(y, y));
+            v[2] = ff_add(v[2], ff_mul(x, y));
+        });
+        block_sums_ff<NT>(v, reds);
+        if (tid < 32) value = 1.0 - ff_to_double(v[2]) * rsqrt(ff_to_double(v[0]) * ff_to_double(v[1]));
     } else if (mode == 4) {
-        float2 ab = make_float2(0.f, 0.f), aa = ab, bb = ab;
-        for (int64_t j = tid; j < len; j += CR_THREADS) {
-            const float2 x = af[j], y = bf[j];
-            ab = ff_add(ab, ff_mul(x, y));
-            aa = ff_add(aa, ff_mul(x, x));
-            bb = ff_add(bb, ff_mul(y, y));
-        }
-        const double dab = block_sum_ff<NT>(ab, redf), daa = block_sum_ff<NT>(aa, redf), dbb = block_sum_ff<NT>(bb, redf);
-        value = 1.0 - dab / (sqrt(daa) * sqrt(dbb));
+        float2 v[3] = {zero, zero, zero};
+        each([&](float2 x, float2 y) {
+            v[0] = ff_add(v[0], ff_mul(x, x));
+            v[1] = ff_add(v[1], ff_mul(y, y));
+            v[2] = ff_add(v[2], ff_mul(x, y));
+        });
+        block_sums_ff<NT>(v, reds);
+        if (tid < 32) value = 1.0 - ff_to_double(v[2]) * rsqrt(ff_to_double(v[0]) * ff_to_double(v[1]));
     } else if (mode == 1) {
-        float2 q = make_float2(0.f, 0.f);
-        for (int64_t j = tid; j < len; j += CR_THREADS) {
-            const float2 x = ff_add(af[j], ff_neg(bf[j]));
-            q = ff_add(q, ff_mul(x, x));
-        }
-        value = sqrt(block_sum_ff<NT>(q, redf) / (double)len);
+        float2 v[1] = {zero};
+        each([&](float2 xx, float2 yy) {
+            const float2 x = ff_add(xx, ff_neg(yy));
+            v[0] = ff_add(v[0], ff_mul(x, x));
+        });
+        block_sums_ff<NT>(v, reds);
+        if (tid < 32) value = sqrt(ff_to_double(v[0]) / (double)len);
     } else {
         // devFromLinear (vectorMath.h:373-404): min/max over the whole simulated lead
+        const double inv = 1.0 / (double)len;
         const double *a = ecg + row;
         const double *b = targets + off;
         double mn = INFINITY, mx = -INFINITY;
@@ -829,13 +863,20 @@ __global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, 
     // values are normalised, so comparing (hi, lo) in order compares the values
     float2 best = make_float2(-INFINITY, 0.f);
     int arg = 0x7fffffff;
-    for (int j = tid; j < steps; j += CR_THREADS) {
-        const float2 v = af[j];
+    auto peak = [&](float2 v, int j) {
         if (ff_greater(v, best)) {
             best = v;
             arg = j;
         }
+    };
+    if constexpr (PER > 0) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            if (tid + q * NT < steps) peak(xs[q], tid + q * NT);
+    } else {
+        for (int j = tid; j < steps; j += CR_THREADS) peak(af[j], j);
     }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float2 v2 = make_float2(__shfl_xor_sync(0xffffffffu, best.x, o), __shfl_xor_sync(0xffffffffu, best.y, o));
         const int a2 = __shfl_xor_sync(0xffffffffu, arg, o);
@@ -1000,14 +1041,14 @@ void launch_criteria(cudaStream_t s, const HeartDev &h, const double *d_ecg, con
                      int ncrit_stride, int i0, int i1, int mode, const double *d_targets, const float2 *d_targets_ff,
                      const int64_t *d_tlen, const double *d_toff, double *d_crit) {
     if (i1 <= i0) return;
-    // one block per (simulation, lead): a warp when the pairs fill the GPU, four warps when few
     const int64_t pairs = (int64_t)(i1 - i0) * n_sims;
-    if (pairs >= 1024)
-        k_criteria<32><<<(unsigned)pairs, 32, 0, s>>>(h.steps, h.nleads, i0, i1, n_sims, mode, d_ecg, d_ecg_ff,
-                                                      d_targets, d_targets_ff, d_tlen, d_toff, ncrit_stride, d_crit);
-    else
-        k_criteria<128><<<(unsigned)pairs, 128, 0, s>>>(h.steps, h.nleads, i0, i1, n_sims, mode, d_ecg, d_ecg_ff,
-                                                        d_targets, d_targets_ff, d_tlen, d_toff, ncrit_stride, d_crit);
+    auto go = [&](auto kern, int nt) {
+        kern<<<(unsigned)pairs, nt, 0, s>>>(h.steps, h.nleads, i0, i1, n_sims, mode, d_ecg, d_ecg_ff, d_targets,
+                                            d_targets_ff, d_tlen, d_toff, ncrit_stride, d_crit);
+    };
+    if (pairs >= 1024) go(k_criteria<32, 0>, 32);
+    else if (h.steps <= CRIT_STEPS) go(k_criteria<128, CRIT_STEPS / 128>, 128);
+    else go(k_criteria<128, 0>, 128);
     EKG_CUDA(cudaGetLastError());
 }
 
