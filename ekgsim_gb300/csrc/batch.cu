@@ -608,8 +608,8 @@ __global__ void __launch_bounds__(LF_THREADS, LF_BLOCKS) k_batch_lead_field(
 // bytes each.  The steady sums of a stage are reduced by a shuffle butterfly within its warp.
 // Same outputs as k_batch_lead_field.
 // The field is evaluated with a thread per voxel of the block's range, read in order, into shared
-// memory, as the two factors of its last product (1 and the value where there is none), and each
-// AP's thread then adds its voxels' products in order: a thread walking its own AP's voxels waits for
+// memory, and each AP's thread then adds its voxels' in order (the second lead of a pair as the two factors
+// of its last product, 1 and the value where there is none, added with one rounding): a thread walking its own AP's voxels waits for
 // their loads one behind the other while its warp diverges over voxel kinds and counts.  Moved-lead
 // operand, one simulation with 2 leads: 128^3 heart 23.4 -> 14.5 us, 64^3 17.9 -> 9.9; 160^3, 4 simulations with
 // 3 leads 79.5 -> 54; 26-cell neighbourhood, 128^3, 2 with 5 leads 210 -> 106.
@@ -665,24 +665,26 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
                 const float4 pos = vox_pos[v];
                 const uint32_t mi = __float_as_uint(pos.w);
                 const MSquares q0 = msq_rn(pos, r0), q1 = msq_rn(pos, r1);
-                float2 f0, f1 = make_float2(0.f, 0.f);
+                float w0;
+                float2 f1 = make_float2(0.f, 0.f);
                 if ((mi & VOX_INTERIOR) && q0.s >= INTERIOR_S_MIN && q1.s >= INTERIOR_S_MIN) {
-                    f0 = interior_f(ic, q0, rsqa(q0.s));
+                    const float2 f0 = interior_f(ic, q0, rsqa(q0.s));
+                    w0 = __fmul_rn(f0.x, f0.y);
                     if (np == 2) f1 = interior_f(ic, q1, rsqa(q1.s));
                 } else {
                     const float4 out = vox_out[v];
-                    f0 = make_float2(1.f, DIAG ? voxel_w_diag(pos, mi, out, r0) : voxel_w_general(pos, mi, out, r0, nnb, s_d));
+                    w0 = DIAG ? voxel_w_diag(pos, mi, out, r0) : voxel_w_general(pos, mi, out, r0, nnb, s_d);
                     if (np == 2)
                         f1 = make_float2(1.f, DIAG ? voxel_w_diag(pos, mi, out, r1) : voxel_w_general(pos, mi, out, r1, nnb, s_d));
                 }
-                s_f[v - c] = make_float4(f0.x, f0.y, f1.x, f1.y);
+                s_f[v - c] = make_float4(w0, f1.x, f1.y, 0.f);
             }
             __syncthreads();
             if (valid)
                 for (int v = max(vb, c); v < min(ve, ce); ++v) {
                     const float4 f = s_f[v - c];
-                    acc0 = __fmaf_rn(f.x, f.y, acc0);
-                    acc1 = __fmaf_rn(f.z, f.w, acc1);
+                    acc0 = __fadd_rn(acc0, f.x);
+                    acc1 = __fmaf_rn(f.y, f.z, acc1);
                 }
         }
         if (P2 && valid) {
