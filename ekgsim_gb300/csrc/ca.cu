@@ -16,7 +16,7 @@
 // hold later ones form the next round's list (k_ca_round).  The host queues rounds in chunks and reads
 // the lists' length once per chunk.
 //
-// GB300, 12 leads aside (relaxation alone, CUDA events): 24^3 0.13 ms, 64^3 0.34, 128^3 0.77, 160^3 1.02
+// GB300 (relaxation alone, CUDA events): 24^3 0.13 ms, 64^3 0.34, 128^3 0.77, 160^3 1.02
 // (49 rounds), 192^3 1.32, 256^3 2.45.  One launch per time bucket over queues in global memory took
 // 0.24, 0.57, 1.40, 1.96, 3.04 and 5.64 ms (9 us a bucket, every access of its chain a trip to L2); rounds
 // of block-wide sweeps to local convergence, without a horizon, 3.4 ms at 160^3 in the calls that
@@ -294,6 +294,10 @@ static double round_window(const double *lag, int nl1, const char *present) {
 
 // Queues rounds in chunks until a round has no tile; the host reads the counts once per chunk (rounds
 // after convergence find an empty list).  `read` copies the four counters to the host, waiting.
+// A chunk's end costs some 22 us (the copy, the wait, the next launch without its predecessor to overlap), a
+// round too many 2.5: the first chunk is as long as hearts of 24 to 256 cells were seen to need, 2.2 to 3.5
+// rounds per tile of the longest side, later ones are short (160^3, 49 rounds: five chunks of 12 1.02 ms,
+// one of 50 0.95).
 template <typename LT, class Read>
 static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, const double *lag, int nl1, double w,
                       u64 *at, const TileLists &T, int cap, int sm_count, Read read) {
@@ -308,12 +312,14 @@ static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, 
     cfg.attrs = &pdl;
     cfg.numAttrs = 1;
     constexpr int CHUNK = 12;
+    int chunk = std::max(CHUNK, 5 * std::max({ntz, nty, ntx}) / 2);
     int32_t h[4];
     for (int r = 0;;) {
-        const int end = std::min(cap, r + CHUNK);
+        const int end = (int)std::min<int64_t>(cap, (int64_t)r + chunk);
         for (; r < end; ++r) {
             EKG_CUDA(cudaLaunchKernelEx(&cfg, k_ca_round<LT>, r, nz, ny, nx, ntz, nty, ntx, layers, lag, nl1, w, at, T));
         }
+        chunk = CHUNK;
         read(h);
         if (h[r % 3] == 0) return h[3];
         if (r >= cap) throw Error{EKG_ERR_CA_NOT_CONVERGED, "activation-time relaxation did not converge"};
