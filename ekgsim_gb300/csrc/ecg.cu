@@ -46,30 +46,38 @@ __device__ __forceinline__ float h_value(float tau, float4 c) {
 }
 
 // ------------------------------------------------------------------ lead field
-// Block per (128 APs, lead l, sim s).  Lead positions FP64 [S][lead_stride][3] (z,y,x); W
-// [S][w_lead_stride][apad].  The block's voxels, read in order, get a thread each, and each AP's thread
-// adds its voxels' values in order in FP64: a thread walking its AP's voxels waits for their loads one
-// behind the other while its warp diverges over voxel counts (160^3 heart, 12 leads, set-up and first
-// simulation with the chunk reduction below: 4.45 -> 3.8 ms).
-constexpr int LFW_CAP = 1024;  // voxels evaluated at a time
+// Block per (128 APs, LFW_LEADS leads, sim s).  Lead positions FP64 [S][lead_stride][3] (z,y,x); W
+// [S][w_lead_stride][apad].  The block's voxels, read in order, get a thread each, which takes the leads
+// together (a neighbour's position is formed once), and each AP's thread then adds its voxels' values in
+// order, as the sum and its rounding errors (two FP32 words, the same W as an FP64 sum gives): a thread
+// walking its AP's voxels waits for their loads one behind the other while its warp diverges over voxel
+// counts, and the FP64 pipe takes 32 clocks for a conversion and an addition of a warp in which most lanes
+// have no voxel left (160^3 heart, 12 leads: 238 us in FP64, a lead or four per block; 131 now).
+constexpr int LFW_CAP = 512, LFW_LEADS = 4;  // voxels evaluated at a time, leads per block
 __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t *__restrict__ a_vox_begin,
                              const int32_t *__restrict__ vox_zyx, const uint32_t *__restrict__ nb_in,
                              const uint32_t *__restrict__ nb_out, int nnb, const int8_t *__restrict__ difs,
                              const double *__restrict__ leads, int nleads, int lead_stride,
                              float *__restrict__ W, int w_lead_stride) {
-    __shared__ int8_t s_dif[26 * 3];
-    __shared__ float s_w[LFW_CAP];
+    __shared__ float4 s_dif[26];
+    __shared__ float s_w[LFW_LEADS][LFW_CAP];
     const int tid = threadIdx.x;
-    if (tid < nnb * 3) s_dif[tid] = difs[tid];
+    if (tid < nnb) s_dif[tid] = make_float4(difs[3 * tid], difs[3 * tid + 1], difs[3 * tid + 2], 0.f);
     const int64_t a0 = blockIdx.x * (int64_t)128, a = a0 + tid;
-    const int l = blockIdx.y, s = blockIdx.z;
+    const int l0 = blockIdx.y * LFW_LEADS, nl = min(LFW_LEADS, nleads - l0), s = blockIdx.z;
     const bool on = a < apad;
-    const double *r = leads + ((size_t)s * lead_stride + l) * 3;
-    const float rz = (float)r[0], ry = (float)r[1], rx = (float)r[2];
-    const float rzl = (float)(r[0] - (double)rz), ryl = (float)(r[1] - (double)ry), rxl = (float)(r[2] - (double)rx);
+    float rz[LFW_LEADS], ry[LFW_LEADS], rx[LFW_LEADS], rzl[LFW_LEADS], ryl[LFW_LEADS], rxl[LFW_LEADS];
+#pragma unroll
+    for (int k = 0; k < LFW_LEADS; ++k) {
+        const double *r = leads + ((size_t)s * lead_stride + l0 + min(k, nl - 1)) * 3;
+        rz[k] = (float)r[0], ry[k] = (float)r[1], rx[k] = (float)r[2];
+        rzl[k] = (float)(r[0] - (double)rz[k]), ryl[k] = (float)(r[1] - (double)ry[k]), rxl[k] = (float)(r[2] - (double)rx[k]);
+    }
     const int v0 = (int)a_vox_begin[a0], v1 = (int)a_vox_begin[a0 + 128 < apad ? a0 + 128 : apad];
     const int vb = on ? (int)a_vox_begin[a] : v1, ve = on ? (int)a_vox_begin[a + 1] : v1;
-    double acc = 0.0;
+    float2 acc[LFW_LEADS];  // (sum, its rounding errors)
+#pragma unroll
+    for (int k = 0; k < LFW_LEADS; ++k) acc[k] = make_float2(0.f, 0.f);
     for (int c = v0; c < v1; c += LFW_CAP) {
         const int ce = min(c + LFW_CAP, v1);
         __syncthreads();
@@ -78,36 +86,58 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
             // bordered coordinates (simlib/simulator.cpp:458-463, 487)
             const float pz = (float)((p >> 20) + 1), py = (float)(((p >> 10) & 1023) + 1), px = (float)((p & 1023) + 1);
             const uint32_t mi = nb_in[v], mo = nb_out[v];
-            float w = 0.f;
-            float sz = 0.f, sy = 0.f, sx = 0.f;
+            float w[LFW_LEADS];
+#pragma unroll
+            for (int k = 0; k < LFW_LEADS; ++k) w[k] = 0.f;
             for (int n = 0; n < nnb; ++n) {
-                const float dz = s_dif[3 * n], dy = s_dif[3 * n + 1], dx = s_dif[3 * n + 2];
-                if (mi & (1u << n)) {
-                    const float mz = (rz - (pz + dz)) + rzl, my = (ry - (py + dy)) + ryl, mx = (rx - (px + dx)) + rxl;
-                    const float ss = fmaf(mz, mz, fmaf(my, my, mx * mx));
-                    const float rs = rsqrtf(ss);
-                    const float f = rs * rs * rs;
-                    w = fmaf(f, fmaf(mz, dz, fmaf(my, dy, mx * dx)), w);
-                }
-                if (mo & (1u << n)) {
-                    sz += dz;
-                    sy += dy;
-                    sx += dx;
-                }
+                if (!(mi & (1u << n))) continue;
+                const float4 d = s_dif[n];
+                const float qz = pz + d.x, qy = py + d.y, qx = px + d.z;
+#pragma unroll
+                for (int k = 0; k < LFW_LEADS; ++k)
+                    if (k < nl) {
+                        const float mz = (rz[k] - qz) + rzl[k], my = (ry[k] - qy) + ryl[k], mx = (rx[k] - qx) + rxl[k];
+                        const float ss = fmaf(mz, mz, fmaf(my, my, mx * mx));
+                        const float rs = rsqrtf(ss);
+                        const float f = rs * rs * rs;
+                        w[k] = fmaf(f, fmaf(mz, d.x, fmaf(my, d.y, mx * d.z)), w[k]);
+                    }
             }
             if (mo) {
-                const float mz = (rz - pz) + rzl, my = (ry - py) + ryl, mx = (rx - px) + rxl;
-                const float ss = fmaf(mz, mz, fmaf(my, my, mx * mx));
-                const float rs = rsqrtf(ss);
-                const float f = rs * rs * rs;
-                w = fmaf(-f, fmaf(mz, sz, fmaf(my, sy, mx * sx)), w);
+                float sz = 0.f, sy = 0.f, sx = 0.f;
+                for (int n = 0; n < nnb; ++n)
+                    if (mo & (1u << n)) {
+                        const float4 d = s_dif[n];
+                        sz += d.x;
+                        sy += d.y;
+                        sx += d.z;
+                    }
+#pragma unroll
+                for (int k = 0; k < LFW_LEADS; ++k)
+                    if (k < nl) {
+                        const float mz = (rz[k] - pz) + rzl[k], my = (ry[k] - py) + ryl[k], mx = (rx[k] - px) + rxl[k];
+                        const float ss = fmaf(mz, mz, fmaf(my, my, mx * mx));
+                        const float rs = rsqrtf(ss);
+                        const float f = rs * rs * rs;
+                        w[k] = fmaf(-f, fmaf(mz, sz, fmaf(my, sy, mx * sx)), w[k]);
+                    }
             }
-            s_w[v - c] = w;
+#pragma unroll
+            for (int k = 0; k < LFW_LEADS; ++k) s_w[k][v - c] = w[k];
         }
         __syncthreads();
-        for (int v = max(vb, c); v < min(ve, ce); ++v) acc += (double)s_w[v - c];
+        for (int v = max(vb, c); v < min(ve, ce); ++v)
+#pragma unroll
+            for (int k = 0; k < LFW_LEADS; ++k)
+                if (k < nl) {
+                    const float2 t = ff_two_sum(acc[k].x, s_w[k][v - c]);
+                    acc[k] = make_float2(t.x, acc[k].y + t.y);
+                }
     }
-    if (on) W[((size_t)s * w_lead_stride + l) * apad + a] = (float)acc;
+    if (on)
+#pragma unroll
+        for (int k = 0; k < LFW_LEADS; ++k)
+            if (k < nl) W[((size_t)s * w_lead_stride + l0 + k) * apad + a] = acc[k].x + acc[k].y;
 }
 
 // ------------------------------------------------------------------ per-layer factors
@@ -957,7 +987,7 @@ void launch_pass_out(cudaStream_t s, const double *dev, double *host, size_t n) 
 }
 void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads, int nleads_in, int lead_stride,
                        int n_sims, float *d_W, int w_lead_stride) {
-    dim3 grid((unsigned)((h.apad + 127) / 128), (unsigned)nleads_in, (unsigned)n_sims);
+    dim3 grid((unsigned)((h.apad + 127) / 128), (unsigned)((nleads_in + LFW_LEADS - 1) / LFW_LEADS), (unsigned)n_sims);
     k_lead_field<<<grid, 128, 0, s>>>(h.apad, h.a_vox_begin.p, h.vox_zyx.p, h.vox_nb.p, h.vox_nbo.p, h.nnb,
                                       h.difs.p, d_leads, nleads_in, lead_stride, d_W, w_lead_stride);
     EKG_CUDA(cudaGetLastError());
