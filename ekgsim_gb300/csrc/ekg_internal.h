@@ -231,7 +231,7 @@ struct DedupResult {
     // the sort's other buffers, free for the stage order
     uint64_t *key2 = nullptr;
     uint8_t *vl2 = nullptr;
-    int *cell2 = nullptr, *hist = nullptr, *totals = nullptr, *base = nullptr, *tsum = nullptr;
+    int *cell2 = nullptr, *hist = nullptr, *totals = nullptr, *tsum = nullptr;
     unsigned long long *n_interior = nullptr;
 };
 size_t setup_scratch_bytes(int64_t n_cells, int64_t nvox);

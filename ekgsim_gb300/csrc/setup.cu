@@ -113,27 +113,48 @@ __global__ void __launch_bounds__(ST) k_compact(F f, int64_t n, const int *__res
 }
 
 // ---- stable LSD radix sort of (layer, time bits) with the cell as payload, 8-bit digits
-// pass p < 8: byte p of the time bits; pass 8: the layer.  One element per thread, tiles of ST.
+// pass p < 8: byte p of the time bits; pass 8: the layer.  Tiles of RTILE elements.  A pass is bound by its
+// three launches and their chains, not by the 26 bytes an element that it moves (160^3, 661,216 voxels:
+// 30 us a pass with a tile per 256 elements and a launch for the digits' bases; 21.5, and 18.5 with a pass's
+// kernels launched ahead).
+constexpr int RITEMS = 4, RTILE = ST * RITEMS;
 __device__ __forceinline__ int digit(int pass, uint64_t key, uint8_t lay) {
     return pass < 8 ? (int)((key >> (8 * pass)) & 0xffu) : (int)lay;
 }
 
-__global__ void __launch_bounds__(ST) k_digit_hist(int pass, int n, const uint64_t *__restrict__ key,
-                                                   const uint8_t *__restrict__ lay, int nblk, int *__restrict__ hist) {
+// The kernels of a pass are launched while their predecessor runs: each lets its successor's blocks take
+// the places that it leaves and waits for its own predecessor's results before its first access (none of
+// their pointers is __restrict__: a load of data that is declared constant may be moved before the wait).
+__device__ __forceinline__ void pass_begin() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(ST) k_digit_hist(int pass, int n, const uint64_t *key,
+                                                   const uint8_t *lay, int nblk, int *hist) {
     __shared__ int s_h[256];
     s_h[threadIdx.x] = 0;
+    pass_begin();
+    int d[RITEMS];
+#pragma unroll
+    for (int k = 0; k < RITEMS; ++k) {
+        const int i = blockIdx.x * RTILE + k * ST + threadIdx.x;
+        d[k] = i < n ? digit(pass, pass < 8 ? key[i] : 0, pass < 8 ? (uint8_t)0 : lay[i]) : -1;
+    }
     __syncthreads();
-    const int i = blockIdx.x * ST + threadIdx.x;
-    if (i < n) atomicAdd(&s_h[digit(pass, key[i], lay[i])], 1);
+#pragma unroll
+    for (int k = 0; k < RITEMS; ++k)
+        if (d[k] >= 0) atomicAdd(&s_h[d[k]], 1);
     __syncthreads();
     hist[(size_t)threadIdx.x * nblk + blockIdx.x] = s_h[threadIdx.x];
 }
 
 // per digit (block): exclusive scan of its counts over the tiles; totals[d] = the digit's count
-__global__ void __launch_bounds__(ST) k_digit_scan(int *__restrict__ hist, int nblk, int *__restrict__ totals) {
+__global__ void __launch_bounds__(ST) k_digit_scan(int *hist, int nblk, int *totals) {
     __shared__ int s_warp[ST / 32];
     int *h = hist + (size_t)blockIdx.x * nblk;
     int carry = 0;
+    pass_begin();
     for (int b = 0; b < nblk; b += ST) {
         const int i = b + (int)threadIdx.x;
         const int v = i < nblk ? h[i] : 0;
@@ -145,46 +166,62 @@ __global__ void __launch_bounds__(ST) k_digit_scan(int *__restrict__ hist, int n
     if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
-__global__ void __launch_bounds__(ST) k_digit_base(const int *__restrict__ totals, int *__restrict__ base) {
-    __shared__ int s_warp[ST / 32];
-    int total;
-    base[threadIdx.x] = block_exscan(totals[threadIdx.x], &total, s_warp);
-}
-
-// rank = digit base + the tile's offset for the digit + equal digits before it in the tile (earlier
-// warps' counts from shared memory, earlier lanes of the warp from a match mask): stable
-__global__ void __launch_bounds__(ST) k_digit_scatter(int pass, int n, const uint64_t *__restrict__ key_in,
-                                                      const uint8_t *__restrict__ lay_in, const int *__restrict__ val_in,
-                                                      int nblk, const int *__restrict__ hist,
-                                                      const int *__restrict__ base, uint64_t *__restrict__ key_out,
-                                                      uint8_t *__restrict__ lay_out, int *__restrict__ val_out) {
+// rank = the digit's base (every block scans the 256 totals) + the tile's offset for the digit + equal
+// digits before it in the tile: a warp takes 32 RITEMS consecutive elements, 32 at a time, with its
+// running counts in shared memory and a match mask for the lanes before; then the earlier warps' counts.
+__global__ void __launch_bounds__(ST) k_digit_scatter(int pass, int n, const uint64_t *key_in,
+                                                      const uint8_t *lay_in, const int *val_in,
+                                                      int nblk, const int *hist,
+                                                      const int *totals, uint64_t *key_out,
+                                                      uint8_t *lay_out, int *val_out) {
     __shared__ int s_cnt[ST / 32][256];
+    __shared__ int s_warp[ST / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i0 = blockIdx.x * RTILE + w * (32 * RITEMS) + lane;
+    pass_begin();
+    uint64_t kv[RITEMS];
+    uint8_t lv[RITEMS];
+    int vv[RITEMS], rank[RITEMS], dg[RITEMS];
+#pragma unroll
+    for (int k = 0; k < RITEMS; ++k) {
+        const int i = i0 + 32 * k;
+        kv[k] = i < n ? key_in[i] : 0;
+        lv[k] = i < n ? lay_in[i] : (uint8_t)0;
+        vv[k] = i < n ? val_in[i] : 0;
+    }
+    const int off = hist[(size_t)threadIdx.x * nblk + blockIdx.x];
+    int all;
+    const int base = block_exscan(totals[threadIdx.x], &all, s_warp);
     for (int k = threadIdx.x; k < (ST / 32) * 256; k += ST) (&s_cnt[0][0])[k] = 0;
     __syncthreads();
-    const int i = blockIdx.x * ST + threadIdx.x;
-    const bool valid = i < n;
-    uint64_t kv = 0;
-    uint8_t lv = 0;
-    int vv = 0;
-    if (valid) {
-        kv = key_in[i];
-        lv = lay_in[i];
-        vv = val_in[i];
+#pragma unroll
+    for (int k = 0; k < RITEMS; ++k) {
+        const bool valid = i0 + 32 * k < n;
+        dg[k] = valid ? digit(pass, kv[k], lv[k]) : 256 + lane;  // invalid lanes match nothing
+        const unsigned m = __match_any_sync(FULL, dg[k]);
+        const int before = valid ? s_cnt[w][dg[k]] : 0, in = __popc(m & ((1u << lane) - 1u));
+        rank[k] = before + in;
+        __syncwarp();
+        if (valid && in == 0) s_cnt[w][dg[k]] = before + __popc(m);
+        __syncwarp();
     }
-    const int d = valid ? digit(pass, kv, lv) : 256 + lane;  // invalid lanes match nothing
-    const unsigned m = __match_any_sync(FULL, d);
-    const int rank_w = __popc(m & ((1u << lane) - 1u));
-    if (valid && rank_w == 0) s_cnt[w][d] = __popc(m);
     __syncthreads();
-    if (valid) {
-        int off = 0;
-        for (int k = 0; k < w; ++k) off += s_cnt[k][d];
-        const int pos = base[d] + hist[(size_t)d * nblk + blockIdx.x] + off + rank_w;
-        key_out[pos] = kv;
-        lay_out[pos] = lv;
-        val_out[pos] = vv;
+    int run = base + off;  // thread = digit
+#pragma unroll
+    for (int k = 0; k < ST / 32; ++k) {
+        const int c = s_cnt[k][threadIdx.x];
+        s_cnt[k][threadIdx.x] = run;
+        run += c;
     }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < RITEMS; ++k)
+        if (i0 + 32 * k < n) {
+            const int pos = s_cnt[w][dg[k]] + rank[k];
+            key_out[pos] = kv[k];
+            lay_out[pos] = lv[k];
+            val_out[pos] = vv[k];
+        }
 }
 
 __global__ void k_gather_keys(int nv, const int *__restrict__ cell, const double *__restrict__ at,
@@ -313,14 +350,25 @@ __global__ void k_voxel_records(int nv, VoxelGeom g, const int *__restrict__ cel
 // Sorts n (key, layer, payload) triples by the digit passes listed; the pointers are left at the sorted
 // buffers (first) and the other ones.
 static void sort_passes(cudaStream_t s, int n, int first, int passes, uint64_t *&key, uint64_t *&key2, uint8_t *&lay,
-                        uint8_t *&lay2, int *&val, int *&val2, int *hist, int *totals, int *base) {
-    const int nblk = (n + ST - 1) / ST;
+                        uint8_t *&lay2, int *&val, int *&val2, int *hist, int *totals) {
+    const int nblk = (n + RTILE - 1) / RTILE;
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(ST);
+    cfg.stream = s;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = 1;
+    auto go = [&](auto kern, int blocks, auto... args) {
+        cfg.gridDim = dim3((unsigned)blocks);
+        EKG_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+    };
     for (int pass = first; pass < first + passes; ++pass) {
-        k_digit_hist<<<nblk, ST, 0, s>>>(pass, n, key, lay, nblk, hist);
-        k_digit_scan<<<256, ST, 0, s>>>(hist, nblk, totals);
-        k_digit_base<<<1, ST, 0, s>>>(totals, base);
-        k_digit_scatter<<<nblk, ST, 0, s>>>(pass, n, key, lay, val, nblk, hist, base, key2, lay2, val2);
-        EKG_CUDA(cudaGetLastError());
+        go(k_digit_hist, nblk, pass, n, (const uint64_t *)key, (const uint8_t *)lay, nblk, hist);
+        go(k_digit_scan, 256, hist, nblk, totals);
+        go(k_digit_scatter, nblk, pass, n, (const uint64_t *)key, (const uint8_t *)lay, (const int *)val, nblk,
+           (const int *)hist, (const int *)totals, key2, lay2, val2);
         std::swap(key, key2);
         std::swap(lay, lay2);
         std::swap(val, val2);
@@ -333,7 +381,7 @@ static size_t sort_capacity(int64_t nvox) { return (size_t)std::max<int64_t>(nvo
 size_t setup_scratch_bytes(int64_t n_cells, int64_t nvox) {
     const size_t m = sort_capacity(nvox), tiles = (size_t)(n_cells + STILE - 1) / STILE + 1;
     return 2 * (Arena::part(m * 8) + Arena::part(m) + Arena::part(m * 4)) + Arena::part((m + 1) * 4) +
-           Arena::part((m + ST - 1) / ST * 256 * 4) + 2 * Arena::part(256 * 4) + Arena::part(tiles * 4) +
+           Arena::part((m + RTILE - 1) / RTILE * 256 * 4) + Arena::part(256 * 4) + Arena::part(tiles * 4) +
            Arena::part(257 * 4) + Arena::part(8);
 }
 
@@ -349,9 +397,8 @@ void setup_voxels_device(cudaStream_t s, int nz, int ny, int nx, const uint8_t *
     r.cell = scratch.take<int>(m);
     r.cell2 = scratch.take<int>(m);
     r.gstart = scratch.take<int>(m + 1);
-    r.hist = scratch.take<int>((m + ST - 1) / ST * 256);
+    r.hist = scratch.take<int>((m + RTILE - 1) / RTILE * 256);
     r.totals = scratch.take<int>(256);
-    r.base = scratch.take<int>(256);
     r.tsum = scratch.take<int>((size_t)(n + STILE - 1) / STILE + 1);
     int *info = scratch.take<int>(257);
     r.n_interior = scratch.take<unsigned long long>(1);
@@ -364,7 +411,7 @@ void setup_voxels_device(cudaStream_t s, int nz, int ny, int nx, const uint8_t *
     // 2. stable radix sort by (layer, time bits); payload = cell
     k_gather_keys<<<(nv + 255) / 256, 256, 0, s>>>(nv, r.cell, d_at_cells, d_lay, r.key, r.vl);
     EKG_CUDA(cudaGetLastError());
-    sort_passes(s, nv, 0, 9, r.key, r.key2, r.vl, r.vl2, r.cell, r.cell2, r.hist, r.totals, r.base);
+    sort_passes(s, nv, 0, 9, r.key, r.key2, r.vl, r.vl2, r.cell, r.cell2, r.hist, r.totals);
     // 3. runs of equal (layer, time): the APs
     const int nt2 = (nv + STILE - 1) / STILE;
     k_tile_counts<<<nt2, ST, 0, s>>>(StartsRun{r.vl, r.key}, nv, r.tsum);
@@ -456,7 +503,7 @@ void setup_stage_order_device(cudaStream_t s, DedupResult &r, const int64_t *a_v
     const uint32_t top = digits == 4 ? 0xffffffffu : (1u << (8 * digits)) - 1u;
     k_stage_keys<<<(nst + 255) / 256, 256, 0, s>>>(nst, top, a_vox_begin, r.key, r.cell);
     EKG_CUDA(cudaGetLastError());
-    sort_passes(s, nst, 0, digits, r.key, r.key2, r.vl, r.vl2, r.cell, r.cell2, r.hist, r.totals, r.base);
+    sort_passes(s, nst, 0, digits, r.key, r.key2, r.vl, r.vl2, r.cell, r.cell2, r.hist, r.totals);
     EKG_CUDA(cudaMemcpyAsync(stage_order, r.cell, (size_t)nst * 4, cudaMemcpyDeviceToDevice, s));
 }
 

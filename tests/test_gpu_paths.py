@@ -182,3 +182,28 @@ def test_fresh_result_pages(engine):
     assert np.array_equal(got[1000:1000 + want.nbytes], want.reshape(-1).view(np.uint8))
     assert not got[:1000].any() and not got[1000 + want.nbytes:].any()
     h.close()
+
+
+@pytest.mark.parametrize("shape,holes", [
+    ((1, 1, 1), 0), ((1, 31, 33), 0), ((1, 32, 32), 0), ((25, 41, 1), 0), ((9, 17, 23), 0.2), ((31, 33, 35), 0.5),
+])
+def test_ap_order(engine, shape, holes):
+    """De-duplicated APs in caller-given times whose bytes all differ: one voxel, one under, at and over the sort's
+    tile of 1024, several tiles.  The numbering is that of first appearance in raster order."""
+    from ekgsim_gb300.engine import Heart
+    rng = np.random.Generator(np.random.PCG64(shape[1] * 100 + shape[2]))
+    grid = rng.integers(1, 4, size=shape).astype(np.int32)
+    if holes:
+        grid[rng.random(shape) < holes] = 0
+    values = np.concatenate([[1.0, 1.0 + 2.0**-52, 3.0e5], rng.random(200) * 10.0 ** rng.integers(-3, 5, size=200)])
+    at = np.where(grid != 0, values[rng.integers(0, values.size, size=shape)], 0.0)
+    h = Heart.create(engine, grid, synth.transfer_matrix(3, [1, 2, 2]), np.array([[90.0, 95.0, 100.0]]), "3D4", 0.0, 10.0,
+                     1.0, activation=at)
+    seen, want = {}, np.full(grid.size, -1, dtype=np.int64)
+    for i, (g, t) in enumerate(zip(grid.reshape(-1), at.reshape(-1))):
+        if g:
+            want[i] = seen.setdefault((int(g), float(t)), len(seen))
+    assert h.info.n_aps == len(seen)
+    got = h.ap_index().reshape(-1)
+    assert np.array_equal(got[want >= 0], want[want >= 0])
+    h.close()
