@@ -422,7 +422,7 @@ __device__ __forceinline__ void chunk_w(int vb, int vend, const float4 *vox_pos,
 }
 
 // Work items: (32-AP stage st, group of LF_THREADS * LF_ROWS rows), taken from the counter `work`
-// (zeroed before the launch) by a grid of one wave of resident blocks, stages in `stage_order`
+// (cleared by the pass's first kernel) by a grid of one wave of resident blocks, stages in `stage_order`
 // (descending voxel count, so that the last items are short); every item writes its own
 // outputs, so the results do not depend on the order.  A thread owns LF_ROWS consecutive rows
 // (row = s * nmove + l) and evaluates their lead positions together, so the voxel loads and tests

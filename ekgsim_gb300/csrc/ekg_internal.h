@@ -297,7 +297,7 @@ void launch_sim_lead_field(cudaStream_t s, const HeartDev &h, const double *d_le
                            int n_sims, const double *d_layer_k, const float *W0, float *W, float *Wp,
                            bool static_rows);
 // the same W of the moved rows for many simulations, with the batched operand kernel's work split;
-// work: a device counter (zeroed here)
+// work: a device counter (cleared by launch_pass_in)
 void launch_sim_lead_field_rows(cudaStream_t s, const HeartDev &h, const double *d_leads, int nmove, int lead_stride,
                                 int n_sims, float *W, int *work, int sm_count);
 // k0w[s][l] = sum_a k0_{layer(a)} W[s][l][a] for the first `rows` leads
