@@ -603,7 +603,7 @@ def run_ours(args):
                       "contract": bm["contract_ms"] / args.steps, "tail": bm["tail_ms"] / args.steps},
         "roofline": roof,
         # the activation-time relaxation (once per heart): N^3 x 1 B layers in + N^3 x 8 B times out;
-        # latency-bound (one dependent launch per time bucket), so the fraction is its byte floor
+        # latency-bound (a chain of rounds over tiles), so the fraction is its byte floor
         "ca": {"kernel": "k_ca_round", "steps": int(info.ca_rounds),
                "form": "tile rounds up to a horizon", "ms": info.ca_ms,
                "algorithmic_bytes": 9 * int(info.n_cells),

@@ -16,8 +16,8 @@
 // hold later ones form the next round's list (k_ca_round).  The host queues rounds in chunks and reads
 // the lists' length once per chunk.
 //
-// GB300 (relaxation alone, CUDA events): 24^3 0.13 ms, 64^3 0.34, 128^3 0.77, 160^3 1.02
-// (49 rounds), 192^3 1.32, 256^3 2.45.  One launch per time bucket over queues in global memory took
+// GB300 (relaxation alone, CUDA events): 24^3 0.11 ms, 64^3 0.31, 128^3 0.71, 160^3 0.94
+// (49 rounds), 192^3 1.23, 256^3 2.07.  One launch per time bucket over queues in global memory took
 // 0.24, 0.57, 1.40, 1.96, 3.04 and 5.64 ms (9 us a bucket, every access of its chain a trip to L2); rounds
 // of block-wide sweeps to local convergence, without a horizon, 3.4 ms at 160^3 in the calls that
 // allocate nothing.
