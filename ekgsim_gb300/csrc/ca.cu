@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(CA_THREADS, 3)
     __shared__ u64 s_e[HCELLS];       // entries of the tile and its halo
     __shared__ uint8_t s_l[HCELLS];   // layers
     __shared__ uint8_t s_dir[HCELLS]; // which of the 27 tiles a cell lies in, 13 = this one ((dz+1)*9+(dy+1)*3+(dx+1))
-    __shared__ uint32_t s_min[2][CA_WARPS];  // by the step's parity: each warp's earliest pending time
     __shared__ uint32_t s_mark;       // tiles to queue, one bit each
     __shared__ uint32_t s_first;      // earliest time they wait for
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -257,8 +256,11 @@ __global__ void __launch_bounds__(256) k_ca_grid(int nz, int ny, int nx, int nty
     if (threadIdx.x < 8 && s_present[threadIdx.x]) atomicOr(&hdr->present[threadIdx.x], s_present[threadIdx.x]);
 }
 
-// entries -> times; unreachable voxels keep excitationDelay 0
-__global__ void k_ca_finish(size_t n, u64 *__restrict__ at) {
+// entries -> times; unreachable voxels keep excitationDelay 0.  Queued behind every chunk of rounds, it
+// leaves the entries alone while tiles are left: the host's look at the counters then is the call's last
+// wait (launched after that look it cost 16 us more).
+__global__ void k_ca_finish(size_t n, u64 *__restrict__ at, const int32_t *__restrict__ left) {
+    if (*left) return;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const u64 t = at[i] >> 1;
         at[i] = t == INF_BITS ? 0 : t;
@@ -320,6 +322,8 @@ static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, 
             EKG_CUDA(cudaLaunchKernelEx(&cfg, k_ca_round<LT>, r, nz, ny, nx, ntz, nty, ntx, layers, lag, nl1, w, at, T));
         }
         chunk = CHUNK;
+        k_ca_finish<<<1024, 256, 0, s>>>((size_t)nz * ny * nx, at, T.counts + r % 3);
+        EKG_CUDA(cudaGetLastError());
         read(h);
         if (h[r % 3] == 0) return h[3];
         if (r >= cap) throw Error{EKG_ERR_CA_NOT_CONVERGED, "activation-time relaxation did not converge"};
@@ -376,8 +380,6 @@ CaResult ca_run(cudaStream_t s, int nz, int ny, int nx, const uint8_t *d_layers,
                                 EKG_CUDA(cudaMemcpyAsync(h, T.counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
                                 EKG_CUDA(cudaStreamSynchronize(s));
                             });
-    k_ca_finish<<<1024, 256, 0, s>>>(n, entries);
-    EKG_CUDA(cudaGetLastError());
     EKG_CUDA(cudaEventRecord(ev.b, s));
     EKG_CUDA(cudaEventSynchronize(ev.b));
     EKG_CUDA(cudaEventElapsedTime(&res.ms, ev.a, ev.b));
@@ -411,7 +413,20 @@ static __device__ __align__(256) NoAllocScratch g_noalloc;
 std::mutex g_noalloc_mu;
 NoAllocScratch *g_noalloc_ptr[64] = {nullptr};
 
-__global__ void k_na_validate(size_t n, const int32_t *__restrict__ layers, NoAllocScratch *sc) {
+// What the host hands over with a launch: a copy of a few words between two kernels takes 4 to 8 us.
+struct CtrlWords {
+    int32_t v[CA_CTRL_WORDS];
+};
+constexpr int LAG_WORDS = 432;  // 11 layers; longer tables are copied
+struct LagTable {
+    int n;
+    double v[LAG_WORDS];
+};
+
+__global__ void k_na_validate(size_t n, const int32_t *__restrict__ layers, NoAllocScratch *sc, CtrlWords first) {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < CA_CTRL_WORDS; ++k) sc->ctrl[k] = first.v[k];
     uint32_t mask = 0;
     int32_t starts = 0, bad = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -433,7 +448,9 @@ __global__ void k_na_validate(size_t n, const int32_t *__restrict__ layers, NoAl
 }
 
 __global__ void k_na_init(int nz, int ny, int nx, int nty, int ntx, const int32_t *__restrict__ layers,
-                          u64 *__restrict__ at, TileLists T) {
+                          u64 *__restrict__ at, TileLists T, const __grid_constant__ LagTable lag, double *__restrict__ d_lag) {
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < lag.n; i += blockDim.x) d_lag[i] = lag.v[i];
     const size_t n = (size_t)nz * ny * nx;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int32_t v = layers[i];
@@ -480,7 +497,9 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
         cudaStream_t s = 0;
         // clear what must start at zero: flags, counters, layer mask (they are contiguous)
         EKG_CUDA(cudaMemsetAsync(sc->flag, 0, offsetof(NoAllocScratch, lag) - offsetof(NoAllocScratch, flag), s));
-        k_na_validate<<<1024, 256, 0, s>>>(n, d_layers, sc);
+        CtrlWords first;
+        std::copy(std::begin(FIRST_ROUND), std::end(FIRST_ROUND), first.v);
+        k_na_validate<<<1024, 256, 0, s>>>(n, d_layers, sc, first);
         EKG_CUDA(cudaGetLastError());
         struct {
             int32_t nstart;
@@ -514,12 +533,14 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
                     lag[((size_t)a * nl1 + b) * 3 + (k - 1)] = l;
                 }
             }
-        EKG_CUDA(cudaMemcpy(sc->lag, lag, (size_t)nl1 * nl1 * 3 * sizeof(double), cudaMemcpyHostToDevice));
         const TileLists T = tile_lists(sc->ctrl, sc->flag, sc->list[0], NOALLOC_MAX_TILES);
-        // k_na_init appends the stimulus tiles
-        EKG_CUDA(cudaMemcpy(sc->ctrl, FIRST_ROUND, sizeof(FIRST_ROUND), cudaMemcpyHostToDevice));
+        LagTable table;
+        table.n = nl1 * nl1 * 3 <= LAG_WORDS ? nl1 * nl1 * 3 : 0;
+        std::copy(lag, lag + table.n, table.v);
+        if (table.n == 0) EKG_CUDA(cudaMemcpy(sc->lag, lag, (size_t)nl1 * nl1 * 3 * sizeof(double), cudaMemcpyHostToDevice));
+        // k_na_init appends the stimulus tiles (k_na_validate has set the words before the first round)
         u64 *entries = reinterpret_cast<u64 *>(d_at);
-        k_na_init<<<1024, 256, 0, s>>>(nz, ny, nx, nty, ntx, d_layers, entries, T);
+        k_na_init<<<1024, 256, 0, s>>>(nz, ny, nx, nty, ntx, d_layers, entries, T, table, sc->lag);
         EKG_CUDA(cudaGetLastError());
         int dev = 0, sm_count = 0;
         EKG_CUDA(cudaGetDevice(&dev));
@@ -528,8 +549,6 @@ extern "C" int ekg_activation_noalloc(int32_t nz, int32_t ny, int32_t nx, const 
                                       (int)std::min<size_t>(n, INT32_MAX / 2) + 64, sm_count, [&](int32_t *h) {
                                           EKG_CUDA(cudaMemcpy(h, T.counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost));
                                       });
-        k_ca_finish<<<1024, 256, 0, s>>>(n, entries);
-        EKG_CUDA(cudaGetLastError());
         EKG_CUDA(cudaStreamSynchronize(s));
         if (rounds_out) *rounds_out = rounds;
     });

@@ -207,3 +207,22 @@ def test_ap_order(engine, shape, holes):
     got = h.ap_index().reshape(-1)
     assert np.array_equal(got[want >= 0], want[want >= 0])
     h.close()
+
+
+@pytest.mark.parametrize("layers", [11, 12, 31])
+def test_noalloc_lag_tables(engine, layers):
+    """Activation times in caller-owned buffers with the largest lag table that goes with a launch, and longer ones."""
+    import torch
+    from ekgsim_gb300 import _lib as L
+    rng = np.random.Generator(np.random.PCG64(layers))
+    grid = rng.integers(0, layers + 1, size=(17, 12, 20)).astype(np.int32)
+    grid[3, 3, 3], grid[0, 0, 0] = layers, -1
+    tm = synth.transfer_matrix(layers, list(rng.random(layers) * 3 + 0.1))
+    ref, _ = O.activation(grid, tm)
+    d = torch.from_numpy(grid).cuda()
+    at = torch.full(grid.shape, -7.0, dtype=torch.float64, device="cuda")
+    t = np.ascontiguousarray(tm, dtype=np.float64)
+    torch.cuda.synchronize()
+    L.check(L.load().ekg_activation_noalloc(*grid.shape, ctypes.c_void_p(d.data_ptr()), t.shape[0], L.dptr(t),
+                                            ctypes.c_void_p(at.data_ptr()), None))
+    assert np.array_equal(at.cpu().numpy().view(np.int64), ref.view(np.int64))
