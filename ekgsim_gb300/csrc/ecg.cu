@@ -292,6 +292,8 @@ __global__ void __launch_bounds__(CC_T) k_contract_cuda(int steps, int nleads, i
 // What bounds it: FP32 issue, and the shared-memory reads of W' in the band.  A block is 128 threads of
 // which each takes two band steps, so that a row of W' read serves both; the steps' APs are dealt to
 // CB_SLICES / rows slices as if 256 threads took one step each, which fixes the order of the sums.
+// 160^3, 12 leads: 20 simulations 0.214 ms before (a branch around each row's load), 0.147 now; 100
+// simulations 1.024 and 0.691 (issue active 51 and 72 %).
 constexpr int CB_THREADS = 128, CB_WARPS = CB_THREADS / 32, CB_SLICES = 256, CB_LB = 16, CB_CAP = CONTRACT_BAND_CAP;
 // dynamic shared memory of a block with NLB leads: W' [CB_CAP][NLB], the activation times, the
 // band passes' partial sums of half the leads [CB_SLICES][NLB / 2 + 1]
@@ -586,7 +588,10 @@ __global__ void __launch_bounds__(CB_THREADS, NLB <= 12 ? 6 : 4) k_contract_band
 // The layer's sum is float-float, times F_L(t) in FP64; the chunk order is fixed, so the result
 // does not depend on scheduling.  Also writes the float-float copy.
 // Bound by latency (a warp's loads and float-float sums, one behind the other): one simulation at 160^3
-// takes as long as dozens.  The band values of eight chunks are fetched together.
+// takes as long as dozens.  The band values of eight chunks are fetched together (160^3, 100 simulations x
+// 12 leads: 151 us one by one, 134 now).  Several warps per lead and tile, each with a share of the chunks,
+// shorten the tiles that hold the upstrokes with few simulations (3: 46 to 29 us) but lengthen every other
+// pass (100: 250 us); limits and sums as broadcast loads instead of shuffles took 160.
 constexpr int RC_AHEAD = 8;
 __global__ void __launch_bounds__(512) k_reduce_chunks(
     int steps, int nleads, int nl, int nchunks, const int32_t *__restrict__ layer_c0, const int32_t *__restrict__ layer_c1,
