@@ -136,9 +136,11 @@ struct Arena {
     DBuf<uint8_t> mem;
     size_t used = 0;
     static size_t part(size_t bytes) { return (bytes + 255) / 256 * 256; }
+    // Frees the old block, and with it what its views point at, before the new one is allocated (both may
+    // not fit): views that outlive a failure are released by the caller first.
     void reserve(size_t bytes) {
-        mem.alloc(bytes);
         used = 0;
+        mem.alloc(bytes);
     }
     template <class T>
     T *take(size_t count) {
@@ -280,6 +282,61 @@ struct EvalDev {
     DBuf<int64_t> target_len;
     DBuf<double> target_off;
     DBuf<uint32_t> basis_err;  // [1] error word of the basis build
+
+    // values of `out` before the ECG: the error words and the criteria, rounded to 16 bytes
+    static size_t ecg_offset(int n_sims, int n_crit_leads) { return (1 + (size_t)n_sims * n_crit_leads * 2 + 1) / 2 * 2; }
+    // Buffers of every pass, for up to n_sims simulations; whether they are new (the error words are to be
+    // cleared).  A larger batch takes a larger block: the views of the old one are given up before it is
+    // freed, so that after EKG_ERR_OUT_OF_MEMORY nothing is held and a later, smaller batch allocates again.
+    bool reserve_pass(const HeartDev &D, int n_sims) {
+        if (cap_sims >= n_sims) return false;
+        cap_sims = 0;
+        layer_c.release();
+        F.release();
+        Ff.release();
+        k0w.release();
+        out.release();
+        ecg_ff.release();
+        err = nullptr;
+        crit = ecg = nullptr;
+        const size_t S = (size_t)n_sims, nf = S * D.nlayers * D.steps, ne = S * D.nleads * D.steps;
+        const size_t no = ecg_offset(n_sims, D.nleads > 1 ? D.nleads : 1) + ne;
+        mem.reserve(Arena::part(S * D.nlayers * 16) + Arena::part(nf * 8) + Arena::part(nf * 4) + Arena::part(S * D.nleads * 8) +
+                    Arena::part(no * 8) + Arena::part(ne * 8));
+        mem.place(layer_c, S * D.nlayers * 4);
+        mem.place(F, nf);
+        mem.place(Ff, nf);
+        mem.place(k0w, S * D.nleads);
+        mem.place(out, no);
+        mem.place(ecg_ff, ne);
+        cap_sims = n_sims;
+        return true;
+    }
+    // Buffers of the per-simulation form, for the band contraction (one block, as above) or a dense one.
+    void reserve_general(const HeartDev &D, int n_sims, bool band_form) {
+        const size_t S = (size_t)n_sims, nc = S * D.nchunks;
+        const size_t nw = S * D.nleads * D.apad, np = nc * D.nleads * D.steps;
+        if (!band_form) {
+            if (W.n < nw) W.alloc(nw);
+            if (Wp.n < nw) Wp.alloc(nw);
+            if (work.n < 1) work.alloc(1);
+            if (partial.n < np) partial.alloc(np);
+            return;
+        }
+        if (W.n >= nw && band.n >= np && cinfo.n >= nc && csum.n >= nc * D.nleads) return;
+        W.release();
+        band.release();
+        csum.release();
+        cinfo.release();
+        work.release();
+        general.reserve(Arena::part(nw * 4) + Arena::part(np * 4) + Arena::part(nc * D.nleads * 8) + Arena::part(nc * 16) +
+                        Arena::part(4));
+        general.place(W, nw);
+        general.place(band, np);
+        general.place(csum, nc * D.nleads);
+        general.place(cinfo, nc);
+        general.place(work, 1);
+    }
 };
 
 void launch_lead_field(cudaStream_t s, const HeartDev &h, const double *d_leads, int nleads_in, int lead_stride,

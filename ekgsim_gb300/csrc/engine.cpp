@@ -477,32 +477,16 @@ int64_t eval_bytes_per_sim(const ekg_heart *h) {
 }
 int64_t eval_bytes_held(const ekg_heart *h) { return (int64_t)h->ev.cap_sims * eval_bytes_per_sim(h); }
 
-// values of EvalDev::out before the ECG: the error words and the criteria, rounded to 16 bytes
-size_t out_ecg_offset(int n_sims, int n_crit_leads) { return (1 + (size_t)n_sims * n_crit_leads * 2 + 1) / 2 * 2; }
 void ensure_eval_capacity(ekg_heart *h, int n_sims) {
-    EvalDev &E = h->ev;
-    const HeartDev &D = h->dev;
-    if (E.cap_sims >= n_sims) return;
-    const size_t S = (size_t)n_sims;
-    const size_t nf = S * D.nlayers * D.steps, ne = S * D.nleads * D.steps;
-    const size_t no = out_ecg_offset(n_sims, std::max(1, D.nleads)) + ne;
-    E.mem.reserve(Arena::part(S * D.nlayers * 16) + Arena::part(nf * 8) + Arena::part(nf * 4) + Arena::part(S * D.nleads * 8) +
-                  Arena::part(no * 8) + Arena::part(ne * 8));
-    E.mem.place(E.layer_c, S * D.nlayers * 4);
-    E.mem.place(E.F, nf);
-    E.mem.place(E.Ff, nf);
-    E.mem.place(E.k0w, S * D.nleads);
-    E.mem.place(E.out, no);
-    E.mem.place(E.ecg_ff, ne);
-    EKG_CUDA(cudaMemsetAsync(E.out.p, 0, sizeof(double), h->stream));  // the error words
-    E.cap_sims = n_sims;
+    if (h->ev.reserve_pass(h->dev, n_sims))
+        EKG_CUDA(cudaMemsetAsync(h->ev.out.p, 0, sizeof(double), h->stream));  // the error words
 }
 // Places a pass's results in EvalDev::out.
 void place_outputs(ekg_heart *h, int n_sims, int n_crit_leads) {
     EvalDev &E = h->ev;
     E.err = reinterpret_cast<uint32_t *>(E.out.p) + h->cur;
     E.crit = E.out.p + 1;
-    E.ecg = E.out.p + out_ecg_offset(n_sims, n_crit_leads);
+    E.ecg = E.out.p + EvalDev::ecg_offset(n_sims, n_crit_leads);
 }
 // moved rows (simulations x moved leads) from which the per-simulation form evaluates their field
 // with the persistent row kernel (below: one thread per (AP, simulation)); measured at 160^3 with 2
@@ -511,28 +495,6 @@ constexpr int SIM_ROWS_PERSISTENT = 8;
 // whether the per-simulation form contracts with the band form (compact outputs)
 bool band_contraction(const ekg_heart *h) {
     return h->eng->contract == EKG_CONTRACT_BAND && h->dev.chunk_max <= CONTRACT_BAND_CAP;
-}
-// buffers of the general (per-simulation AP) form
-void ensure_general_capacity(ekg_heart *h, int n_sims) {
-    EvalDev &E = h->ev;
-    const HeartDev &D = h->dev;
-    const size_t S = (size_t)n_sims;
-    const size_t nw = S * D.nleads * D.apad, np = S * D.nchunks * D.nleads * D.steps;
-    if (band_contraction(h)) {
-        if (E.W.n >= nw && E.band.n >= np && E.cinfo.n >= S * D.nchunks && E.csum.n >= S * D.nchunks * D.nleads) return;
-        E.general.reserve(Arena::part(nw * 4) + Arena::part(np * 4) + Arena::part(S * D.nchunks * D.nleads * 8) +
-                          Arena::part(S * D.nchunks * 16) + Arena::part(4));
-        E.general.place(E.W, nw);
-        E.general.place(E.band, np);
-        E.general.place(E.csum, S * D.nchunks * D.nleads);
-        E.general.place(E.cinfo, S * D.nchunks);
-        E.general.place(E.work, 1);
-        return;
-    }
-    if (E.W.n < nw) E.W.alloc(nw);
-    if (E.Wp.n < nw) E.Wp.alloc(nw);
-    if (E.work.n < 1) E.work.alloc(1);
-    if (E.partial.n < np) E.partial.alloc(np);
 }
 
 // Device pass for n_sims simulations, split into upload / compute / download so the benchmark
@@ -681,6 +643,7 @@ void ensure_basis(ekg_heart *h, const std::vector<double> &key) {
     BatchState &B = h->bs;
     HeartDev &D = h->dev;
     if (B.basis_ok && B.key == key) return;
+    B.basis_ok = false;  // until the tables below are whole again
     cudaStream_t s = h->stream;
     const int nl = D.nlayers, L = D.nleads, J = 10;
     // centre and half-range of the activation times of each layer
@@ -1069,13 +1032,11 @@ void upload_inputs(ekg_heart *h, const PassPlan &P, const double *layer_k, const
             }
             if (!B.work.p) B.work.alloc(1);
             const size_t ub = (size_t)P.rows_used * D.nlayers * B.max_ent;
-            if (B.U.n < ub) {
-                B.U.alloc(ub);
-                B.Up.alloc(ub * band_u_parts());
-            }
+            if (B.U.n < ub) B.U.alloc(ub);
+            if (B.Up.n < ub * band_u_parts()) B.Up.alloc(ub * band_u_parts());
         }
     } else {
-        ensure_general_capacity(h, n_sims);
+        h->ev.reserve_general(D, n_sims, band_contraction(h));
     }
 }
 
@@ -1397,7 +1358,7 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
     const size_t L = D.nleads, S = n_sims, T = D.steps;
     // a small ECG comes with the criteria in the pass's own copy to pinned memory and is handed over from
     // there: the copy into pageable memory makes the driver wait for the pass and copy twice by itself
-    const size_t ecg_off = out_ecg_offset(n_sims, n_crit_leads);
+    const size_t ecg_off = EvalDev::ecg_offset(n_sims, n_crit_leads);
     const bool small = ecg_host && S * L * T * 8 <= SMALL_ECG_BYTES;
     const size_t need = ecg_off + (small ? S * L * T : 0);
     if (pd.out_cap < need) {
@@ -1909,10 +1870,15 @@ void set_eval(ekg_heart *h, const ekg_eval_config *c) {
     drain_pending(h);  // evaluations in flight are handed over with the settings they ran with
     // device copies of the targets
     EvalDev &E = h->ev;
-    E.targets.alloc(off);
-    E.targets_ff.alloc(off);
-    E.target_len.alloc(c->n_targets);
-    E.target_off.alloc(c->n_targets);
+    try {
+        E.targets.alloc(off);
+        E.targets_ff.alloc(off);
+        E.target_len.alloc(c->n_targets);
+        E.target_off.alloc(c->n_targets);
+    } catch (...) {
+        h->has_eval = false;  // the targets of the settings before are gone
+        throw;
+    }
     EKG_CUDA(cudaSetDevice(h->eng->device));
     EKG_CUDA(cudaMemcpy(E.targets.p, c->targets, off * 8, cudaMemcpyHostToDevice));
     {
