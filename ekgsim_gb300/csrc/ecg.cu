@@ -20,6 +20,7 @@
 #include <cstdio>
 
 #include "ekg_internal.h"
+#include "word_sum.h"
 
 namespace ekg {
 
@@ -49,11 +50,13 @@ __device__ __forceinline__ float h_value(float tau, float4 c) {
 // Block per (128 APs, LFW_LEADS leads, sim s).  Lead positions FP64 [S][lead_stride][3] (z,y,x); W
 // [S][w_lead_stride][apad].  The block's voxels, read in order, get a thread each, which takes the leads
 // together (a neighbour's position is formed once), and each AP's thread then adds its voxels' values in
-// order, as the sum and its rounding errors (two FP32 words, the same W as an FP64 sum gives): a thread
-// walking its AP's voxels waits for their loads one behind the other while its warp diverges over voxel
-// counts, and the FP64 pipe takes 32 clocks for a conversion and an addition of a warp in which most lanes
-// have no voxel left (160^3 heart, 12 leads: 238 us in FP64, a lead or four per block; 131 now).
+// order: a thread walking its AP's voxels waits for their loads one behind the other while its warp diverges
+// over voxel counts.  The sum is held in three FP32 words, and APs of more than WORD_SUM_MAX voxels add those of
+// every LFW_CAP voxels in FP64 (word_sum.h: no more is lost than by a sum in FP64): the FP64 pipe takes 32
+// clocks for a conversion and an addition of a warp in which most lanes have no voxel left (160^3 heart,
+// 12 leads: 238 us in FP64, a lead or four per block; 144 now).
 constexpr int LFW_CAP = 512, LFW_LEADS = 4;  // voxels evaluated at a time, leads per block
+static_assert(LFW_CAP <= WORD_SUM_MAX, "the words of a part are added up before they are too many");
 __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t *__restrict__ a_vox_begin,
                              const int32_t *__restrict__ vox_zyx, const uint32_t *__restrict__ nb_in,
                              const uint32_t *__restrict__ nb_out, int nnb, const int8_t *__restrict__ difs,
@@ -75,9 +78,11 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
     }
     const int v0 = (int)a_vox_begin[a0], v1 = (int)a_vox_begin[a0 + 128 < apad ? a0 + 128 : apad];
     const int vb = on ? (int)a_vox_begin[a] : v1, ve = on ? (int)a_vox_begin[a + 1] : v1;
-    float2 acc[LFW_LEADS];  // (sum, its rounding errors)
+    const bool many = ve - vb > WORD_SUM_MAX;
+    WordSum acc[LFW_LEADS];
+    double wide[LFW_LEADS];
 #pragma unroll
-    for (int k = 0; k < LFW_LEADS; ++k) acc[k] = make_float2(0.f, 0.f);
+    for (int k = 0; k < LFW_LEADS; ++k) wide[k] = 0.0;
     for (int c = v0; c < v1; c += LFW_CAP) {
         const int ce = min(c + LFW_CAP, v1);
         __syncthreads();
@@ -129,15 +134,18 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
         for (int v = max(vb, c); v < min(ve, ce); ++v)
 #pragma unroll
             for (int k = 0; k < LFW_LEADS; ++k)
-                if (k < nl) {
-                    const float2 t = ff_two_sum(acc[k].x, s_w[k][v - c]);
-                    acc[k] = make_float2(t.x, acc[k].y + t.y);
-                }
+                if (k < nl) acc[k].add(s_w[k][v - c]);
+        if (many)
+#pragma unroll
+            for (int k = 0; k < LFW_LEADS; ++k) {
+                wide[k] += acc[k].wide();
+                acc[k] = WordSum();
+            }
     }
     if (on)
 #pragma unroll
         for (int k = 0; k < LFW_LEADS; ++k)
-            if (k < nl) W[((size_t)s * w_lead_stride + l0 + k) * apad + a] = acc[k].x + acc[k].y;
+            if (k < nl) W[((size_t)s * w_lead_stride + l0 + k) * apad + a] = many ? (float)wide[k] : acc[k].value();
 }
 
 // ------------------------------------------------------------------ per-layer factors
