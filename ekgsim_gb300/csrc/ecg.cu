@@ -794,12 +794,14 @@ __device__ __forceinline__ bool ff_greater(float2 a, float2 b) { return a.x > b.
 // throughout.  Writes the criterion value and the argmax (first maximum) of the lead.
 // Bound by the FP64 pipe (an instruction costs it the same for one lane as for 32) and, with few pairs, by
 // latency: the sums of a pass over the steps are reduced together, the number of steps cancels out of the
-// closing quotient, which is one rsqrt, and with few pairs a thread keeps its steps in registers (64^3, one
-// simulation x 2 leads: 6.2 us, now 4.2; 160^3, 256 x 12: 21, now 15.7, where registers or two warps per
-// pair give 19.5).
+// closing quotient, which is one rsqrt, a whole lead's means take its reciprocal as an argument, and with
+// few pairs a thread keeps its steps in registers (64^3, one simulation x 2 leads: 6.2 us, now 5.1; 160^3,
+// 256 x 12: 21, now 16.6, where registers or two warps per pair gave 4 more; the means as float-float products
+// save another 0.3 and 1.2, but that holds them in fewer bits).
 constexpr int CRIT_STEPS = 1024;  // steps that a block keeps in registers
 template <int NT, int PER>
-__global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, int i1, int n_sims, int mode,
+__global__ void __launch_bounds__(NT) k_criteria(int steps, double inv_steps, int nleads, int i0, int i1,
+                                                         int n_sims, int mode,
                                                          const double *__restrict__ ecg,
                                                          const float2 *__restrict__ ecg_ff,
                                                          const double *__restrict__ targets,
@@ -840,17 +842,15 @@ __global__ void __launch_bounds__(NT) k_criteria(int steps, int nleads, int i0, 
     const float2 zero = make_float2(0.f, 0.f);
     double value = 0.0;
     if (mode == 2) {
-        // 1 - cov / (sigma_a sigma_b); the number of steps cancels, and an error of a mean enters the sums
-        // with its square
+        // 1 - cov / (sigma_a sigma_b); the number of steps cancels there.  The means are formed in FP64
         float2 m[2] = {zero, zero};
         each([&](float2 x, float2 y) {
             m[0] = ff_add(m[0], x);
             m[1] = ff_add(m[1], y);
         });
         block_sums_ff<NT>(m, reds);
-        const float n = (float)len, rn = 1.0f / n;
-        const float2 ninv = make_float2(-rn, -rn * fmaf(-rn, n, 1.0f));
-        const float2 ma = ff_mul(m[0], ninv), mb = ff_mul(m[1], ninv);
+        const double inv = len == steps ? -inv_steps : -1.0 / (double)len;
+        const float2 ma = ff_from_double(ff_to_double(m[0]) * inv), mb = ff_from_double(ff_to_double(m[1]) * inv);
         float2 v[3] = {zero, zero, zero};
         each([&](float2 xx, float2 yy) {
             const float2 x = ff_add(xx, ma), y = ff_add(yy, mb);
@@ -1086,8 +1086,8 @@ void launch_criteria(cudaStream_t s, const HeartDev &h, const double *d_ecg, con
     if (i1 <= i0) return;
     const int64_t pairs = (int64_t)(i1 - i0) * n_sims;
     auto go = [&](auto kern, int nt) {
-        kern<<<(unsigned)pairs, nt, 0, s>>>(h.steps, h.nleads, i0, i1, n_sims, mode, d_ecg, d_ecg_ff, d_targets,
-                                            d_targets_ff, d_tlen, d_toff, ncrit_stride, d_crit);
+        kern<<<(unsigned)pairs, nt, 0, s>>>(h.steps, 1.0 / (double)h.steps, h.nleads, i0, i1, n_sims, mode, d_ecg, d_ecg_ff,
+                                            d_targets, d_targets_ff, d_tlen, d_toff, ncrit_stride, d_crit);
     };
     if (pairs >= 1024) go(k_criteria<32, 0>, 32);
     else if (h.steps <= CRIT_STEPS) go(k_criteria<128, CRIT_STEPS / 128>, 128);
