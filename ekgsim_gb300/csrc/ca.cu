@@ -298,8 +298,10 @@ static double round_window(const double *lag, int nl1, const char *present) {
 // after convergence find an empty list).  `read` copies the four counters to the host, waiting.
 // A chunk's end costs some 22 us (the copy, the wait, the next launch without its predecessor to overlap), a
 // round too many 2.5: the first chunk is as long as hearts of 24 to 256 cells were seen to need, 2.2 to 3.5
-// rounds per tile of the longest side, later ones are short (160^3, 49 rounds: five chunks of 12 1.02 ms,
-// one of 50 0.95).
+// rounds per tile of the longest side (160^3, 49 rounds: five chunks of 12 1.02 ms, one of 50 0.95), but no
+// more than 128, and later ones are a quarter of the rounds behind: how many a long strip takes depends on its
+// stimuli (8 x 8 x 524,288 cells: 3 rounds with one in every tile, 364 ms behind a first chunk of 163,840,
+// 5.3 now; 147,337 rounds with a single one, 2.05 s and 1.99).
 template <typename LT, class Read>
 static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, const double *lag, int nl1, double w,
                       u64 *at, const TileLists &T, int cap, int sm_count, Read read) {
@@ -313,15 +315,15 @@ static int run_rounds(cudaStream_t s, int nz, int ny, int nx, const LT *layers, 
     cfg.stream = s;
     cfg.attrs = &pdl;
     cfg.numAttrs = 1;
-    constexpr int CHUNK = 12;
-    int chunk = std::max(CHUNK, 5 * std::max({ntz, nty, ntx}) / 2);
+    constexpr int CHUNK = 12, FIRST_MAX = 128;
+    int chunk = std::max(CHUNK, std::min(FIRST_MAX, 5 * std::min(FIRST_MAX, std::max({ntz, nty, ntx})) / 2));
     int32_t h[4];
     for (int r = 0;;) {
         const int end = (int)std::min<int64_t>(cap, (int64_t)r + chunk);
         for (; r < end; ++r) {
             EKG_CUDA(cudaLaunchKernelEx(&cfg, k_ca_round<LT>, r, nz, ny, nx, ntz, nty, ntx, layers, lag, nl1, w, at, T));
         }
-        chunk = CHUNK;
+        chunk = std::max(CHUNK, r / 4);
         k_ca_finish<<<1024, 256, 0, s>>>((size_t)nz * ny * nx, at, T.counts + r % 3);
         EKG_CUDA(cudaGetLastError());
         read(h);

@@ -49,3 +49,32 @@ def test_criteria_long_leads(engine, sims, steps, mode):
             assert crit[s, 2 * l] == pytest.approx(ref, rel=1e-9, abs=1e-12), (s, l)
             assert crit[s, 2 * l + 1] == abs(int(np.argmax(ecg[s, l])) - int(np.argmax(target[l]))), (s, l)
     h.close()
+
+
+def test_strip_with_many_stimuli():
+    """A strip of 65,536 tiles with a stimulus in each has its activation times after a few rounds: nothing is
+    queued for a front that would run along all of it (that took 0.36 s; a few milliseconds without)."""
+    import time
+    import torch
+    from ekgsim_gb300 import _lib as L
+    shape = (8, 8, 8 * 65536)
+    d = torch.ones(shape, dtype=torch.int32, device="cuda")
+    d[0, 0, ::8] = -1
+    at = torch.empty(shape, dtype=torch.float64, device="cuda")
+    tm = np.ascontiguousarray(synth.transfer_matrix(1, [1.0]))
+    rounds, took = ctypes.c_int32(0), []
+    for _ in range(3):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        L.check(L.load().ekg_activation_noalloc(*shape, ctypes.c_void_p(d.data_ptr()), tm.shape[0], L.dptr(tm),
+                                                ctypes.c_void_p(at.data_ptr()), ctypes.byref(rounds)))
+        took.append(time.perf_counter() - t)
+    assert rounds.value < 20
+    assert min(took) < 0.1
+    grid = np.ones((8, 8, 8 * 4), dtype=np.int32)
+    grid[0, 0, ::8] = -1
+    ref, _ = O.activation(grid, tm)
+    got = at.cpu().numpy()
+    for tile, like in ((0, 0), (1, 1), (30000, 1), (65534, 2)):  # two tiles each: the first, inner ones, the last
+        assert np.array_equal(got[:, :, 8 * tile:8 * tile + 16].view(np.int64),
+                              ref[:, :, 8 * like:8 * like + 16].view(np.int64))
