@@ -2008,8 +2008,9 @@ int ekg_heart_activation(ekg_heart *h, double *at_out) {
         std::lock_guard<std::mutex> lk(h->mu);
         EKG_CUDA(cudaSetDevice(h->eng->device));
         touch_pages(at_out, h->ncell * 8);
-        EKG_CUDA(cudaMemcpyAsync(at_out, h->at_cells.p, h->ncell * 8, cudaMemcpyDeviceToHost, h->stream));
-        EKG_CUDA(cudaStreamSynchronize(h->stream));
+        // on the engine's stream: the times are final, and the heart's stream may hold queued evaluations
+        EKG_CUDA(cudaMemcpyAsync(at_out, h->at_cells.p, h->ncell * 8, cudaMemcpyDeviceToHost, h->eng->stream));
+        EKG_CUDA(cudaStreamSynchronize(h->eng->stream));
     });
 }
 
