@@ -105,13 +105,20 @@ void interior_field(HeartDev &D) {
 }
 
 // ------------------------------------------------------------------ heart setup
-// Host worker threads (the FP64 layer-AP fits of a pass, fresh pages of a result buffer): run(n, f)
-// calls f(begin, end) on contiguous parts of [0, n), one per thread, the caller taking the first; one
-// job at a time.
+// Host worker threads: run(n, f) calls f(begin, end) on contiguous parts of [0, n), one per thread, the
+// caller taking the first; one job at a time.  One pool for the host part of evaluations (the FP64 layer-AP
+// fits: milliseconds a job), and a smaller one for fresh pages of result buffers, which would otherwise
+// wait for another heart's fits (16 cores, 32.8 MB of activation times into fresh memory beside such fits:
+// 3.6 to 12.4 ms, median 9.3, in one pool; 0.5 to 5.2, median 0.6, in two; alone 0.94, 0.61, 0.53 and 0.55
+// ms with 2, 4, 8 and 16 threads).
 class HostPool {
   public:
     static HostPool &get() {
-        static HostPool p;
+        static HostPool p(32);
+        return p;
+    }
+    static HostPool &pages() {
+        static HostPool p(8);
         return p;
     }
     void run(size_t n, const std::function<void(size_t, size_t)> &f) {
@@ -152,9 +159,9 @@ class HostPool {
     }
 
   private:
-    HostPool() {
+    explicit HostPool(unsigned most) {
         const unsigned hc = std::thread::hardware_concurrency();
-        const size_t nw = hc > 1 ? std::min<unsigned>(hc, 32) - 1 : 0;
+        const size_t nw = hc > 1 ? std::min(hc, most) - 1 : 0;
         for (size_t w = 0; w < nw; ++w) workers_.emplace_back([this, w] { loop(w + 1); });
     }
     void loop(size_t part) {
@@ -195,8 +202,9 @@ class HostPool {
 
 // Host memory about to receive a device-to-host copy: pages that the program has not touched yet are
 // brought in here, by the host's threads.  Left to the copy, each is a fault that the GPU waits for
-// (64 KB pages: 32.8 MB of fresh memory 27 ms; brought in first, a copy like any other).
-void touch_pages(void *p, size_t bytes) {
+// (64 KB pages: 32.8 MB of fresh memory 27 ms; brought in first, a copy like any other).  Only a help to the
+// copy: what goes wrong here is left to it, as a pass may be running already.
+void touch_pages(void *p, size_t bytes) try {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
         cudaGetLastError();
@@ -208,10 +216,11 @@ void touch_pages(void *p, size_t bytes) {
     std::vector<unsigned char> in(n);
     if (mincore((void *)a, e - a, in.data()) != 0) return;
     if (std::all_of(in.begin(), in.end(), [](unsigned char v) { return v & 1; })) return;
-    HostPool::get().run(n, [&](size_t b, size_t end) {
+    HostPool::pages().run(n, [&](size_t b, size_t end) {
         for (size_t i = b; i < end; ++i)
             if (!(in[i] & 1)) *(volatile unsigned char *)std::max((uintptr_t)p, a + i * page) = 0;
     });
+} catch (...) {
 }
 
 void heart_setup(ekg_heart *h, const ekg_heart_desc *d) {

@@ -1,4 +1,8 @@
 """Calls beside evaluations that are queued on the device."""
+import ctypes
+import mmap
+import statistics
+import threading
 import time
 
 import numpy as np
@@ -45,4 +49,60 @@ def test_activation_times_beside_a_queued_generation():
     assert alone < whole / 8, (alone, whole)  # the generation is long enough to tell
     assert min(beside) < whole / 4 and max(left) > whole / 8, (alone, whole, beside, left)
     h.close()
+    e.close()
+
+
+def test_fresh_pages_beside_another_hearts_fits():
+    """Results into fresh memory do not wait for the layer-AP fits of another heart's generation."""
+    from ekgsim_gb300 import _lib as L
+    from ekgsim_gb300.engine import Engine, Heart
+    e = Engine(0)
+    rng = np.random.Generator(np.random.PCG64(8))
+    spec = synth.small_spec(40, n_leads=2, seed=8)
+    grid, tm = synth.ellipsoid_heart(spec), synth.transfer_matrix(3, spec.delays)
+    leads = synth.leads(spec, rng)[:, ::-1].copy()
+    big = Heart.create(e, np.pad(grid, ((0, 100), (0, 80), (0, 80))), tm, leads, "3D4", 0.0, 10.0, 1.0)
+    want = big.activation()
+    layers = 10
+    many = np.where(grid != 0, (np.arange(grid.size).reshape(grid.shape) % layers) + 1, 0).astype(np.int32)
+    many[grid < 0] *= -1
+    fit = Heart.create(e, many, synth.transfer_matrix(layers, [1.0] * layers), leads, "3D4", 0.0, 50.0, 1.0)
+    fit.set_eval([synth.BASE_AP] * 3, synth.K_MIN, synth.K_MAX, [5, 6, 7, 8], list(synth.analytic_target(2, 50, 3)),
+                 mid_position=0.6)
+    genes = np.zeros((64, 16))
+    genes[:, :12] = synth.GENE_MIN[:12] + (synth.GENE_MAX - synth.GENE_MIN)[:12] * rng.random((64, 12))
+
+    def fresh():
+        m = mmap.mmap(-1, want.nbytes)
+        p = ctypes.addressof(ctypes.c_char.from_buffer(m))
+        t = time.perf_counter()
+        L.check(L.load().ekg_heart_activation(big._h, ctypes.cast(p, ctypes.POINTER(ctypes.c_double))))
+        t = time.perf_counter() - t
+        assert np.array_equal(np.frombuffer(m, dtype=np.int64), want.view(np.int64).reshape(-1))
+        return t
+
+    def generation():
+        t = time.perf_counter()
+        fit.eval_batch(genes)
+        return time.perf_counter() - t
+
+    for _ in range(3):
+        fresh(), generation()
+    whole = statistics.median(generation() for _ in range(5))
+    stop = threading.Event()
+
+    def loop():
+        while not stop.is_set():
+            fit.eval_batch(genes)
+
+    other = threading.Thread(target=loop)
+    other.start()
+    try:
+        beside = [fresh() for _ in range(41)]
+    finally:
+        stop.set()
+        other.join()
+    assert statistics.median(beside) < whole / 2, (whole, sorted(beside))
+    big.close()
+    fit.close()
     e.close()
