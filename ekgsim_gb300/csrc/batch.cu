@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(128) k_batch_lead_field_small(
 // Both run beside the band GEMM, but the GEMM's ten warps leave no registers for another block (168 a
 // thread; at 152 they share an SM and the GEMM takes 115 us instead of 102), so they live on the SMs that
 // it leaves or ends on: one-warp blocks are placed there soonest (160^3, 256 simulations x 2 moved leads:
-// the sums are ready 20 us behind the GEMM with 128-thread blocks and a warp per output in k_band_u2, now
+// the sums are ready 20 us behind the GEMM with blocks of four and, in k_band_u2, eight warps, now
 // 12; where the GEMM is short the second pass is the longer one: 96^3, 17 simulations: 25 us to 6).
 constexpr int BU_PARTS = 128, BU_AHEAD = 4, BU_THREADS = 32;
 template <int ME>  // entries a layer has at most
@@ -786,44 +786,28 @@ __global__ void __launch_bounds__(BU_THREADS, 32) k_band_u(int rows_used, int nl
         if (e < ne) Up[(((size_t)p * rows_used + rr) * nl + L) * max_ent + e] = make_float2(a[e], b[e]);
 }
 
-// A warp takes O outputs (4 where there are many): lane p adds parts p, p + 32, ..., then 2 O values per lane
-// are added over the lanes by recursive halving (in the order of an xor tree), which takes 9 FP64 additions
-// for four outputs instead of 40.  Bound by the FP64 pipe.
-template <int O>
+// A warp per output: lane p adds parts p, p + 32, ..., then the upper half warp's lanes take S1 over from
+// the lower one's and give it S0, and each half adds its 16 values (in the order of an xor tree over 32 lanes),
+// 5 FP64 additions instead of 10.  Bound by the FP64 pipe.  Four outputs a warp take 9 for all of them, but
+// fewer warps: 96^3, 100 simulations x 12 moved leads 536 us a call against 528, 48^3, 500 x 2 413 and 397,
+// and no less with more (160^3, 256 x 12: 3,555 and 3,553).
 __global__ void __launch_bounds__(32) k_band_u2(int64_t n_out, const float2 *__restrict__ Up, float2 *__restrict__ U) {
     const int lane = threadIdx.x;
-    const int64_t i = (int64_t)blockIdx.x * O;
-    float2 v[O][BU_PARTS / 32];
+    const int64_t i = blockIdx.x;
+    float2 v[BU_PARTS / 32];
 #pragma unroll
-    for (int q = 0; q < O; ++q)
+    for (int k = 0; k < BU_PARTS / 32; ++k) v[k] = Up[(lane + k * 32) * n_out + i];
+    double s0 = (double)v[0].x, s1 = (double)v[0].y;
 #pragma unroll
-        for (int k = 0; k < BU_PARTS / 32; ++k) v[q][k] = Up[(lane + k * 32) * n_out + min(i + q, n_out - 1)];
-    double x[2 * O];
-#pragma unroll
-    for (int q = 0; q < O; ++q) {
-        x[q] = (double)v[q][0].x;
-        x[O + q] = (double)v[q][0].y;
-#pragma unroll
-        for (int k = 1; k < BU_PARTS / 32; ++k) {
-            x[q] += (double)v[q][k].x;
-            x[O + q] += (double)v[q][k].y;
-        }
+    for (int k = 1; k < BU_PARTS / 32; ++k) {
+        s0 += (double)v[k].x;
+        s1 += (double)v[k].y;
     }
-    int idx = 0, d = 16;
+    const bool up = lane & 16;
+    double x = (up ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up ? s0 : s1, 16);
 #pragma unroll
-    for (int n = O; n >= 1; n >>= 1, d >>= 1) {
-        const bool up = lane & d;
-#pragma unroll
-        for (int j = 0; j < n; ++j) {
-            const double keep = up ? x[j + n] : x[j], give = up ? x[j] : x[j + n];
-            x[j] = keep + __shfl_xor_sync(0xffffffffu, give, d);
-        }
-        idx += up ? n : 0;
-    }
-#pragma unroll
-    for (; d >= 1; d >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], d);
-    // value idx: S0 of output idx, or S1 of output idx - O; lanes that share one write the same
-    if (i + idx % O < n_out) reinterpret_cast<float *>(U)[(i + idx % O) * 2 + idx / O] = (float)x[0];
+    for (int d = 8; d >= 1; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+    if ((lane & 15) == 0) reinterpret_cast<float *>(U)[i * 2 + (up ? 1 : 0)] = (float)x;
 }
 
 // ------------------------------------------------------------------ batch GEMM
@@ -1744,11 +1728,13 @@ void launch_band_u(cudaStream_t s, const BandArgs &A) {
     auto go = [&](auto kern) {
         kern<<<grid, BU_THREADS, 0, s>>>(A.rows_used, A.nl, A.max_ent, A.nent, A.esplit, A.ls0, A.ls1, A.goff, A.gtab, A.P1, A.Up);
     };
+    // most hearts' times make two or three entries a layer; with the loops over all eight compiled in, 160^3, 256
+    // simulations x 12 moved leads take 3,565 us a call instead of 3,555 (this kernel 58 instead of 50), 60 x 12
+    // 1,019 instead of 1,012
     if (A.max_ent <= 4) go(k_band_u<4>);
     else go(k_band_u<MAXE>);
     const int64_t n = (int64_t)A.rows_used * A.nl * A.max_ent;
-    if (n >= 4096) k_band_u2<4><<<(unsigned)((n + 3) / 4), 32, 0, s>>>(n, A.Up, A.U);
-    else k_band_u2<1><<<(unsigned)n, 32, 0, s>>>(n, A.Up, A.U);
+    k_band_u2<<<(unsigned)n, 32, 0, s>>>(n, A.Up, A.U);
     EKG_CUDA(cudaGetLastError());
 }
 
