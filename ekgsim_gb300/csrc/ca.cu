@@ -6,8 +6,8 @@
 // lags that search returns the unique fixed point of
 //     at(v) = min(init(v), min_u fl(at(u) + fl(T[L(u)][L(v)] * sqrt(k))))
 // (every offered time is >= the offering voxel's own time), so a chaotic min-relaxation from
-// +inf converges to the same doubles bit for bit, in any order.  Products and sums use
-// __dmul_rn / __dadd_rn so the compiler cannot fuse them into an FMA.
+// +inf converges to the same doubles bit for bit, in any order.  The products are formed on the host,
+// the sums with __dadd_rn.
 //
 // Layout: the grid is cut into 8x8x8 tiles.  A round visits the tiles that hold pending times, one
 // CTA each: the tile and a one-voxel halo are staged in shared memory (the FP64 times as their bit
@@ -70,13 +70,12 @@ __device__ __forceinline__ void tile_append(const TileLists &T, int tile, int ro
 //
 // What bounds it: latency -- a chain of rounds, in a round the slowest tile's chain of settling steps,
 // in a step its barriers and dependent shared-memory accesses.  Hence:
-//  - a tile settles its voxels in the order of their times, as the search itself does: per step the
-//    voxels whose pending time lies within the smallest lag of the earliest pending one (nothing
-//    later inside the tile can improve them) offer to their 26 neighbours, a warp per voxel and a
-//    lane per neighbour, so that each voxel offers about once;
+//  - a tile settles in steps: every voxel whose pending time lies within the round's horizon offers it to its
+//    26 neighbours, a warp per voxel and a lane per neighbour, and offers again where a later step brings
+//    it an earlier time (settling the earliest pending times first took as long, 1.11 and 1.12 ms at 160^3);
 //  - a step has one barrier and no list: a warp expands the selected ones of its own 32 voxels, which
-//    lie spread over the tile so that a front falls on all warps, and the earliest pending time of
-//    the next step is taken from each warp's own voxels and the offers that it made;
+//    lie spread over the tile so that a front falls on all warps, and another step follows where
+//    a voxel was selected, or an offer within the horizon may have come after its target's read;
 //  - offers across the tile's surface go to the neighbour's cells in global memory (an atomicMin whose
 //    result nothing waits for), so that a visit starts from the pending cells alone;
 //  - a round settles only times up to its horizon, the earliest pending time of the heart + `window`
@@ -152,14 +151,15 @@ __global__ void __launch_bounds__(CA_THREADS, 3)
         const u64 orig = s_e[me];
         const int myl = s_l[me];
         u64 offered = orig & 1 ? ~0ULL : orig >> 1;  // the time that the voxel has offered
-        uint32_t mark = 0, first = NONE, sent = NONE;  // sent: earliest offer of the last step within the tile
+        uint32_t mark = 0, first = NONE;
+        bool sent = false;  // an offer of the last step within the tile and the horizon
         // settling steps: every voxel with a pending time up to the horizon offers it; they end, as times only fall
         for (;;) {
             const u64 mine = s_e[me] >> 1;
             const bool sel = mine != offered && mine <= upto;
             // an offer made in the last step may have come too late for its target's read
-            if (!__syncthreads_or(sel || sent != NONE)) break;
-            sent = NONE;
+            if (!__syncthreads_or(sel || sent)) break;
+            sent = false;
             if (sel) offered = mine;
             for (unsigned b = __ballot_sync(0xffffffffu, sel); b; b &= b - 1) {
                 const int src = __ffs(b) - 1;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(CA_THREADS, 3)
                     if (ce < ev && ce < atomicMin(&s_e[v], ce)) {
                         const int dir = s_dir[v];
                         if (dir == 13) {
-                            if (c <= upto) sent = min(sent, (uint32_t)(c >> 32));
+                            sent = sent || c <= upto;
                         } else {
                             const int hx = v % HS, hy = (v / HS) % HS, hz = v / (HS * HS);
                             atomicMin(&at[((size_t)(tz0 + hz - 1) * ny + (ty0 + hy - 1)) * nx + (tx0 + hx - 1)], ce);
@@ -284,8 +284,8 @@ static const int32_t FIRST_ROUND[CA_CTRL_WORDS] = {0, 0, 0, 0, 0x3ff00000 /* hig
 
 // The width of a round, 5 of the largest lag between present layers: in a narrower one the rounds' fixed
 // cost shows (launch, staging, write-back), in a wider one the wave leaves the tile and its successors
-// wait.  160^3 heart with lags 1, 2, 2 ms: 1.06, 1.03, 1.02, 1.04, 1.15, 1.69 ms at 2.5, 4, 6, 8, 16 and
-// without an end; 256^3: 2.47, 2.43, 2.50, 2.58, 3.3, 7.7 ms.
+// wait.  160^3 heart with lags 1, 2, 2 ms (a whole call): 1.06, 1.07, 1.07, 1.10, 1.11, 1.16 and 1.71 ms at 2.5, 4, 5,
+// 6, 8, 16 and without an end, repeats within 2 %; 256^3, ten layers: 2.42, 2.45, 2.47, 2.51, 2.58, 2.91, 6.1 ms.
 static double round_window(const double *lag, int nl1, const char *present) {
     double hi = 0.0;
     for (int a = 1; a < nl1; ++a)

@@ -975,7 +975,10 @@ __global__ void __launch_bounds__(PIO_THREADS) k_pass_out(const double *src, dou
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
-// up to these sizes by kernel, larger ones by the copy engine
+// Up to these sizes by kernel, larger ones by the copy engine.  Where the lines lie matters little (24^3 heart, us a
+// call, kernel / copy engine: inputs of 54 KB 124 / 128, 542 KB 466 / 474, 868 KB 582 / 594, 1.4 MB 796 /
+// 795, 2.7 MB 1,269 / 1,266; criteria of 18 KB 124 / 132, 187 KB 466 / 474, 300 KB 578 / 585, 937 KB 1,263
+// / 1,273), but a larger ECG keeps blocks of the kernel waiting for the host's memory: see SMALL_ECG_BYTES.
 constexpr size_t PASS_IN_MAX = 1 << 20, PASS_OUT_MAX = 1 << 18;
 static unsigned pass_blocks(size_t n) {
     return (unsigned)std::max<size_t>(1, (n + PIO_THREADS - 1) / PIO_THREADS);

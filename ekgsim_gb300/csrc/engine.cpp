@@ -1351,11 +1351,15 @@ void assemble_criteria(const ekg_heart *h, const double *crit2, bool done, doubl
 TuneChoice tune_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, int reps,
                      double *builtin_ms);
 
+// An ECG up to SMALL_ECG_BYTES reaches the caller from the pass's own copy to page-locked memory, a larger one
+// by a copy into the caller's (24^3 heart, one simulation, us a call, the one / the other: 9 KB 28 / 37, 61 KB
+// 32 / 39, 127 KB 37 / 43, 188 KB 41 / 42, 253 KB 46 / 42, 502 KB 68 / 48).
+constexpr size_t SMALL_ECG_BYTES = 128 << 10;
+
 // Queues one device pass from the current staging buffer (h->cur): plan, the pass with the copies of its
 // inputs and of its criterion values and error word (one graph replay), and a larger ECG's copies to
 // ecg_host.  pend[h->cur].done marks the pass and its copies complete.
 // The pass's kernels wait for the previous pass's copies to the host (they overwrite its outputs).
-constexpr size_t SMALL_ECG_BYTES = 128 << 10;
 void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, double *ecg_host,
                  int n_crit_leads, int mode) {
     HeartDev &D = h->dev;
