@@ -1360,8 +1360,8 @@ constexpr size_t SMALL_ECG_BYTES = 128 << 10;
 // inputs and of its criterion values and error word (one graph replay), and a larger ECG's copies to
 // ecg_host.  pend[h->cur].done marks the pass and its copies complete.
 // The pass's kernels wait for the previous pass's copies to the host (they overwrite its outputs).
-void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, double *ecg_host,
-                 int n_crit_leads, int mode) {
+void queue_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, double *ecg_host,
+                int n_crit_leads, int mode) {
     HeartDev &D = h->dev;
     EvalDev &E = h->ev;
     cudaStream_t s = h->stream;
@@ -1432,6 +1432,18 @@ void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *
     EKG_CUDA(cudaEventRecord(h->copies_done, h->copy_stream));
     EKG_CUDA(cudaEventRecord(pd.done, h->copy_stream));
     h->copies_pending = true;
+}
+// A pass that fails half-way has kernels queued that read its staging buffer and write its results, and no
+// event that marks their end: they are waited for before the slot is used again.
+void launch_pass(ekg_heart *h, int n_sims, const double *layer_k, const double *leads, double *ecg_host,
+                 int n_crit_leads, int mode) {
+    try {
+        queue_pass(h, n_sims, layer_k, leads, ecg_host, n_crit_leads, mode);
+    } catch (...) {
+        for (cudaStream_t q : {h->stream, h->aux_stream, h->copy_stream})
+            if (q) cudaStreamSynchronize(q);
+        throw;
+    }
 }
 
 // Clears a slot's error word once it is reported (no pass of the slot is in flight then).

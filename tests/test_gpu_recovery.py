@@ -49,3 +49,30 @@ def test_batch_after_one_that_does_not_fit(form, free, n_leads, steps, dt):
             assert np.array_equal(a, c) and np.array_equal(b, c)
     h.close()
     e.close()
+
+
+@pytest.mark.parametrize("want_ecg", [False, True])
+def test_batch_after_one_that_failed_half_way(want_ecg):
+    """A batch with more moved rows (65,544) than a grid has: its first kernels are queued when the driver refuses
+    the launch.  The batch after it waits for them and gives what it gave before."""
+    from ekgsim_gb300.engine import Engine, EkgError, Heart
+    e = Engine(0)
+    spec = synth.small_spec(24, n_leads=12, seed=4)
+    grid, tm = synth.ellipsoid_heart(spec), synth.transfer_matrix(3, spec.delays)
+    rng = np.random.Generator(np.random.PCG64(5))
+    leads = synth.leads(spec, rng)[:, ::-1].copy()
+    h = Heart.create(e, grid, tm, leads, "3D4", 0.0, 40.0, 1.0)
+    h.set_eval([synth.BASE_AP] * 3, synth.K_MIN, synth.K_MAX, [5, 6, 7, 8], list(synth.analytic_target(12, 40, 3)),
+               mid_position=0.6)
+    genes = np.zeros((5462, 36))
+    genes[:, :12] = synth.GENE_MIN[:12] + (synth.GENE_MAX - synth.GENE_MIN)[:12] * rng.random((5462, 12))
+    genes[:, 12:] = rng.uniform(-10, 10, size=(5462, 24))
+    want = h.eval_batch(genes[:9], want_ecg=want_ecg)
+    for _ in range(2):
+        with pytest.raises(EkgError) as err:
+            h.eval_batch(genes, want_ecg=want_ecg)
+        assert err.value.code == -4
+        for a, b in zip(want, h.eval_batch(genes[:9], want_ecg=want_ecg)):
+            assert np.array_equal(a, b)
+    h.close()
+    e.close()
