@@ -10,7 +10,7 @@ enum { EKG_CONTRACT_BAND = 0, EKG_CONTRACT_DENSE_UMMA = 1, EKG_CONTRACT_DENSE_CU
 
 struct ekg_engine {
     int device = 0;
-    cudaStream_t stream = nullptr;  // copies of what is final since a heart's set-up (activation times)
+    cudaStream_t stream = nullptr;  // a heart's activation times while evaluations are queued on its own
     int chunk_len = 512;  // APs per K chunk of the contraction (multiple of 64)
     // per-simulation contraction: band form (default), dense on the tensor cores (EKG_CONTRACT=umma)
     // or dense on the CUDA cores (EKG_CONTRACT=cuda)

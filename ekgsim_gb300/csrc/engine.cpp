@@ -2033,9 +2033,10 @@ int ekg_heart_activation(ekg_heart *h, double *at_out) {
         std::lock_guard<std::mutex> lk(h->mu);
         EKG_CUDA(cudaSetDevice(h->eng->device));
         touch_pages(at_out, h->ncell * 8);
-        // on the engine's stream: the times are final, and the heart's stream may hold queued evaluations
-        EKG_CUDA(cudaMemcpyAsync(at_out, h->at_cells.p, h->ncell * 8, cudaMemcpyDeviceToHost, h->eng->stream));
-        EKG_CUDA(cudaStreamSynchronize(h->eng->stream));
+        // the times are final: beside queued evaluations, not behind them
+        const cudaStream_t s = h->pend[0].busy || h->pend[1].busy ? h->eng->stream : h->stream;
+        EKG_CUDA(cudaMemcpyAsync(at_out, h->at_cells.p, h->ncell * 8, cudaMemcpyDeviceToHost, s));
+        EKG_CUDA(cudaStreamSynchronize(s));
     });
 }
 
