@@ -54,7 +54,8 @@ __device__ __forceinline__ float h_value(float tau, float4 c) {
 // over voxel counts.  The sum is held in three FP32 words, and APs of more than WORD_SUM_MAX voxels add those of
 // every LFW_CAP voxels in FP64 (word_sum.h: no more is lost than by a sum in FP64): the FP64 pipe takes 32
 // clocks for a conversion and an addition of a warp in which most lanes have no voxel left (160^3 heart,
-// 12 leads: 238 us in FP64, a lead or four per block; 144 now).
+// 12 leads: 238 us in FP64, a lead or four per block; 133 now: 144 with the parts' sums in registers and every
+// term added in full).
 constexpr int LFW_CAP = 512, LFW_LEADS = 4;  // voxels evaluated at a time, leads per block
 static_assert(LFW_CAP <= WORD_SUM_MAX, "the words of a part are added up before they are too many");
 __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t *__restrict__ a_vox_begin,
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
                              float *__restrict__ W, int w_lead_stride) {
     __shared__ float4 s_dif[26];
     __shared__ float s_w[LFW_LEADS][LFW_CAP];
+    __shared__ double s_wide[LFW_LEADS][128];  // long APs: sums over the parts
     const int tid = threadIdx.x;
     if (tid < nnb) s_dif[tid] = make_float4(difs[3 * tid], difs[3 * tid + 1], difs[3 * tid + 2], 0.f);
     const int64_t a0 = blockIdx.x * (int64_t)128, a = a0 + tid;
@@ -80,9 +82,8 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
     const int vb = on ? (int)a_vox_begin[a] : v1, ve = on ? (int)a_vox_begin[a + 1] : v1;
     const bool many = ve - vb > WORD_SUM_MAX;
     WordSum acc[LFW_LEADS];
-    double wide[LFW_LEADS];
-#pragma unroll
-    for (int k = 0; k < LFW_LEADS; ++k) wide[k] = 0.0;
+    if (many)
+        for (int k = 0; k < LFW_LEADS; ++k) s_wide[k][tid] = 0.0;
     for (int c = v0; c < v1; c += LFW_CAP) {
         const int ce = min(c + LFW_CAP, v1);
         __syncthreads();
@@ -131,21 +132,31 @@ __global__ void __launch_bounds__(128) k_lead_field(int64_t apad, const int64_t 
             for (int k = 0; k < LFW_LEADS; ++k) s_w[k][v - c] = w[k];
         }
         __syncthreads();
-        for (int v = max(vb, c); v < min(ve, ce); ++v)
+        int v = max(vb, c);
+        const int end = min(ve, ce);
+        if (v < end && (v == vb || many)) {  // nothing in the words yet; many APs have one or two voxels
+            const bool two = v + 1 < end;
 #pragma unroll
-            for (int k = 0; k < LFW_LEADS; ++k)
-                if (k < nl) acc[k].add(s_w[k][v - c]);
+            for (int k = 0; k < LFW_LEADS; ++k) {
+                acc[k].s = s_w[k][v - c];
+                if (two) acc[k].second(s_w[k][v + 1 - c]);
+            }
+            v += 2;
+        }
+        for (; v < end; ++v)
+#pragma unroll
+            for (int k = 0; k < LFW_LEADS; ++k) acc[k].add(s_w[k][v - c]);
         if (many)
 #pragma unroll
             for (int k = 0; k < LFW_LEADS; ++k) {
-                wide[k] += acc[k].wide();
+                s_wide[k][tid] += acc[k].wide();
                 acc[k] = WordSum();
             }
     }
     if (on)
 #pragma unroll
         for (int k = 0; k < LFW_LEADS; ++k)
-            if (k < nl) W[((size_t)s * w_lead_stride + l0 + k) * apad + a] = many ? (float)wide[k] : acc[k].value();
+            if (k < nl) W[((size_t)s * w_lead_stride + l0 + k) * apad + a] = many ? (float)s_wide[k][tid] : acc[k].value();
 }
 
 // ------------------------------------------------------------------ per-layer factors

@@ -29,6 +29,8 @@ struct WordSum {
 #endif
         return r;
     }
+    // the second term behind a first one that was put into s
+    EKG_HOST_DEVICE void second(float w) { s = two_sum(s, w, e); }
     EKG_HOST_DEVICE void add(float w) {
         float d, d2;
         s = two_sum(s, w, d);

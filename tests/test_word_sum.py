@@ -21,7 +21,7 @@ def lib(tmp_path_factory):
                         "-o", out], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     lib = ctypes.CDLL(out)
-    for f in (lib.word_sum, lib.word_sum_parts):
+    for f in (lib.word_sum, lib.word_sum_short, lib.word_sum_parts):
         f.restype = ctypes.c_float
         f.argtypes = [ctypes.c_void_p, ctypes.c_int]
     return lib
@@ -44,6 +44,7 @@ def test_no_more_is_lost_than_in_64_bits(lib, n):
         want = math.fsum(w.astype(np.float64))
         size = math.fsum(np.abs(w.astype(np.float64)))
         got = lib.word_sum(w.ctypes.data, n)
+        assert lib.word_sum_short(w.ctypes.data, n) == got
         assert abs(got - want) <= 2.0**-23 * abs(want) + n**3 * 2.0**-72 * size
 
 
@@ -63,6 +64,6 @@ def test_parts_in_64_bits(lib, n):
                                     ([math.inf, -math.inf], math.nan), ([1, math.nan], math.nan), ([-0.0], 0.0)])
 def test_not_finite(lib, w, want):
     a = np.array(w, dtype=np.float32)
-    for f in (lib.word_sum, lib.word_sum_parts):
+    for f in (lib.word_sum, lib.word_sum_short, lib.word_sum_parts):
         got = f(a.ctypes.data, a.size)
         assert (math.isnan(want) and math.isnan(got)) or got == want
