@@ -53,8 +53,8 @@ def test_batch_after_one_that_does_not_fit(form, free, n_leads, steps, dt):
 
 @pytest.mark.parametrize("want_ecg", [False, True])
 def test_batch_after_one_that_failed_half_way(want_ecg):
-    """A batch with more moved rows (65,544) than a grid has: its first kernels are queued when the driver refuses
-    the launch.  The batch after it waits for them and gives what it gave before."""
+    """A batch with more moved rows (65,544) than a grid has: its first kernels are queued when CUDA refuses the
+    launch.  The batch after it waits for them and gives what it gave before."""
     from ekgsim_gb300.engine import Engine, EkgError, Heart
     e = Engine(0)
     spec = synth.small_spec(24, n_leads=12, seed=4)
